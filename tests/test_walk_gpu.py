@@ -1,0 +1,50 @@
+"""The tiled half-steps at the edges of their tiles (8 columns, up to 120 rows
+in four warps of diagonals): one to three rows and columns, a tile exactly full
+and one row or column over, two tiles of uneven remainder, a surface row that
+is not a multiple of four. The per-cell kernels perform the same operations in
+the same order, so fields and traces must agree bit for bit."""
+import numpy as np
+import pytest
+
+import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(kernel, monkeypatch, variant, nz, nx, eal, fs, dz):
+    import ttifd
+
+    monkeypatch.setenv("TTIFD_EXACT", "1")
+    monkeypatch.setenv("TTIFD_KERNEL", kernel)
+    nt = 60
+    cfg = dict(variant=variant, nz=nz, nx=nx, nt=nt, dx=10.0, dz=dz, dt=0.0008, fpeak=30.0, ealThick=eal,
+               freesurface=fs, stype=1, seistype=3)
+    m = synthetic.layered_model(nz, nx, seed=5)
+    with ttifd.Modeling(**cfg) as h:
+        h.upload_model(*synthetic.padded(m, eal))
+        h.set_source([nx // 2], [min(2, nz - 1)], synthetic.ricker(nt, cfg["dt"], cfg["fpeak"], delay=0.01)[None, :])
+        for k in (0, 1, 2):
+            h.set_receivers(k, np.arange(nx), nz // 2)
+        h.run()
+        out = [h.fetch_traces(k) for k in (0, 1, 2)]
+        out += [h.fetch_field(f) for f in range(8 if variant == "tensor_rotation" else 5)]
+    return out
+
+
+# updated rows: nz + 2 (eal + 5) - 10 without a free surface, less eal + 5 with one
+@pytest.mark.parametrize("nz,nx,eal,fs,dz", [
+    (1, 1, 1, 0, 10.0),      # 3 x 3 cells
+    (2, 7, 2, 1, 10.0),      # surface row 7
+    (118, 6, 1, 0, 10.0),    # 120 rows, 8 columns: one full tile
+    (119, 7, 1, 0, 8.0),     # 121 rows, 9 columns: two tiles each way
+    (113, 23, 4, 1, 10.0),   # surface row 9, 121 rows from row 8
+    (236, 9, 2, 0, 12.5),    # 240 rows: two full tiles
+    (237, 16, 2, 1, 10.0),   # surface row 7, two tiles and a remainder
+])
+@pytest.mark.parametrize("variant", ["coordinate_rotation", "tensor_rotation", "bond_transformation"])
+def test_tile_edges(variant, nz, nx, eal, fs, dz, monkeypatch, gpu_lib):
+    ref = _run("naive", monkeypatch, variant, nz, nx, eal, fs, dz)
+    got = _run("tiled", monkeypatch, variant, nz, nx, eal, fs, dz)
+    for k, (a, b) in enumerate(zip(got, ref)):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (k, np.max(np.abs(a - b)))
+    assert any(np.any(b != 0) for b in ref)

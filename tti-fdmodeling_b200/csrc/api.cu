@@ -11,7 +11,7 @@
 #include <algorithm>
 #include <numeric>
 
-#include "tiled.cuh"
+#include "walk.cuh"
 
 using namespace ttifd;
 
@@ -144,11 +144,9 @@ int launch_one_step(tti_handle *h, const SourceTables &tab, cudaEvent_t *ev = nu
   // txx tzz txz) after the sources, from whose stencils the adjoint works.
   const bool keep_tiled = keep && h->use_tiled;
   if (h->use_tiled) {
-    const CUtensorMap *tm = static_cast<const CUtensorMap *>(h->tmaps);
     ha.g = h->g;
     ha.f = a.f;
     ha.p = a.p;
-    ha.pk = packed::Packed{h->pk_cf, h->pk_vsc, h->pk_sc, h->pk_c4};
     ha.invdx = h->invdx;
     ha.invdz = h->invdz;
     ha.dt = c.dt;
@@ -158,9 +156,7 @@ int launch_one_step(tti_handle *h, const SourceTables &tab, cudaEvent_t *ev = nu
     tiled::set_square(ha, h->exact);
     ha.wait_limit = h->wait_limit;
     ha.err = h->d_flag;
-    ha.map[0] = tm[2];  // sxx szz sxz for the velocity update
-    ha.map[1] = tm[3];
-    ha.map[2] = tm[4];
+    tiled::set_half(ha, static_cast<const CUtensorMap *>(h->tmaps), c.variant, true);
     if (keep_tiled && c.variant == TTI_COORDINATE)
       for (int k = 0; k < 4; ++k) ha.kd[k] = keep[4 + k];
   }
@@ -177,9 +173,7 @@ int launch_one_step(tti_handle *h, const SourceTables &tab, cudaEvent_t *ev = nu
   }
   if (ev) CK(h, cudaEventRecord(ev[2], h->stream));
   if (h->use_tiled) {
-    const CUtensorMap *tm = static_cast<const CUtensorMap *>(h->tmaps);
-    ha.map[0] = tm[0];  // vx vz for the stress update
-    ha.map[1] = tm[1];
+    tiled::set_half(ha, static_cast<const CUtensorMap *>(h->tmaps), c.variant, false);
     for (int k = 0; k < 4; ++k) ha.kd[k] = keep_tiled ? keep[k] : nullptr;
     for (int k = 0; k < 3; ++k) ha.kt[k] = keep_tiled && c.variant == TTI_TENSOR ? keep[4 + k] : nullptr;
     CK(h, tiled::launch_stress(ha, c.variant, h->exact, h->stream));
@@ -567,20 +561,6 @@ int create_handle(tti_handle **out, const tti_config *cfg, int device, const tti
   }
   for (int f = 0; f < nfields(cfg->variant); ++f)
     if ((rc = alloc(&h->fld[f]))) return fail(rc);
-  if (h->use_tiled) {
-    void *mem = nullptr;
-    if (posix_memalign(&mem, 64, 5 * sizeof(CUtensorMap)) != 0) {
-      set_err(h, TTI_ERR_NOMEM, "host allocation failed");
-      return fail(TTI_ERR_NOMEM);
-    }
-    h->tmaps = mem;
-    CUtensorMap *tm = static_cast<CUtensorMap *>(mem);
-    for (int k = 0; k < 5; ++k)
-      if (!tiled::encode_map(tm + k, g, h->fld[k])) {
-        set_err(h, TTI_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-        return fail(TTI_ERR_CUDA);
-      }
-  }
   if (share) {
     h->owner = share;
     for (int p = 0; p < TTI_P_COUNT; ++p) h->par[p] = share->par[p];
@@ -602,6 +582,18 @@ int create_handle(tti_handle **out, const tti_config *cfg, int device, const tti
   }
   for (int p = 0; p < TTI_P_COUNT && !share; ++p)
     if (param_used(cfg->variant, p) && (rc = alloc(&h->par[p]))) return fail(rc);
+  if (h->use_tiled) {
+    if (posix_memalign(&h->tmaps, 64, tiled::MAPS * sizeof(CUtensorMap)) != 0) {
+      h->tmaps = nullptr;
+      set_err(h, TTI_ERR_NOMEM, "host allocation failed");
+      return fail(TTI_ERR_NOMEM);
+    }
+    const StepArgs a = step_args(h);
+    if (!tiled::encode_maps(static_cast<CUtensorMap *>(h->tmaps), g, cfg->variant, a.f, a.p)) {
+      set_err(h, TTI_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+      return fail(TTI_ERR_CUDA);
+    }
+  }
   if (pool_alloc(reinterpret_cast<void **>(&h->d_flag), sizeof(int), h->stream) != cudaSuccess ||
       pool_alloc(reinterpret_cast<void **>(&h->d_energy), sizeof(double) * 2 * (size_t)cfg->nt, h->stream) !=
           cudaSuccess) {

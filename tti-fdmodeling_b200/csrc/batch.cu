@@ -16,7 +16,7 @@
 #include <string>
 #include <vector>
 
-#include "tiled.cuh"
+#include "walk.cuh"
 
 using namespace ttifd;
 
@@ -110,24 +110,22 @@ int build_tables(tti_batch *b)
   std::vector<BatchSrc> src(n);
   std::vector<SourceTables> tab(nm);
   for (int m = 0; m < nm; ++m) handle_source_tables(b->models[m], &tab[m]);
-  std::vector<int> tiles(n);
+  std::vector<dim3> tiles(n);
   bool all_square = true;
   sync_instances(b);
   for (int i = 0; i < n; ++i) {
     tti_handle *h = b->inst[i];
     const tti_config &c = h->cfg;
     const StepArgs a = handle_step_args(h);
-    const CUtensorMap *tm = static_cast<const CUtensorMap *>(h->tmaps);
     tiled::HalfArgs ha{};
     memset(&ha, 0, sizeof ha);
     ha.g = h->g;
     ha.f = a.f;
     ha.p = a.p;
-    ha.pk = packed::Packed{h->pk_cf, h->pk_vsc, h->pk_sc, h->pk_c4};
     ha.invdx = h->invdx;
     ha.invdz = h->invdz;
     ha.dt = c.dt;
-    const dim3 gr = tiled::grid(h->g, &ha.z_base);
+    const dim3 gr = tiled::grid(h->g, &ha.z_base, &ha.tile_rows);
     ha.x_base = NH;
     ha.undamped_ok = h->undamped_ok;
     ha.freesurface = c.freesurface;
@@ -135,16 +133,11 @@ int build_tables(tti_batch *b)
     all_square = all_square && ha.square;
     ha.wait_limit = h->wait_limit;
     ha.err = h->d_flag;
-    ha.nt = c.nt;
-    ha.tiles_z = (int)gr.x;
-    tiles[i] = (int)(gr.x * gr.y);
+    tiles[i] = gr;
     vel[i] = ha;
-    vel[i].map[0] = tm[2];
-    vel[i].map[1] = tm[3];
-    vel[i].map[2] = tm[4];
     str[i] = ha;
-    str[i].map[0] = tm[0];
-    str[i].map[1] = tm[1];
+    tiled::set_half(vel[i], static_cast<const CUtensorMap *>(h->tmaps), c.variant, true);
+    tiled::set_half(str[i], static_cast<const CUtensorMap *>(h->tmaps), c.variant, false);
     SourceSet s{h->nsrc, h->d_sx, h->d_sz, h->d_src, c.nt};
     BatchPost &bp = post[i];
     memset(&bp, 0, sizeof bp);
@@ -188,9 +181,15 @@ int build_tables(tti_batch *b)
     for (int i = 0; i < n; ++i)
       if (b->model_of[i] == m) mine.push_back(i);
     const int G = b->group > 0 ? b->group : (int)mine.size();
+    const unsigned gz = tiles[mine[0]].x, nt = gz * tiles[mine[0]].y;
     for (size_t g0 = 0; g0 < mine.size(); g0 += G)
-      for (int t = 0; t < tiles[mine[0]]; ++t)
-        for (size_t k = g0; k < std::min(mine.size(), g0 + G); ++k) work.push_back(tiled::Work{mine[k], t});
+      for (unsigned t = 0; t < nt; ++t)
+        for (size_t k = g0; k < std::min(mine.size(), g0 + G); ++k) {
+          const tiled::HalfArgs &a = vel[mine[k]];
+          const int z0 = a.z_base + (int)(t % gz) * a.tile_rows, x0 = a.x_base + (int)(t / gz) * walk::WX;
+          const int und = tiled::tile_undamped(a, z0, x0, walk::WX) ? tiled::Work::UNDAMPED : 0;
+          work.push_back(tiled::Work{mine[k], z0, x0 | und, b->inst[mine[k]]->cfg.nt});
+        }
   }
   if ((int)work.size() != b->nwork) return berr(b, TTI_ERR_STATE, "work table size changed");
   if (all_square != b->square && b->exec) {  // the captured launches select the kernels
@@ -212,34 +211,36 @@ int build_tables(tti_batch *b)
 }
 
 // Launch description of a half-step (`vel`: the velocity tables, else the stress ones).
-tiled::BatchLaunch batch_launch(const tti_batch *b, bool vel)
+tiled::BatchLaunch batch_launch(const tti_batch *b, bool vel, int offset)
 {
-  return tiled::BatchLaunch{vel ? b->d_vel : b->d_str, b->d_work, b->nwork, b->d_step, b->variant, b->exact,
-                            b->square, b->persistent};
+  return tiled::BatchLaunch{vel ? b->d_vel : b->d_str, b->d_work, b->nwork, b->d_step, offset, b->variant, b->exact,
+                            b->square, b->inst[0]->wait_limit, b->persistent};
 }
 
-// The launches of one time step (all instances).
-int launch_step(tti_batch *b)
+// The launches of `n` time steps of all instances: each launch adds its own
+// step's offset to the device counter, which moves on once at the end.
+int launch_steps(tti_batch *b, int n)
 {
-  const int n = (int)b->inst.size();
-  BCK(b, tiled::launch_velocity_batch(batch_launch(b, true), b->stream));
-  if (b->any_vsrc) launch_sources_batch(b->d_src, n, b->d_step, b->stream);
-  BCK(b, tiled::launch_stress_batch(batch_launch(b, false), b->stream));
-  launch_post_batch(b->d_post, n, b->max_Nx, b->d_step, b->stream);
-  launch_advance(b->d_step, b->stream);
-  BCK(b, cudaGetLastError());
+  const int ni = (int)b->inst.size();
+  for (int k = 0; k < n; ++k) {
+    BCK(b, tiled::launch_velocity_batch(batch_launch(b, true, k), b->stream));
+    if (b->any_vsrc) BCK(b, launch_sources_batch(b->d_src, ni, b->d_step, k, b->stream));
+    BCK(b, tiled::launch_stress_batch(batch_launch(b, false, k), b->stream));
+    BCK(b, launch_post_batch(b->d_post, ni, b->max_Nx, b->d_step, k, b->stream));
+  }
+  BCK(b, launch_advance(b->d_step, n, b->stream));
   return TTI_OK;
 }
 
-int launches_per_step(const tti_batch *b) { return 4 + (b->any_vsrc ? 1 : 0); }
+// kernels of launch_steps(n)
+int launches_of(const tti_batch *b, int n) { return n * (3 + (b->any_vsrc ? 1 : 0)) + 1; }
 
 int ensure_graph(tti_batch *b)
 {
   if (b->exec || b->graph_steps <= 0) return TTI_OK;
-  BCK(b, tiled::prepare_batch(batch_launch(b, true)));
+  BCK(b, tiled::prepare_batch(batch_launch(b, true, 0)));
   BCK(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = TTI_OK;
-  for (int k = 0; k < b->graph_steps && rc == TTI_OK; ++k) rc = launch_step(b);
+  const int rc = launch_steps(b, b->graph_steps);
   cudaGraph_t g = nullptr;
   const cudaError_t e = cudaStreamEndCapture(b->stream, &g);
   if (rc) {
@@ -342,8 +343,8 @@ int tti_batch_create(tti_batch **out, int nmodels, const tti_config *cfg, int ni
     return fail(TTI_ERR_CUDA, "stream/event creation failed");
   b->nwork = 0;
   for (int i = 0; i < ninst; ++i) {
-    int zb;
-    const dim3 gr = tiled::grid(b->inst[i]->g, &zb);
+    int zb, rows;
+    const dim3 gr = tiled::grid(b->inst[i]->g, &zb, &rows);
     b->nwork += (int)(gr.x * gr.y);
     b->max_nt = std::max(b->max_nt, b->inst[i]->cfg.nt);
     b->max_Nx = std::max(b->max_Nx, b->inst[i]->g.Nx);
@@ -446,12 +447,12 @@ int tti_batch_step(tti_batch *b, int nsteps)
   int left = nsteps;
   while (b->exec && left >= b->graph_steps) {
     BCK(b, cudaGraphLaunch(b->exec, b->stream));
-    b->launches += (long long)b->graph_steps * launches_per_step(b);
+    b->launches += launches_of(b, b->graph_steps);
     left -= b->graph_steps;
   }
-  for (; left > 0; --left) {
-    if ((rc = launch_step(b))) return rc;
-    b->launches += launches_per_step(b);
+  if (left > 0) {
+    if ((rc = launch_steps(b, left))) return rc;
+    b->launches += launches_of(b, left);
   }
   BCK(b, cudaEventRecord(b->ev1, b->stream));
   BCK(b, cudaEventSynchronize(b->ev1));

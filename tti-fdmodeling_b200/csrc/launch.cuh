@@ -76,8 +76,8 @@ void launch_post(const StepArgs &a, const PostArgs &p, cudaStream_t st);
 
 // ---------------- batched (many instances per launch) ----------------
 // Per-instance arguments in device memory; the time index comes from the
-// shared step counter `step` (it = step, or nt - 1 - step for mode 2), and an
-// instance whose nt has been reached does nothing.
+// shared step counter `step` plus the launch's offset (it = that, or nt - 1 -
+// that for mode 2), and an instance whose nt has been reached does nothing.
 struct BatchPost {
   Grid g;
   Fields f;
@@ -91,9 +91,9 @@ struct BatchSrc {
   const SourceTables *tab;  // device
   int variant, stype, nt, mode2;
 };
-void launch_post_batch(const BatchPost *d, int n, int maxNx, const int *step, cudaStream_t st);
-void launch_sources_batch(const BatchSrc *d, int n, const int *step, cudaStream_t st);
-void launch_advance(int *step, cudaStream_t st);
+cudaError_t launch_post_batch(const BatchPost *d, int n, int maxNx, const int *step, int offset, cudaStream_t st);
+cudaError_t launch_sources_batch(const BatchSrc *d, int n, const int *step, int offset, cudaStream_t st);
+cudaError_t launch_advance(int *step, int n, cudaStream_t st);
 // dst[f][0..n) = src[f][0..n), f < 5 (n a multiple of 4, 16-byte aligned arrays)
 // the first nf (<= 5) of the arrays src[] into dst[], n floats each, one launch
 void launch_copy5(float *const *src, float *const *dst, int nf, size_t n, cudaStream_t st);

@@ -235,21 +235,28 @@ __device__ void sources_block(const Grid &g, const Fields &f, const SourceSet &s
   }
 }
 
-__global__ void k_sources(Grid g, Fields f, SourceSet s, SourceTables t, int variant, int stype, int stage, int it)
+__global__ void k_sources(Grid g, Fields f, SourceSet s, const __grid_constant__ SourceTables t, int variant, int stype,
+                          int stage, int it)
 {
+  pdl_sync();
   sources_block(g, f, s, t, variant, stype, stage, it);
 }
 
 // Batched velocity sources: one block per instance, time index from the step counter.
-__global__ void k_sources_batch(const BatchSrc *bs, const int *step)
+__global__ void k_sources_batch(const BatchSrc *bs, const int *step, int offset)
 {
   const BatchSrc &b = bs[blockIdx.x];
-  const int n = *step;
+  pdl_sync();
+  const int n = *step + offset;
   if (n >= b.nt || b.s.n == 0) return;
   sources_block(b.g, b.f, b.s, *b.tab, b.variant, b.stype, 0, b.mode2 ? b.nt - 1 - n : n);
 }
 
-__global__ void k_advance(int *step) { ++*step; }
+__global__ void k_advance(int *step, int n)
+{
+  pdl_sync();
+  *step += n;
+}
 
 // isoelastic.c:103-144; recorded time-major on the device ([irec][trace]).
 __global__ void k_receivers(Grid g, Fields f, ReceiverSet r, int want_v, int want_p, int irec, int *flag)
@@ -408,10 +415,11 @@ __global__ void k_post(Grid g, Fields f, PostArgs p)
 }
 
 // Batched: blockIdx.y = instance; time index and receiver slot from the step counter.
-__global__ void k_post_batch(const BatchPost *bp, const int *step)
+__global__ void k_post_batch(const BatchPost *bp, const int *step, int offset)
 {
   const BatchPost &b = bp[blockIdx.y];
-  const int n = *step;
+  pdl_sync();
+  const int n = *step + offset;
   if (n >= b.nt) return;
   const int it = b.mode2 ? b.nt - 1 - n : n;
   const int irec = b.rec_on && it % b.mt == 0 ? it / b.mt : -1;
@@ -473,7 +481,7 @@ void launch_sources(const StepArgs &a, const SourceSet &s, const SourceTables *t
   if (s.n <= 0) return;
   if (stage == 0 && (stype < 2 || stype > 8)) return;
   if (stage == 1 && stype != 1) return;
-  k_sources<<<1, 128, 0, st>>>(a.g, a.f, s, *tab, a.variant, stype, stage, it);
+  launch_pdl(k_sources, dim3(1), dim3(128), 0, st, a.g, a.f, s, *tab, a.variant, stype, stage, it);
 }
 
 void launch_receivers(const StepArgs &a, const ReceiverSet &r, int seistype, int irec, int *flag, cudaStream_t st)
@@ -495,14 +503,14 @@ void launch_post(const StepArgs &a, const PostArgs &p, cudaStream_t st)
   launch_pdl(k_post, dim3((a.g.Nx + 3) / 4), dim3(128), 0, st, a.g, a.f, p);  // 4 columns (warps) per block
 }
 
-void launch_post_batch(const BatchPost *d, int n, int maxNx, const int *step, cudaStream_t st)
+cudaError_t launch_post_batch(const BatchPost *d, int n, int maxNx, const int *step, int offset, cudaStream_t st)
 {
-  if (n > 0) k_post_batch<<<dim3((maxNx + 3) / 4, n), 128, 0, st>>>(d, step);
+  return launch_pdl(k_post_batch, dim3((maxNx + 3) / 4, n), dim3(128), 0, st, d, step, offset);
 }
 
-void launch_sources_batch(const BatchSrc *d, int n, const int *step, cudaStream_t st)
+cudaError_t launch_sources_batch(const BatchSrc *d, int n, const int *step, int offset, cudaStream_t st)
 {
-  if (n > 0) k_sources_batch<<<n, 128, 0, st>>>(d, step);
+  return launch_pdl(k_sources_batch, dim3(n), dim3(128), 0, st, d, step, offset);
 }
 
 // up to five state arrays copied in one launch (the gradient's kept states)
@@ -555,7 +563,10 @@ void launch_transpose(const float *in, float *out, int nts, int n, int r0, int n
   k_transpose<<<dim3((nr + 31) / 32, (nts + 31) / 32), dim3(32, 8), 0, st>>>(in, out, nts, n, r0, nr);
 }
 
-void launch_advance(int *step, cudaStream_t st) { k_advance<<<1, 1, 0, st>>>(step); }
+cudaError_t launch_advance(int *step, int n, cudaStream_t st)
+{
+  return launch_pdl(k_advance, dim3(1), dim3(1), 0, st, step, n);
+}
 
 void launch_snapshot(const StepArgs &a, int kind, int savew, float *dst, cudaStream_t st)
 {

@@ -17,23 +17,31 @@ constexpr int NT = 512;       // threads per CTA: one row x TX/4 columns each (6
 // floats per field region in shared memory, 128-byte aligned
 constexpr int FIELD = (BX * BZ * 4 + 127) / 128 * 128 / 4;
 
+// A handle's tensor maps: the halo boxes of vx vz sxx szz
+// sxz, then the tile inputs of the stress update (HalfArgs::in).
+constexpr int HALO_MAPS = 5, IN_MAPS = 10, MAPS = HALO_MAPS + IN_MAPS;
+constexpr int AHEAD = 7;  // entries of HalfArgs::ahead
+
 struct alignas(64) HalfArgs {
-  CUtensorMap map[3];  // velocity kernel: sxx szz sxz; stress kernel: vx vz
+  CUtensorMap map[3];  // velocity update: sxx szz sxz; stress update: vx vz
+  // The stress update's own inputs. Coordinate sxx szz sxz sin cos c11 c13 c33
+  // c55; tensor txx tzz txz sin^2 cos^2 c11 c13 c33 c55 sin2theta; Bond sxx szz
+  // sxz c15 c35 c11 c13 c33 c55.
+  CUtensorMap in[IN_MAPS];
   Grid g;
   Fields f;
   Params p;
-  packed::Packed pk;
   float invdx, invdz, dt;
   int z_base;  // first tile row (multiple of 4, <= izStart)
   int x_base;  // first tile column (= 5)
+  int tile_rows;  // rows of a tile (multiple of 8, at most walk::WZ)
   int undamped_ok;
   int freesurface;
   int *err;    // bit 4: a TMA wait timed out
-  int nt;      // batched launches: time steps of this instance (its CTAs idle once the step counter reaches it)
-  int tiles_z; // batched launches: tile rows of this instance's grid
   int square;  // FMA mode with dx == dz: stencil coefficients hc fold in h = 0.5 / dx
   unsigned wait_limit;  // polls of the first TMA wait before it gives up (tma::WAIT_LIMIT)
   float hc[5]; // h * C_k
+  float nzero; // -0.0f (see walk::coefs)
   // Gradient forward pass (null: nothing kept). Velocity update, coordinate
   // rotation: per cell the stress derivative combinations the adjoint's
   // theta_v terms need (sxz_x - sxx_z, szz_x - sxz_z, sxx_x + sxz_z,
@@ -41,24 +49,45 @@ struct alignas(64) HalfArgs {
   // rotated), and for the tensor rotation the tau it starts from (kt).
   float *kd[4];
   float *kt[3];
+  // the arrays the velocity update reads per cell, for the L2 prefetch: vx vz
+  // invrho, coordinate also sin cos of theta_v, coef1, coef2
+  const float *ahead[AHEAD];
+  int nahead;
 };
+
+// Encodes a handle's MAPS tensor maps.
+bool encode_maps(CUtensorMap *map, const Grid &g, int variant, const Fields &f, const Params &p);
+// Fills map, in and ahead for the velocity or the stress update from a handle's
+// maps (f and p set).
+void set_half(HalfArgs &a, const CUtensorMap *maps, int variant, bool velocity);
 
 // Sets square / hc for FMA-mode launches on grids with dx == dz.
 inline void set_square(HalfArgs &a, bool exact)
 {
   a.square = !exact && a.invdx == a.invdz;
   for (int k = 0; k < 5; ++k) a.hc[k] = 0.5f * a.invdx * rsg(k);
+  a.nzero = -0.0f;
 }
 
-// One CTA of a batched launch: instance `inst`, tile `tile` (row tile % tiles_z, column tile / tiles_z).
-struct Work {
-  int inst, tile;
+// One item of a batched launch: instance, tile origin (x0 with the UNDAMPED
+// bit: tile_undamped), the instance's time steps.
+struct alignas(16) Work {
+  static constexpr int UNDAMPED = 1 << 30;
+  int inst, z0, x0, nt;
 };
 
+// true when every cell of the tile of WX columns lies where coef1 = 1 and coef2 = dt
+__host__ __device__ __forceinline__ bool tile_undamped(const HalfArgs &a, int z0, int x0, int wx)
+{
+  const Grid &g = a.g;
+  return a.undamped_ok && x0 >= g.E && x0 + wx <= g.Nx - g.E && z0 >= (a.freesurface ? 0 : g.E) &&
+         z0 + a.tile_rows <= g.Nz - g.E;
+}
+
 // Encodes the 2D tensor map of one [Nx][ldz] field for the halo box.
-bool encode_map(CUtensorMap *map, const Grid &g, float *field);
-// Tile grid; *z_base receives the first tile row.
-dim3 grid(const Grid &g, int *z_base);
+bool encode_map(CUtensorMap *map, const Grid &g, float *field, int box_rows = BZ, int box_cols = BX);
+// Tile grid; *z_base receives the first tile row, *tile_rows the height of a tile.
+dim3 grid(const Grid &g, int *z_base, int *tile_rows);
 cudaError_t launch_velocity(const HalfArgs &a, int variant, bool exact, cudaStream_t st);
 cudaError_t launch_stress(const HalfArgs &a, int variant, bool exact, cudaStream_t st);
 // Batched: one launch over all instances' tiles (each instance's arguments
@@ -68,8 +97,10 @@ struct BatchLaunch {
   const Work *work;      // device: the CTA -> (instance, tile) table
   int nwork;
   const int *step;       // device: the shared step counter
+  int offset;            // this launch's step: the counter plus offset
   int variant;
   bool exact, square;    // square: every instance has folded coefficients (set_square)
+  unsigned wait_limit;   // polls of a box wait before it gives up
   bool persistent;       // one resident wave of CTAs walks the table (else one CTA per item)
 };
 cudaError_t launch_velocity_batch(const BatchLaunch &l, cudaStream_t st);

@@ -149,7 +149,7 @@ struct tti_handle {
   float *m_eps = nullptr, *m_delta = nullptr;  // epsilon, delta as uploaded (gradient chain rule)
   float *m_theta = nullptr;                    // theta (degrees) as uploaded (Bond gradient chain rule)
   struct GradState *grad = nullptr;            // adjoint-state gradient buffers (adjoint.cu)
-  void *tmaps = nullptr;   // host copy of the 5 tensor maps (vx vz sxx szz sxz), 64-byte aligned
+  void *tmaps = nullptr;   // host copy of the tensor maps (tiled::encode_maps), 64-byte aligned
   int undamped_ok = 0;  // coef1 == 1, coef2 == dt outside the absorbing rims (checked at upload)
   int *d_rcol[3] = {}, *d_rzs[3] = {}, *d_rid[3] = {};  // receivers grouped by column
   float2 *pk_cf = nullptr, *pk_vsc = nullptr, *pk_sc = nullptr;  // packed parameters (pack.cuh)
