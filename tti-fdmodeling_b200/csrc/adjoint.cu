@@ -31,7 +31,7 @@
 #include <mutex>
 #include <vector>
 
-#include "tiled.cuh"
+#include "walk.cuh"
 
 using namespace ttifd;
 
@@ -39,7 +39,8 @@ struct GradState {
   int ncheck = 0, seg = 0;  // checkpoints, steps per segment
   float *lam[8] = {};       // adjoint vx vz sxx szz sxz (+ txx tzz txz: tensor rotation)
   float *T[4] = {};         // stress-half adjoint strain terms (read by the transposed stress stencils)
-  float *TV[6] = {};        // velocity-half adjoint derivative terms (read by the transposed velocity stencils)
+  float *TV[6] = {};        // velocity-half adjoint derivative terms (read by the transposed velocity stencils):
+                            // per-cell path 6, tiled path 4 (coordinate: cos Fx, sin Fx, cos Fz, sin Fz) or 2 (Fx, Fz)
   float *acc[7] = {};       // sums. coordinate: c11 c13 c33 (c55 kept zero) theta(stress node) sin_v cos_v;
                             // Bond: c11 c13 c33 c55 c15 c35 (the rotated moduli)
   float *out[4] = {};       // vp eps delta theta
@@ -52,7 +53,7 @@ struct GradState {
   int gsrc_n = 0;
   double *d_J = nullptr;
   bool have_obs[3] = {};
-  CUtensorMap *maps = nullptr;  // host copies, 64-byte aligned: T0..T3, TV0..TV5
+  CUtensorMap *maps = nullptr;  // host copies, 64-byte aligned: T0..T3, TV0..TV3, the kept steps, 7 parameters
   // velocity sources (stype 2-8): per source vm cells (ix, iz, index in the
   // rim list or -1; ix < 0: off the grid) with weights (wx, wz),
   // v[cell] += w src(t); the cells of all windows outside the velocity update,
@@ -62,8 +63,8 @@ struct GradState {
   int2 *vrim = nullptr;
   double *vrim_acc = nullptr;
   int vm = 0, vrim_n = 0;
-  int surf_zorg = -1;  // row origin of the stress-half adjoint that folds in the column work; -1: a separate launch
-  int surf_zend = 0;   // rows at or below this hold no column work
+  bool surf_merged = false;  // the column work runs inside the stress-half adjoint (else a separate launch)
+  int surf_zend = 0;         // rows at or below this hold no column work
 };
 
 namespace {
@@ -73,65 +74,14 @@ constexpr int BZ = 32, BX = 8;
 struct AdjArgs {
   Grid g;
   Params p;
-  packed::Packed pk;  // packed parameters (null on the per-cell path)
   float *lam[8];
   float *T[4];
   float *TV[6];
   float *acc[7];
   const float *keep[8];  // this step's kept fields (keep_fields), null past them
   float hx, hz, dt;
-  int z_lo;         // first row of the transposed velocity stencils
-  int undamped_ok;  // coef1 == 1, coef2 == dt on [E, Nx - E) x [und_z0, Nz - E) (checked at upload)
-  int und_z0;
+  int z_lo;  // first row of the transposed velocity stencils
 };
-
-__device__ __forceinline__ bool cell_undamped(const AdjArgs &a, int ix, int iz)
-{
-  const Grid &g = a.g;
-  return a.undamped_ok && ix >= g.E && ix < g.Nx - g.E && iz >= a.und_z0 && iz < g.Nz - g.E;
-}
-
-// Stress-node parameters of one cell: coef1, coef2 (the constants 1 and dt in
-// the undamped interior), c11 c13 c33 c55, and the formulation's pair
-// (coordinate: sin, cos theta; tensor: sin^2, cos^2; Bond: c15, c35), from the
-// packed arrays (PK) or the plain ones.
-struct SParams {
-  float c1, b, c11, c13, c33, c55, p, q;
-};
-template <bool PK, int V>
-__device__ __forceinline__ SParams stress_params(const AdjArgs &a, size_t i, bool und)
-{
-  SParams s;
-  if (und) {
-    s.c1 = 1.0f;
-    s.b = a.dt;
-  } else if (PK) {
-    const float2 cf = __ldg(a.pk.cf + i);
-    s.c1 = cf.x;
-    s.b = cf.y;
-  } else {
-    s.c1 = a.p.coef1[i];
-    s.b = a.p.coef2[i];
-  }
-  if (PK) {
-    const float4 c4 = __ldg(a.pk.c4 + i);
-    const float2 sc = __ldg(a.pk.sc + i);
-    s.c11 = c4.x;
-    s.c13 = c4.y;
-    s.c33 = c4.z;
-    s.c55 = c4.w;
-    s.p = sc.x;
-    s.q = sc.y;
-  } else {
-    s.c11 = a.p.c11[i];
-    s.c13 = a.p.c13[i];
-    s.c33 = a.p.c33[i];
-    s.c55 = a.p.c55[i];
-    s.p = V == TTI_BOND ? a.p.c15[i] : V == TTI_TENSOR ? a.p.s2[i] : a.p.sn[i];
-    s.q = V == TTI_BOND ? a.p.c35[i] : V == TTI_TENSOR ? a.p.c2[i] : a.p.cs[i];
-  }
-  return s;
-}
 
 __device__ __forceinline__ void pair_v(const float *a, size_t L, int ix, int iz, float &d1, float &d2)
 {
@@ -367,47 +317,25 @@ __device__ __forceinline__ void store_T(const AdjArgs &a, size_t i, float t0, fl
   a.T[3][i] = a.hx * t2 - a.hz * t3;
 }
 
-// stress-half adjoint, local part: gradient sums, T0..T3, lambda_sigma *= coef1.
-// PK (tiled path): packed parameters, and the strain rates the forward stress
-// kernel kept (keep[0..3], tensor tau keep[4..6]); otherwise the stencils of
-// the kept v (keep[0..1], tensor tau keep[2..4]). Block rows start at z_org.
-// SURF: each warp (one column, 32 rows) first does the column work of its
-// rows (surface_warp): the residual injection, the source gradient and, in the
-// block whose rows hold izStart - 5 .. izStart + 5, the free-surface adjoint.
-// That is all of it when z_org is at or above every receiver row, source
-// window row and image row; the host checks this. Blocks from row z_end down
-// have no column work and skip it.
-template <int V, bool PK, bool SURF>
-__global__ void __launch_bounds__(BZ *BX) k_adj_stress_local(AdjArgs a, SurfaceArgs sa, int z_org, int z_end)
+// stress-half adjoint, local part, one cell per thread: gradient sums, T0..T3,
+// lambda_sigma *= coef1, from the stencils of the kept v (keep[0..1], tensor
+// tau keep[2..4]).
+template <int V>
+__global__ void __launch_bounds__(BZ *BX) k_adj_stress_local(AdjArgs a)
 {
-  pdl_sync();
   const Grid &g = a.g;
-  const int r0 = z_org + blockIdx.x * BZ;
-  const int iz = r0 + threadIdx.x, ix = blockIdx.y * BX + threadIdx.y;
-  if (SURF && ix < g.Nx && r0 < z_end) surface_warp(sa, ix, r0, r0 + BZ, threadIdx.x);
+  const int iz = blockIdx.x * BZ + threadIdx.x, ix = blockIdx.y * BX + threadIdx.y;
   if (!interior(g, ix, iz)) return;
   const size_t L = g.ldz, i = (size_t)ix * L + iz;
-  const SParams m = stress_params<PK, V>(a, i, cell_undamped(a, ix, iz));
-  const float la = a.lam[2][i], lb = a.lam[3][i], le = a.lam[4][i], b = m.b, c1 = m.c1;
-  const float c11 = m.c11, c13 = m.c13, c33 = m.c33, c55 = m.c55;
-  float vxx, vxz, vzx, vzz;
-  if (PK) {
-    vxx = a.keep[0][i];
-    vxz = a.keep[1][i];
-    vzx = a.keep[2][i];
-    vzz = a.keep[3][i];
-  } else {
-    float a1, a2, b1, b2;
-    pair_s(a.keep[0], L, ix, iz, a1, a2);
-    pair_s(a.keep[1], L, ix, iz, b1, b2);
-    vxx = a.hx * (a1 + a2);
-    vxz = a.hz * (a1 - a2);
-    vzx = a.hx * (b1 + b2);
-    vzz = a.hz * (b1 - b2);
-  }
-  const float *const *tau = a.keep + (PK ? 4 : 2);
+  const float la = a.lam[2][i], lb = a.lam[3][i], le = a.lam[4][i], b = a.p.coef2[i], c1 = a.p.coef1[i];
+  const float c11 = a.p.c11[i], c13 = a.p.c13[i], c33 = a.p.c33[i], c55 = a.p.c55[i];
+  float a1, a2, b1, b2;
+  pair_s(a.keep[0], L, ix, iz, a1, a2);
+  pair_s(a.keep[1], L, ix, iz, b1, b2);
+  const float vxx = a.hx * (a1 + a2), vxz = a.hz * (a1 - a2), vzx = a.hx * (b1 + b2), vzz = a.hz * (b1 - b2);
+  const float *const *tau = a.keep + 2;
   if (V == TTI_BOND) {  // sigma += coef2 H (vxx, vzz, vzx + vxz), H symmetric with c15, c35 (bond:836-873)
-    const float c15 = m.p, c35 = m.q, sh = vzx + vxz;
+    const float c15 = a.p.c15[i], c35 = a.p.c35[i], sh = vzx + vxz;
     a.acc[0][i] += b * la * vxx;
     a.acc[1][i] += b * (la * vzz + lb * vxx);
     a.acc[2][i] += b * lb * vzz;
@@ -424,7 +352,7 @@ __global__ void __launch_bounds__(BZ *BX) k_adj_stress_local(AdjArgs a, SurfaceA
   if (V == TTI_TENSOR) {
     // forward (tensor:826-851): n = coef1 tau + coef2 H e(theta, v); tau' = n; sigma' = R(theta) n,
     // with tau the kept one from before the stress half.
-    const float s2 = m.p, c2 = m.q, st = a.p.s2t[i], cd = c2 - s2, sh = vxz + vzx;
+    const float s2 = a.p.s2[i], c2 = a.p.c2[i], st = a.p.s2t[i], cd = c2 - s2, sh = vxz + vzx;
     const float exx = c2 * vxx + s2 * vzz - 0.5f * st * sh, ezz = s2 * vxx + c2 * vzz + 0.5f * st * sh;
     const float exz = st * (vxx - vzz) + cd * sh;
     const float nxx = c1 * tau[0][i] + b * (c11 * exx + c13 * ezz);
@@ -452,7 +380,7 @@ __global__ void __launch_bounds__(BZ *BX) k_adj_stress_local(AdjArgs a, SurfaceA
     a.lam[2][i] = a.lam[3][i] = a.lam[4][i] = 0.0f;  // sigma is overwritten by R tau
     return;
   }
-  const float s = m.p, co = m.q;
+  const float s = a.p.sn[i], co = a.p.cs[i];
   const float rxx = co * vxx - s * vxz, rxz = s * vxx + co * vxz;
   const float rzx = co * vzx - s * vzz, rzz = s * vzx + co * vzz;
   a.acc[0][i] += b * la * rxx;
@@ -537,274 +465,458 @@ __global__ void __launch_bounds__(BZ *BX) k_adj_velocity_stencil(AdjArgs a)
 }
 
 // ---------------------------------------------------------------- tiled adjoint
-// The two stencil passes of the adjoint on the forward path's 128 x 16 tiles:
-// every stencil tap comes from a TMA halo box in shared memory (one 2D copy per
-// field, the box origin rounded down to a 16-byte boundary, zeros outside the
-// array), per-cell parameters from the packed arrays.
+// A reverse step is two kernels over the forward path's tiles (walk.cuh):
+//
+//  k_adj_stress    the transposed velocity stencils of the step after it into
+//                  lambda_sigma, then this step's column work (surface_warp)
+//                  and the local stress-half adjoint at the same cells
+//  k_adj_velocity_walk
+//                  the transposed stress stencils into lambda_v, then the
+//                  velocity-half adjoint at the same cells
+//
+// lambda_sigma thus goes from one step's stencils to the next step's local
+// part in registers. The stencils are linear, so the velocity-half adjoint
+// leaves the factors of its derivative terms instead of the six terms: with
+// A = cos Fx, B = sin Fx, C = cos Fz, D = sin Fz (theta at the velocity node)
+//   lambda_sxx -= hx ((d1 + d2)(A) - (d1 - d2)(B))
+//   lambda_szz -= hx (d1 + d2)(D) + hz (d1 - d2)(C)
+//   lambda_sxz -= hx ((d1 + d2)(B) + (d1 + d2)(C)) + hz ((d1 - d2)(A) - (d1 - d2)(D))
+// and without a rotation at the velocity node (tensor, Bond) A = Fx, C = Fz,
+// B = D = 0: two boxes.
+//
+// Both are bound by memory latency and throughput: the first moves 128 bytes a
+// cell (coordinate), the second 92, 5 TB/s through L2 at 600 x 1200. What they
+// read per cell is requested before anything is waited for: halo boxes, kept
+// fields and moduli by TMA, lambda and the gradient sums into registers, which
+// sets the CTAs per SM (two of 128 registers; three of 80 spill and take 71
+// against 69 us a step at 600 x 1200, 352 against 272 in the tensor rotation at
+// 1126 x 3000). Loading them after the walks from lines prefetched into L2 took
+// 83 and 305. One reverse step: 600 x 1200 about 46 us (three kernels with a
+// cell per thread and the six terms: 63), 1126 x 3000 160 (237).
+using walk::F4;
+using walk::ld4;
+using walk::ldg4;
+using walk::st4;
+using walk::WX;
+
 struct alignas(64) AdjTile {
-  CUtensorMap map[6];  // velocity pass: T0..T3; stress-node pass: TV0..TV5
+  CUtensorMap map[4];  // stress: A B C D or Fx Fz; velocity: T0..T3
+  CUtensorMap kept;    // the kept steps as one [steps x fields][Nx][ldz] array
+  CUtensorMap par[7];  // stress: c11 c13 c33 c55, then sin cos / sin^2 cos^2 sin2theta / c15 c35
   AdjArgs a;
-  packed::Packed pk;
-  int z_base;  // first tile row (multiple of 4)
-  int *err;    // bit 4: a TMA wait timed out
+  int kept0;           // this step's first field in `kept`
+  int z_base, rows;    // first tile row (multiple of 8), rows of a tile
+  int undamped_ok, und_z0;  // coef1 == 1, coef2 == dt on [E, Nx - E) x [und_z0, Nz - E) (checked at upload)
+  int surf_zend;       // rows at or below this hold no column work
+  float nzero;         // -0.0f
+  int *err;            // bit 4: a TMA wait timed out
 };
 
+constexpr int stress_boxes(int V) { return V == TTI_COORDINATE ? 4 : 2; }
+constexpr int stress_kept(int V) { return V == TTI_TENSOR ? 7 : 4; }   // strain rates, tensor tau
+constexpr int stress_par(int V) { return V == TTI_TENSOR ? 7 : 6; }
+constexpr int velocity_kept(int V) { return V == TTI_COORDINATE ? 4 : 0; }  // P Q R S
+constexpr int kept_off(int boxes) { return walk::LEAD + boxes * walk::BOX; }
+constexpr int adj_bar(int boxes, int kept) { return kept_off(boxes) + kept * walk::WZ * WX; }
+constexpr size_t adj_smem(int boxes, int kept) { return (size_t)(adj_bar(boxes, kept) + 16) * sizeof(float); }
+
 struct TileCells {
-  int x0, z0, xc, z;
+  int x0, z0, x, z;
+  bool on;  // some of the thread's rows lie in [lo, Nz - NH)
 };
-__device__ __forceinline__ TileCells tile_cells(int z_base)
+__device__ __forceinline__ TileCells tile_cells(const AdjTile &at, int lo)
 {
   TileCells c;
-  c.z0 = z_base + blockIdx.x * tiled::TZ;
-  c.x0 = NH + blockIdx.y * tiled::TX;
-  c.xc = c.x0 + (tiled::TX / 4) * (threadIdx.x >> 7);
-  c.z = c.z0 + (threadIdx.x & 127);
+  c.z0 = at.z_base + blockIdx.x * at.rows;
+  c.x0 = NH + blockIdx.y * WX;
+  c.x = c.x0 + (threadIdx.x >> 5);
+  c.z = c.z0 + 4 * (threadIdx.x & 31);
+  c.on = c.x < at.a.g.Nx - NH && 4 * (int)(threadIdx.x & 31) < at.rows && c.z + 3 >= lo && c.z < at.a.g.Nz - NH;
   return c;
 }
 
-// stress-node pair of shared field q centred on (x, z): q[m * BZ + n] = value at (x + m, z + n)
-__device__ __forceinline__ void spair(const float *q, float &d1, float &d2)
+__device__ __forceinline__ bool adj_undamped(const AdjTile &at, const TileCells &c)
 {
-  constexpr int B = tiled::BZ;
-  float s1 = rsg(0) * (q[0] - q[-B - 1]), s2 = rsg(0) * (q[-1] - q[-B]);
-#pragma unroll
-  for (int k = 2; k <= NH; ++k) {
-    s1 += rsg(k - 1) * (q[(k - 1) * B + k - 1] - q[-k * B - k]);
-    s2 += rsg(k - 1) * (q[(k - 1) * B - k] - q[-k * B + k - 1]);
+  const Grid &g = at.a.g;
+  return at.undamped_ok && c.x0 >= g.E && c.x0 + WX <= g.Nx - g.E && c.z0 >= at.und_z0 && c.z0 + at.rows <= g.Nz - g.E;
+}
+
+// The tile's copies: nb halo boxes and the kept fields k0 .. k0 + nk - 1 of
+// this step; one thread.
+__device__ __forceinline__ void issue_adj(const AdjTile &at, float *sm, unsigned long long *bar, int nb, int xoff, int k0,
+                                          int nk, int np, const TileCells &c)
+{
+  if (threadIdx.x != 0) return;
+  tiled::tma::mbar_arrive_expect_tx(bar, (nb * walk::WBX * walk::WB + (nk + np) * at.rows * WX) * 4);
+  for (int f = 0; f < nb; ++f)
+    tiled::tma::tma_load_2d(sm + walk::LEAD + f * walk::BOX, at.map + f, c.z0 - 8, c.x0 - xoff, bar);
+  for (int k = 0; k < nk; ++k)
+    tiled::tma::tma_load_3d(sm + kept_off(nb) + k * at.rows * WX, &at.kept, c.z0, c.x0, at.kept0 + k0 + k, bar);
+  for (int k = 0; k < np; ++k)
+    tiled::tma::tma_load_2d(sm + kept_off(nb) + (nk + k) * at.rows * WX, at.par + k, c.z0, c.x0, bar);
+}
+
+__device__ __forceinline__ void adj_coefs(const AdjTile &at, bool und, size_t i, F4 &c1, F4 &c2)
+{
+  if (und) {
+    c1.p[0] = c1.p[1] = walk::pack2(1.0f, 1.0f);
+    c2.p[0] = c2.p[1] = walk::pack2(at.a.dt, at.a.dt);
+  } else {
+    c1 = ldg4(at.a.p.coef1 + i);
+    c2 = ldg4(at.a.p.coef2 + i);
   }
-  d1 = s1;
-  d2 = s2;
 }
 
-// one diagonal of the velocity-node pair of shared field q centred on (x, z)
-__device__ __forceinline__ float vdiag1(const float *q)
+// Walks of NB boxes, two at a time (d1 of box PAIR ? 2p : f, d2 of box PAIR ?
+// 2p + 1 : f), whose sums take the boxes' place: PAIR: arrays 2p, 2p + 1 are
+// d1 of box 2p and d2 of box 2p + 1, one walk for both; else arrays 2f, 2f + 1
+// are d1 and d2 of box f.
+template <int O, int NB, bool PAIR>
+__device__ __forceinline__ void adj_walks(const AdjTile &at, const walk::Coefs &k, float *sm)
 {
-  constexpr int B = tiled::BZ;
-  float s = rsg(0) * (q[B + 1] - q[0]);
+  static_assert(4 * walk::SUM <= 2 * walk::BOX, "the sums fit in place of the boxes");
+  const int gr = walk::groups(at.rows), t = threadIdx.x >> 5, q = t >= gr;
+  const int d = (t - q * gr) * 32 + (threadIdx.x & 31);
+  const bool on = t < 2 * gr && d < at.rows + WX - 1;
+  float *boxes = sm + walk::LEAD;
+  walk::u64 out[WX];
 #pragma unroll
-  for (int k = 2; k <= NH; ++k) s += rsg(k - 1) * (q[k * B + k] - q[(1 - k) * B + 1 - k]);
-  return s;
+  for (int p = 0; p < (PAIR ? NB / 4 : NB / 2); ++p) {
+    const int f = 2 * p + q;  // the walk's box (PAIR: its pair of boxes)
+    const float *ba = boxes + (PAIR ? 2 * f : f) * walk::BOX, *bb = PAIR ? ba + walk::BOX : ba;
+    if (on) walk::diagonals<O, false>(ba, bb, d, k, out);
+    __syncthreads();  // these boxes have been read
+    // p's four sum arrays fit in the boxes just read
+    float *o = boxes + p * (PAIR ? 4 : 2) * walk::BOX + q * 2 * walk::SUM;
+    if (on) walk::put_sums(o, o + walk::SUM, d, out);
+  }
+  __syncthreads();  // the sums are complete
 }
-__device__ __forceinline__ float vdiag2(const float *q)
+// d1 and d2 of the q-th walk of step p of adj_walks at a thread's rows
+template <bool PAIR>
+__device__ __forceinline__ void adj_sums(const float *sm, const TileCells &c, int w, F4 &d1, F4 &d2)
 {
-  constexpr int B = tiled::BZ;
-  float s = rsg(0) * (q[B] - q[1]);
-#pragma unroll
-  for (int k = 2; k <= NH; ++k) s += rsg(k - 1) * (q[k * B + 1 - k] - q[(1 - k) * B + k]);
-  return s;
+  const float *o = sm + walk::LEAD + (w >> 1) * (PAIR ? 4 : 2) * walk::BOX + (w & 1) * 2 * walk::SUM;
+  d1 = ld4(o + walk::d1_at(c.x - c.x0, c.z - c.z0));
+  d2 = ld4(o + walk::SUM + walk::d2_at(c.x - c.x0, c.z - c.z0));
 }
 
-// While the halo boxes are in flight, the lanes of each warp ask L2 for the
-// per-cell lines the velocity-half adjoint reads after the wait (coef1/coef2,
-// invrho; coordinate also sin/cos theta_v, the kept P Q R S and the two theta_v
-// sums): one 128-byte line per column and array, two for the float2 arrays.
+typedef walk::Rows<false> R;
+__device__ __forceinline__ float at4(const F4 &f, int i) { return R::get(f, i); }
+
+// A thread's inputs of the local stress-half adjoint that come from global memory.
 template <int V>
-__device__ __forceinline__ void prefetch_adj_velocity(const AdjTile &at, const TileCells &c)
+struct LocalIn {
+  static constexpr int NA = V == TTI_BOND ? 6 : 5;  // gradient sums (coordinate: the fourth unused)
+  F4 c1, b, m[3], acc[NA];
+};
+template <int V>
+__device__ __forceinline__ void load_local(const AdjTile &at, bool und, size_t i, LocalIn<V> &n)
 {
-  constexpr int SLOTS = V == TTI_COORDINATE ? 11 : 3;
   const AdjArgs &a = at.a;
-  const int lane = threadIdx.x & 31, z = c.z - lane;  // the warp's first row
-  if (z >= a.g.Nz - NH) return;
-  for (int q = lane; q < (tiled::TX / 4) * SLOTS; q += 32) {
-    const int col = q / SLOTS, k = q % SLOTS, x = c.xc + col;
-    if (x >= a.g.Nx - NH) continue;
-    const size_t i = (size_t)x * a.g.ldz + z;
-    const void *p;
-    if (k < 2) p = at.pk.cf + i + 16 * k;
-    else if (k == 2) p = a.p.invrho + i;
-    else if (k < 5) p = at.pk.vsc + i + 16 * (k - 3);
-    else if (k < 9) p = a.keep[4 + (k - 5)] + i;
-    else p = a.acc[5 + (k - 9)] + i;
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+  adj_coefs(at, und, i, n.c1, n.b);
+  if (V == TTI_TENSOR) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) n.m[k] = ld4(a.lam[5 + k] + i);
   }
+#pragma unroll
+  for (int k = 0; k < LocalIn<V>::NA; ++k)
+    if (!(V == TTI_COORDINATE && k == 3)) n.acc[k] = ld4(a.acc[k] + i);
 }
 
-// transposed stress stencils into lambda_v, then the velocity-half adjoint
-// (maps: T0..T3; coordinate: the theta_v terms from the kept stress
-// derivative combinations P Q R S that the forward velocity kernel wrote)
+// The local stress-half adjoint of a thread's rows: gradient sums, T0..T3 and
+// lambda_sigma *= coef1 (tensor: lambda_tau, lambda_sigma zeroed), from the
+// strain rates (tensor: and tau) the forward stress kernel kept.
 template <int V>
-__global__ void __launch_bounds__(tiled::NT, 3) k_adj_velocity_tiled(const __grid_constant__ AdjTile at)
+__device__ __forceinline__ void stress_local(const AdjTile &at, const TileCells &c, size_t i, F4 (&l)[3], LocalIn<V> &n,
+                                             const float *kept, bool store_zero)
 {
-  pdl_sync();
-  constexpr int F = tiled::FIELD, B = tiled::BZ;
+  const AdjArgs &a = at.a;
+  const int lo = a.g.izStart, hi = min(a.g.Nz - NH, c.z0 + at.rows);
+  auto keep = [&](int k) { return ld4(kept + (k * WX + c.x - c.x0) * at.rows + (c.z - c.z0)); };
+  const F4 k0 = keep(0), k1 = keep(1), k2 = keep(2), k3 = keep(3);
+  constexpr int NK = stress_kept(V);
+  const F4 &c1 = n.c1, &b = n.b;
+  const F4 c11 = keep(NK), c13 = keep(NK + 1), c33 = keep(NK + 2), c55 = keep(NK + 3), p4 = keep(NK + 4), q4 = keep(NK + 5);
+  F4 t[4];
+  constexpr int NA = LocalIn<V>::NA;
+  auto add = [&](int k, int q, float v) { R::set(n.acc[k], q, at4(n.acc[k], q) + v); };
+  auto set_T = [&](int q, float t0, float t1, float t2, float t3) {
+    R::set(t[0], q, a.hx * t0 + a.hz * t1);
+    R::set(t[1], q, a.hx * t0 - a.hz * t1);
+    R::set(t[2], q, a.hx * t2 + a.hz * t3);
+    R::set(t[3], q, a.hx * t2 - a.hz * t3);
+  };
+  if (V == TTI_TENSOR) {
+    // forward (tensor:826-851): n = coef1 tau + coef2 H e(theta, v); tau' = n; sigma' = R(theta) n,
+    // with tau the kept one from before the stress half.
+    const F4 &s24 = p4, &c24 = q4, st4_ = keep(NK + 6);
+    F4 (&m)[3] = n.m;
+    const F4 t5 = keep(4), t6 = keep(5), t7 = keep(6);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float vxx = at4(k0, q), vxz = at4(k1, q), vzx = at4(k2, q), vzz = at4(k3, q);
+      const float la = at4(l[0], q), lb = at4(l[1], q), le = at4(l[2], q), bq = at4(b, q), cq = at4(c1, q);
+      const float m11 = at4(c11, q), m13 = at4(c13, q), m33 = at4(c33, q), m55 = at4(c55, q);
+      const float s2 = at4(s24, q), c2 = at4(c24, q), st = at4(st4_, q), cd = c2 - s2, sh = vxz + vzx;
+      const float exx = c2 * vxx + s2 * vzz - 0.5f * st * sh, ezz = s2 * vxx + c2 * vzz + 0.5f * st * sh;
+      const float exz = st * (vxx - vzz) + cd * sh;
+      const float nxx = cq * at4(t5, q) + bq * (m11 * exx + m13 * ezz);
+      const float nzz = cq * at4(t6, q) + bq * (m13 * exx + m33 * ezz);
+      const float nxz = cq * at4(t7, q) + bq * m55 * exz;
+      // lambda_n = lambda_tau' + R^T lambda_sigma'
+      const float lxx = at4(m[0], q) + c2 * la + s2 * lb - 0.5f * st * le;
+      const float lzz = at4(m[1], q) + s2 * la + c2 * lb + 0.5f * st * le;
+      const float lxz = at4(m[2], q) + st * la - st * lb + cd * le;
+      add(0, q, bq * lxx * exx);
+      add(1, q, bq * (lxx * ezz + lzz * exx));
+      add(2, q, bq * lzz * ezz);
+      add(3, q, bq * lxz * exz);
+      // theta: through the strain rotation (d s2 = st, d c2 = -st, d st = 2 cd) and through R
+      const float dexx = st * (vzz - vxx) - cd * sh, dexz = 2.0f * cd * (vxx - vzz) - 2.0f * st * sh;
+      const float rxx_ = -st * nxx + st * nzz + 2.0f * cd * nxz, rxz_ = -cd * (nxx - nzz) - 2.0f * st * nxz;
+      add(4, q,
+          lxx * bq * (m11 - m13) * dexx + lzz * bq * (m13 - m33) * dexx + lxz * bq * m55 * dexz + (la - lb) * rxx_ +
+              le * rxz_);
+      const float Lexx = bq * (m11 * lxx + m13 * lzz), Lezz = bq * (m13 * lxx + m33 * lzz), Lexz = bq * m55 * lxz;
+      const float Lsh = 0.5f * st * (Lezz - Lexx) + cd * Lexz;
+      set_T(q, c2 * Lexx + s2 * Lezz + st * Lexz, Lsh, Lsh, s2 * Lexx + c2 * Lezz - st * Lexz);
+      R::set(m[0], q, cq * lxx);
+      R::set(m[1], q, cq * lzz);
+      R::set(m[2], q, cq * lxz);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) st4(a.lam[5 + k] + i, m[k], c.z, lo, hi);
+    l[0].p[0] = l[0].p[1] = walk::pack2(0.0f, 0.0f);  // sigma is overwritten by R tau
+    if (store_zero)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) st4(a.lam[2 + k] + i, l[0], c.z, lo, hi);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float vxx = at4(k0, q), vxz = at4(k1, q), vzx = at4(k2, q), vzz = at4(k3, q);
+      const float la = at4(l[0], q), lb = at4(l[1], q), le = at4(l[2], q), bq = at4(b, q), cq = at4(c1, q);
+      const float m11 = at4(c11, q), m13 = at4(c13, q), m33 = at4(c33, q), m55 = at4(c55, q);
+      if (V == TTI_BOND) {  // sigma += coef2 H (vxx, vzz, vzx + vxz), H symmetric with c15, c35 (bond:836-873)
+        const float c15 = at4(p4, q), c35 = at4(q4, q), sh = vzx + vxz;
+        add(0, q, bq * la * vxx);
+        add(1, q, bq * (la * vzz + lb * vxx));
+        add(2, q, bq * lb * vzz);
+        add(3, q, bq * le * sh);
+        add(4, q, bq * (la * sh + le * vxx));
+        add(NA - 1, q, bq * (lb * sh + le * vzz));
+        const float Lsh = bq * (c15 * la + c35 * lb + m55 * le);
+        set_T(q, bq * (m11 * la + m13 * lb + c15 * le), Lsh, Lsh, bq * (m13 * la + m33 * lb + c35 * le));
+      } else {
+        const float s = at4(p4, q), co = at4(q4, q);
+        const float rxx = co * vxx - s * vxz, rxz = s * vxx + co * vxz;
+        const float rzx = co * vzx - s * vzz, rzz = s * vzx + co * vzz;
+        add(0, q, bq * la * rxx);
+        add(1, q, bq * (la * rzz + lb * rxx));
+        add(2, q, bq * lb * rzz);
+        add(4, q, bq * (la * (m13 * rzx - m11 * rxz) + lb * (m33 * rzx - m13 * rxz) + le * m55 * (rxx - rzz)));
+        const float Lxx = bq * (m11 * la + m13 * lb), Lzz = bq * (m13 * la + m33 * lb), Lq = bq * m55 * le;
+        set_T(q, co * Lxx + s * Lq, co * Lq - s * Lxx, co * Lq + s * Lzz, co * Lzz - s * Lq);
+      }
+      R::set(l[0], q, cq * la);
+      R::set(l[1], q, cq * lb);
+      R::set(l[2], q, cq * le);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) st4(a.lam[2 + k] + i, l[k], c.z, lo, hi);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) st4(a.T[k] + i, t[k], c.z, lo, hi);
+#pragma unroll
+  for (int k = 0; k < NA; ++k)
+    if (!(V == TTI_COORDINATE && k == 3)) st4(a.acc[k] + i, n.acc[k], c.z, lo, hi);
+}
+
+// MODE 0: stencils, column work, local part. Where the column work reaches
+// cells outside the tiles, three launches instead: MODE 1 (stencils only),
+// k_adj_surface, MODE 2 (local part only).
+// One warp holds one column of the tile, so a tile with column work (rows
+// above surf_zend) stores lambda_sigma, does its columns' work warp by warp on
+// global memory, and reads it back.
+template <int V, int MODE>
+__global__ void __launch_bounds__(walk::NT, 2) k_adj_stress(const __grid_constant__ AdjTile at,
+                                                            const __grid_constant__ SurfaceArgs sa)
+{
+  constexpr int NB = MODE == 2 ? 0 : stress_boxes(V), NK = MODE == 1 ? 0 : stress_kept(V);
+  constexpr int NP = MODE == 1 ? 0 : stress_par(V);
   extern __shared__ __align__(128) float sm[];
-  unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + 4 * F);
+  unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + adj_bar(NB, NK + NP));
   const AdjArgs &a = at.a;
   const Grid &g = a.g;
-  const TileCells c = tile_cells(at.z_base);
-  tiled::tma::issue_tiles(at.map, sm, bar, 4, c.z0, c.x0, 4);
-  const int z = c.z;
-  const bool zin = z >= g.izStart && z < g.Nz - NH;
-  // this row's lambda_v, loaded while the halo boxes are in flight
-  constexpr int NJ = tiled::TX / 4;
-  float l[NJ][2];
-#pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    const int x = c.xc + j;
-    const size_t i = (size_t)x * g.ldz + z;
-    const bool on = zin && x < g.Nx - NH;
-    l[j][0] = on ? a.lam[0][i] : 0.0f;
-    l[j][1] = on ? a.lam[1][i] : 0.0f;
-  }
-  prefetch_adj_velocity<V>(at, c);
-  if (!tiled::tma::wait_tiles(at.err, bar)) return;
-  if (!zin) return;
-  const float hx = a.hx, hz = a.hz;
-#pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    const int x = c.xc + j;
-    if (x >= g.Nx - NH) break;
-    const size_t i = (size_t)x * g.ldz + z;
-    // the cell's inputs are requested before its stencil (the kept fields are
-    // read-only here, so their loads need not wait behind the previous
-    // column's stores)
-    const float2 cf = cell_undamped(a, x, z) ? make_float2(1.0f, a.dt) : __ldg(at.pk.cf + i);
-    const float ir = __ldg(a.p.invrho + i);
-    float sv = 0.0f, cv = 1.0f;  // tensor and Bond: fx = sxx_x + sxz_z, fz = sxz_x + szz_z
-    float kp = 0.0f, kq = 0.0f, kr = 0.0f, ks = 0.0f, a5 = 0.0f, a6 = 0.0f;
-    if (V == TTI_COORDINATE) {
-      const float2 vsc = __ldg(at.pk.vsc + i);
-      sv = vsc.x;
-      cv = vsc.y;
-      kp = __ldg(a.keep[4] + i);
-      kq = __ldg(a.keep[5] + i);
-      kr = __ldg(a.keep[6] + i);
-      ks = __ldg(a.keep[7] + i);
-      a5 = a.acc[5][i];
-      a6 = a.acc[6][i];
-    }
-    const float *q = sm + (x - c.x0 + 4) * B + (z - c.z0 + 8);
-    const float lx = l[j][0] - (vdiag1(q) + vdiag2(q + F));
-    const float lz = l[j][1] - (vdiag1(q + 2 * F) + vdiag2(q + 3 * F));
-    const float br = cf.y * ir;
-    const float Fx = br * lx, Fz = br * lz;
-    if (V == TTI_COORDINATE) {
-      // P = sxz_x - sxx_z, Q = szz_x - sxz_z, R = sxx_x + sxz_z, S = sxz_x + szz_z
-      a.acc[5][i] = a5 + (Fx * kp + Fz * kq);
-      a.acc[6][i] = a6 + (Fx * kr + Fz * ks);
-    }
-    const float Axx_x = cv * Fx, Axx_z = -sv * Fx;
-    const float Axz_x = sv * Fx + cv * Fz, Axz_z = cv * Fx - sv * Fz;
-    const float Azz_x = sv * Fz, Azz_z = cv * Fz;
-    a.TV[0][i] = hx * (Axx_x + Axx_z);
-    a.TV[1][i] = hx * (Axx_x - Axx_z);
-    a.TV[2][i] = hx * Azz_x + hz * Azz_z;
-    a.TV[3][i] = hx * Azz_x - hz * Azz_z;
-    a.TV[4][i] = hx * Axz_x + hz * Axz_z;
-    a.TV[5][i] = hx * Axz_x - hz * Axz_z;
-    a.lam[0][i] = cf.x * lx;
-    a.lam[1][i] = cf.x * lz;
-  }
-}
-
-// TMA boxes of the TV pair p (components sxx, szz, sxz) into shared buffers
-// 2b, 2b + 1, completing on barrier p; called by one thread.
-__device__ __forceinline__ void issue_tv_pair(const AdjTile &at, float *sm, unsigned long long *bar, int p, int b,
-                                              const TileCells &c)
-{
-  constexpr unsigned BOX_BYTES = tiled::BX * tiled::BZ * 4;
-  tiled::tma::mbar_arrive_expect_tx(bar + p, 2 * BOX_BYTES);
-  for (int k = 0; k < 2; ++k)
-    tiled::tma::tma_load_2d(sm + (2 * b + k) * tiled::FIELD, at.map + 2 * p + k, c.z0 - 8, c.x0 - 5, bar + p);
-}
-
-// transposed velocity stencils into lambda_sigma (maps: TV0..TV5), rows from
-// z_lo. The boxes come in three pairs (sxx: TV0 TV1, szz: TV2 TV3, sxz: TV4
-// TV5) through two pair buffers: pairs 0 and 1 are in flight from the start,
-// and pair 2 goes into pair 0's buffer once every thread is done with it. Four
-// boxes (58 KB) instead of six let three CTAs share an SM.
-__global__ void __launch_bounds__(tiled::NT, 3) k_adj_vstencil_tiled(const __grid_constant__ AdjTile at)
-{
+  const TileCells c = tile_cells(at, a.z_lo);
+  walk::init_bar(bar);
   pdl_sync();
-  constexpr int F = tiled::FIELD, B = tiled::BZ;
+  issue_adj(at, sm, bar, NB, 5, 0, NK, NP, c);
+  const walk::Coefs k = walk::coefs(rsg(0), rsg(1), rsg(2), rsg(3), rsg(4), at.nzero);
+  const size_t i = (size_t)c.x * g.ldz + c.z;
+  const int hi = min(g.Nz - NH, c.z0 + at.rows);
+  const bool surf = MODE == 0 && c.z0 < at.surf_zend;
+  const bool local = MODE != 1 && c.on && c.z + 3 >= g.izStart;
+  // this thread's inputs, requested while the copies are in flight
+  F4 l[3];
+  LocalIn<V> n;
+  if (c.on) {
+    // tensor: lambda_sigma is zero after the local part, and kept nowhere but
+    // in tiles with column work (the image rows)
+    if (V == TTI_TENSOR && MODE == 0 && !surf)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) l[q].p[0] = l[q].p[1] = walk::pack2(0.0f, 0.0f);
+    else
+#pragma unroll
+      for (int q = 0; q < 3; ++q) l[q] = ld4(a.lam[2 + q] + i);
+  }
+  if (local) load_local<V>(at, adj_undamped(at, c), i, n);
+  if (!walk::wait_boxes(at.err, bar, tiled::tma::WAIT_LIMIT, 0)) return;
+  if (MODE != 2) adj_walks<1, NB, false>(at, k, sm);
+  if (c.on) {
+    if (MODE != 2) {
+      F4 s[NB ? NB : 1][2];
+#pragma unroll
+      for (int f = 0; f < NB; ++f) adj_sums<false>(sm, c, f, s[f][0], s[f][1]);
+      auto sum = [&](int f, int q) { return at4(s[f][0], q) + at4(s[f][1], q); };
+      auto dif = [&](int f, int q) { return at4(s[f][0], q) - at4(s[f][1], q); };
+      const float hx = a.hx, hz = a.hz;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float dxx, dzz, dxz;
+        if (V == TTI_COORDINATE) {  // boxes A B C D
+          dxx = hx * (sum(0, q) - dif(1, q));
+          dzz = hx * sum(3 % NB, q) + hz * dif(2 % NB, q);
+          dxz = hx * (sum(1, q) + sum(2 % NB, q)) + hz * (dif(0, q) - dif(3 % NB, q));
+        } else {  // Fx, Fz
+          dxx = hx * sum(0, q);
+          dzz = hz * dif(1, q);
+          dxz = hx * sum(1, q) + hz * dif(0, q);
+        }
+        R::set(l[0], q, at4(l[0], q) - dxx);
+        R::set(l[1], q, at4(l[1], q) - dzz);
+        R::set(l[2], q, at4(l[2], q) - dxz);
+      }
+    }
+    if (MODE == 1 || surf)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) st4(a.lam[2 + q] + i, l[q], c.z, a.z_lo, hi);
+  }
+  if (MODE == 1) return;
+  if (surf) {
+    __syncwarp();
+    if (c.x < g.Nx - NH) surface_warp(sa, c.x, c.z0, c.z0 + at.rows, threadIdx.x & 31);
+    __syncwarp();
+    if (c.on)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const float4 v = __ldcg(reinterpret_cast<const float4 *>(a.lam[2 + q] + i));
+        l[q] = F4{{walk::pack2(v.x, v.y), walk::pack2(v.z, v.w)}};
+      }
+  }
+  if (local) stress_local<V>(at, c, i, l, n, sm + kept_off(NB), MODE == 2 || surf);
+}
+
+// Transposed stress stencils into lambda_v, then the velocity-half adjoint:
+// coordinate the theta_v sums (from the kept stress derivative combinations
+// P = sxz_x - sxx_z, Q = szz_x - sxz_z, R = sxx_x + sxz_z, S = sxz_x + szz_z),
+// the factors of the derivative terms, lambda_v *= coef1.
+template <int V>
+__global__ void __launch_bounds__(walk::NT, 3) k_adj_velocity_walk(const __grid_constant__ AdjTile at)
+{
+  constexpr int NK = velocity_kept(V);
   extern __shared__ __align__(128) float sm[];
-  unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + 4 * F);
+  unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + adj_bar(4, NK));
   const AdjArgs &a = at.a;
   const Grid &g = a.g;
-  const TileCells c = tile_cells(at.z_base);
-  if (threadIdx.x == 0) {
-    for (int q = 0; q < 3; ++q) tiled::tma::mbar_init(bar + q, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    issue_tv_pair(at, sm, bar, 0, 0, c);
-    issue_tv_pair(at, sm, bar, 1, 1, c);
-  }
-  const int z = c.z;
-  const bool zin = z >= a.z_lo && z < g.Nz - NH;
-  // this row's lambda_sigma, loaded while the halo boxes are in flight
-  constexpr int NJ = tiled::TX / 4;
-  float l[NJ][3];
-#pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    const int x = c.xc + j;
-    const size_t i = (size_t)x * g.ldz + z;
-    const bool on = zin && x < g.Nx - NH;
-    l[j][0] = on ? a.lam[2][i] : 0.0f;
-    l[j][1] = on ? a.lam[3][i] : 0.0f;
-    l[j][2] = on ? a.lam[4][i] : 0.0f;
-  }
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    if (q == 1) {
-      // every thread is done with pair 0's buffer: pair 2 goes there while pair 1 is used
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        issue_tv_pair(at, sm, bar, 2, 0, c);
-      }
-    }
-    // on a timeout the pairs still in flight get a bounded drain: q .. 1 before pair 2 is issued, q .. 2 after
-    if (!tiled::tma::wait_group(at.err, bar, q, q == 0 ? 2 : 3)) return;
-    if (zin) {
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const float *p = sm + (c.xc + j - c.x0 + 5) * B + (z - c.z0 + 8) + 2 * (q & 1) * F;
-        float d1, d2, u;
-        spair(p, d1, u);
-        spair(p + F, u, d2);
-        l[j][q] -= d1 + d2;
-      }
+  const TileCells c = tile_cells(at, g.izStart);
+  walk::init_bar(bar);
+  pdl_sync();
+  issue_adj(at, sm, bar, 4, 4, 4, NK, 0, c);
+  const bool und = adj_undamped(at, c);
+  const walk::Coefs k = walk::coefs(rsg(0), rsg(1), rsg(2), rsg(3), rsg(4), at.nzero);
+  // this thread's inputs, requested while the copies are in flight
+  const size_t i = (size_t)c.x * g.ldz + c.z;
+  const int lo = g.izStart, hi = min(g.Nz - NH, c.z0 + at.rows);
+  F4 lx, lz, c1, b, ir, sv, cv, a5, a6;
+  if (c.on) {
+    lx = ld4(a.lam[0] + i);
+    lz = ld4(a.lam[1] + i);
+    ir = ldg4(a.p.invrho + i);
+    adj_coefs(at, und, i, c1, b);
+    if (V == TTI_COORDINATE) {
+      sv = ldg4(a.p.snv + i);
+      cv = ldg4(a.p.csv + i);
+      a5 = ld4(a.acc[5] + i);
+      a6 = ld4(a.acc[6] + i);
     }
   }
-  if (!zin) return;
+  if (!walk::wait_boxes(at.err, bar, tiled::tma::WAIT_LIMIT, 0)) return;
+  adj_walks<0, 4, true>(at, k, sm);
+  if (!c.on) return;
+  F4 d1, d2;
+  adj_sums<true>(sm, c, 0, d1, d2);
 #pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    const int x = c.xc + j;
-    if (x >= g.Nx - NH) break;
-    const size_t i = (size_t)x * g.ldz + z;
-    a.lam[2][i] = l[j][0];
-    a.lam[3][i] = l[j][1];
-    a.lam[4][i] = l[j][2];
+  for (int q = 0; q < 4; ++q) R::set(lx, q, at4(lx, q) - (at4(d1, q) + at4(d2, q)));
+  adj_sums<true>(sm, c, 1, d1, d2);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) R::set(lz, q, at4(lz, q) - (at4(d1, q) + at4(d2, q)));
+  F4 o[4], kp[NK ? NK : 1];
+#pragma unroll
+  for (int f = 0; f < NK; ++f) kp[f] = ld4(sm + kept_off(4) + (f * WX + c.x - c.x0) * at.rows + (c.z - c.z0));
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float br = at4(b, q) * at4(ir, q), Fx = br * at4(lx, q), Fz = br * at4(lz, q);
+    if (V == TTI_COORDINATE) {
+      R::set(a5, q, at4(a5, q) + (Fx * at4(kp[0], q) + Fz * at4(kp[1 % (NK ? NK : 1)], q)));
+      R::set(a6, q, at4(a6, q) + (Fx * at4(kp[2 % (NK ? NK : 1)], q) + Fz * at4(kp[3 % (NK ? NK : 1)], q)));
+      R::set(o[0], q, at4(cv, q) * Fx);
+      R::set(o[1], q, at4(sv, q) * Fx);
+      R::set(o[2], q, at4(cv, q) * Fz);
+      R::set(o[3], q, at4(sv, q) * Fz);
+    } else {
+      R::set(o[0], q, Fx);
+      R::set(o[1], q, Fz);
+    }
+    R::set(lx, q, at4(c1, q) * at4(lx, q));
+    R::set(lz, q, at4(c1, q) * at4(lz, q));
+  }
+  st4(a.lam[0] + i, lx, c.z, lo, hi);
+  st4(a.lam[1] + i, lz, c.z, lo, hi);
+#pragma unroll
+  for (int q = 0; q < (V == TTI_COORDINATE ? 4 : 2); ++q) st4(a.TV[q] + i, o[q], c.z, lo, hi);
+  if (V == TTI_COORDINATE) {
+    st4(a.acc[5] + i, a5, c.z, lo, hi);
+    st4(a.acc[6] + i, a6, c.z, lo, hi);
   }
 }
 
-template <typename K>
-cudaError_t launch_adj_tile(K kernel, const AdjTile &at, int nfields, int z_first, const Grid &g, cudaStream_t st)
+// Tiles over rows z_first .. Nz - NH - 1; launches `kernel` with its boxes and
+// kept fields in shared memory.
+template <typename K, typename... Args>
+cudaError_t launch_adj(K kernel, AdjTile &at, int boxes, int kept, int z_first, cudaStream_t st, const Args &...args)
 {
-  const size_t bytes = (size_t)nfields * tiled::FIELD * sizeof(float) + 64;  // + up to 8 barriers
+  const Grid &g = at.a.g;
+  const size_t bytes = adj_smem(boxes, kept);
   static std::mutex mu;
-  static const void *done[8];
-  static int ndone = 0;
+  static std::vector<std::pair<const void *, int>> done;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
   {
     std::lock_guard<std::mutex> lock(mu);
-    bool seen = false;
-    for (int k = 0; k < ndone; ++k) seen = seen || done[k] == (const void *)kernel;
-    if (!seen) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    const std::pair<const void *, int> key{(const void *)kernel, dev};
+    if (std::find(done.begin(), done.end(), key) == done.end()) {
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       if (e != cudaSuccess) return e;
-      if (ndone < 8) done[ndone++] = (const void *)kernel;
+      done.push_back(key);
     }
   }
-  AdjTile b = at;
-  b.z_base = z_first & ~31;  // 32-row aligned: a warp's rows are one 128-byte line
-  const int nz = g.Nz - NH - b.z_base, nx = g.Nx - 2 * NH;
-  if (nz <= 0 || nx <= 0) return cudaSuccess;
-  return launch_pdl(kernel, dim3((nz + tiled::TZ - 1) / tiled::TZ, (nx + tiled::TX - 1) / tiled::TX), dim3(tiled::NT),
-                    bytes, st, b);
+  const dim3 gr = tiled::tiles(g, z_first, &at.z_base, &at.rows);
+  if (gr.x == 0 || gr.y == 0) return cudaSuccess;
+  return launch_pdl(kernel, gr, dim3(walk::NT), bytes, st, at, args...);
 }
 
 // residuals d - dobs (time-major) and J
@@ -955,6 +1067,12 @@ int grad_check(tti_handle *h)
   return TTI_OK;
 }
 
+// first row of the transposed velocity stencils: with a free surface the image rows too
+int adj_z_lo(const tti_handle *h)
+{
+  return h->cfg.freesurface ? std::max(NH, h->g.izStart - NH) : h->g.izStart;
+}
+
 int grad_alloc(tti_handle *h)
 {
   if (h->grad) return TTI_OK;
@@ -968,7 +1086,8 @@ int grad_alloc(tti_handle *h)
   bool ok = true;
   for (int k = 0; k < (h->cfg.variant == TTI_TENSOR ? 8 : 5); ++k) ok = ok && al(&s->lam[k]);
   for (auto &p : s->T) ok = ok && al(&p);
-  for (auto &p : s->TV) ok = ok && al(&p);
+  const int ntv = !h->use_tiled ? 6 : h->cfg.variant == TTI_COORDINATE ? 4 : 2;
+  for (int k = 0; k < ntv; ++k) ok = ok && al(&s->TV[k]);
   for (auto &p : s->acc) ok = ok && al(&p);
   for (auto &p : s->out) ok = ok && al(&p);
   ok = ok && cudaMalloc(&s->d_J, sizeof(double)) == cudaSuccess;
@@ -978,11 +1097,22 @@ int grad_alloc(tti_handle *h)
   }
   if (h->use_tiled) {
     void *mem = nullptr;
-    if (posix_memalign(&mem, 64, 10 * sizeof(CUtensorMap)) != 0)
+    if (posix_memalign(&mem, 64, 16 * sizeof(CUtensorMap)) != 0)
       return gerr(h, TTI_ERR_NOMEM, "host allocation failed");
     s->maps = static_cast<CUtensorMap *>(mem);
-    for (int k = 0; k < 10; ++k)
-      if (!tiled::encode_map(s->maps + k, h->g, k < 4 ? s->T[k] : s->TV[k - 4]))
+    for (int k = 0; k < 4 + ntv; ++k)
+      if (!tiled::encode_map(s->maps + k, h->g, k < 4 ? s->T[k] : s->TV[k - 4], walk::WB, walk::WBX))
+        return gerr(h, TTI_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    for (int k = 4 + ntv; k < 8; ++k) s->maps[k] = s->maps[4];  // unused
+    const Params p = handle_step_args(h).p;
+    const int v = h->cfg.variant;
+    const float *const par[7] = {p.c11, p.c13, p.c33, p.c55, v == TTI_TENSOR ? p.s2 : v == TTI_BOND ? p.c15 : p.sn,
+                                 v == TTI_TENSOR ? p.c2 : v == TTI_BOND ? p.c35 : p.cs,
+                                 v == TTI_TENSOR ? p.s2t : p.c55};
+    int z_base, rows;
+    tiled::tiles(h->g, adj_z_lo(h), &z_base, &rows);
+    for (int k = 0; k < 7; ++k)
+      if (!tiled::encode_map(s->maps + 9 + k, h->g, const_cast<float *>(par[k]), rows, WX))
         return gerr(h, TTI_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   }
   GCK(h, cudaStreamSynchronize(h->stream));
@@ -1003,10 +1133,7 @@ AdjArgs adj_args(tti_handle *h, int slot)
   a.hx = 0.5f * h->invdx;
   a.hz = 0.5f * h->invdz;
   a.dt = h->cfg.dt;
-  a.pk = packed::Packed{h->pk_cf, h->pk_vsc, h->pk_sc, h->pk_c4};
-  a.undamped_ok = h->use_tiled && h->undamped_ok;
-  a.und_z0 = h->cfg.freesurface ? 0 : h->g.E;
-  a.z_lo = h->cfg.freesurface ? std::max(NH, h->g.izStart - NH) : h->g.izStart;
+  a.z_lo = adj_z_lo(h);
   return a;
 }
 
@@ -1093,40 +1220,51 @@ int vsource_tables(tti_handle *h, const SourceTables &tab)
   return TTI_OK;
 }
 
-// Row origin for the stress-half adjoint with the column work folded in: the
-// highest of the image rows (free surface), the receiver rows and the stress
-// source's window rows, so that every warp's rows hold all the column work
-// below them; -1 when the free-surface rows would not fall in one warp.
-int surface_origin(tti_handle *h, int *z_org, int *z_end)
+// Whether the column work can run inside the stress-half adjoint: every
+// receiver, stress-source window and image row must lie in the tiles (columns
+// [NH, Nx - NH), rows from the first tile's to Nz - NH), the image rows and
+// their mirrors in the first; *z_end: the first row below all of them.
+int surface_extent(tti_handle *h, bool *merged, int *z_end)
 {
   const Grid &g = h->g;
   const tti_config &c = h->cfg;
-  int z = c.freesurface == 1 ? g.izStart - NH : g.izStart;
-  int e = c.freesurface == 1 ? g.izStart + NH + 1 : 0;
-  std::vector<int> rows;
+  const bool fs = c.freesurface == 1;
+  int z_base, tile_rows;
+  tiled::tiles(g, adj_z_lo(h), &z_base, &tile_rows);
+  int z = fs ? g.izStart - NH : g.Nz, e = fs ? g.izStart + NH + 1 : 0, x0 = g.Nx, x1 = 0;
+  std::vector<int> v;
   for (int k = 0; k < 3; ++k) {
     if (h->nrec[k] <= 0) continue;
-    rows.resize(h->nrec[k]);
-    GCK(h, cudaMemcpyAsync(rows.data(), h->d_rz[k], sizeof(int) * rows.size(), cudaMemcpyDeviceToHost, h->stream));
+    v.resize(h->nrec[k] + g.Nx + 1);  // rows in the caller's order; the column offsets
+    GCK(h, cudaMemcpyAsync(v.data(), h->d_rz[k], sizeof(int) * h->nrec[k], cudaMemcpyDeviceToHost, h->stream));
+    GCK(h, cudaMemcpyAsync(v.data() + h->nrec[k], h->d_rcol[k], sizeof(int) * (g.Nx + 1), cudaMemcpyDeviceToHost,
+                           h->stream));
     GCK(h, cudaStreamSynchronize(h->stream));
-    for (int r : rows) {
-      z = std::min(z, r);
-      e = std::max(e, r + 1);
+    for (int r = 0; r < h->nrec[k]; ++r) {
+      z = std::min(z, v[r]);
+      e = std::max(e, v[r] + 1);
     }
+    for (int x = 0; x < g.Nx; ++x)
+      if (v[h->nrec[k] + x + 1] > v[h->nrec[k] + x]) {
+        x0 = std::min(x0, x);
+        x1 = std::max(x1, x + 1);
+      }
   }
   if (c.stype == 1 && h->nsrc > 0) {
-    rows.resize(h->nsrc);
-    GCK(h, cudaMemcpyAsync(rows.data(), h->d_sz, sizeof(int) * rows.size(), cudaMemcpyDeviceToHost, h->stream));
+    v.resize(2 * h->nsrc);
+    GCK(h, cudaMemcpyAsync(v.data(), h->d_sz, sizeof(int) * h->nsrc, cudaMemcpyDeviceToHost, h->stream));
+    GCK(h, cudaMemcpyAsync(v.data() + h->nsrc, h->d_sx, sizeof(int) * h->nsrc, cudaMemcpyDeviceToHost, h->stream));
     GCK(h, cudaStreamSynchronize(h->stream));
-    for (int r : rows) {
-      z = std::min(z, std::max(0, r - NH));
-      e = std::max(e, std::min(g.Nz, r + NH + 1));
+    for (int n = 0; n < h->nsrc; ++n) {
+      z = std::min(z, std::max(0, v[n] - NH));
+      e = std::max(e, std::min(g.Nz, v[n] + NH + 1));
+      x0 = std::min(x0, std::max(0, v[h->nsrc + n] - NH));
+      x1 = std::max(x1, std::min(g.Nx, v[h->nsrc + n] + NH + 1));
     }
   }
-  z = std::max(z, 0);
   *z_end = e;
-  // the free-surface adjoint needs rows izStart - 5 .. izStart + 5 in the first warp's 32 rows
-  *z_org = c.freesurface == 1 && z < g.izStart + NH + 1 - BZ ? -1 : z;
+  *merged = z >= z_base && e <= g.Nz - NH && (x1 == 0 || (x0 >= NH && x1 <= g.Nx - NH)) &&
+            (!fs || g.izStart + NH + 1 <= z_base + tile_rows);
   return TTI_OK;
 }
 
@@ -1153,6 +1291,42 @@ int launch_vsource(tti_handle *h, const AdjArgs &a, int it)
   v.it = it;
   GCK(h, launch_pdl(k_adj_vsource, dim3(1), dim3(VSRC_THREADS), 0, h->stream, v));
   h->launches++;
+  return TTI_OK;
+}
+
+// The tiled kernels of one reverse step (see k_adj_stress).
+template <int V>
+int adjoint_tiles(tti_handle *h, const AdjArgs &a, const SurfaceArgs &sa, bool work, int slot)
+{
+  GradState *s = h->grad;
+  AdjTile at;
+  memset(&at, 0, sizeof at);
+  at.a = a;
+  at.kept = s->maps[8];
+  at.kept0 = slot * s->nkeep;
+  at.undamped_ok = h->undamped_ok;
+  at.und_z0 = h->cfg.freesurface ? 0 : h->g.E;
+  at.nzero = -0.0f;
+  at.err = h->d_flag;
+  for (int k = 0; k < 4; ++k) at.map[k] = s->maps[4 + k];
+  for (int k = 0; k < 7; ++k) at.par[k] = s->maps[9 + k];
+  constexpr int NB = stress_boxes(V), NK = stress_kept(V);
+  const int z0 = a.z_lo;  // the first tile row, the same for every kernel (the kept fields' boxes have one height)
+  if (!work || s->surf_merged) {
+    at.surf_zend = work ? s->surf_zend : 0;
+    GCK(h, launch_adj(k_adj_stress<V, 0>, at, NB, NK + stress_par(V), z0, h->stream, sa));
+  } else {
+    GCK(h, launch_adj(k_adj_stress<V, 1>, at, NB, 0, z0, h->stream, sa));
+    GCK(h, launch_pdl(k_adj_surface, dim3((h->g.Nx + 3) / 4), dim3(128), 0, h->stream, sa));
+    GCK(h, launch_adj(k_adj_stress<V, 2>, at, 0, NK + stress_par(V), z0, h->stream, sa));
+    h->launches += 2;
+  }
+  if (int rc = launch_vsource(h, a, sa.it)) return rc;
+  for (int k = 0; k < 4; ++k) at.map[k] = s->maps[k];
+  // tensor and Bond share the kernel: no rotation at the velocity node
+  GCK(h, launch_adj(k_adj_velocity_walk<V == TTI_TENSOR ? TTI_BOND : V>, at, 4, velocity_kept(V), z0,
+                    h->stream));
+  h->launches += 2;
   return TTI_OK;
 }
 
@@ -1188,52 +1362,24 @@ int adjoint_step(tti_handle *h, int n, int slot, const SourceTables &tab)
   sa.it = it;
   sa.fs = c.freesurface == 1;
   sa.tensor = c.variant == TTI_TENSOR;
-  const bool merged = h->use_tiled && s->surf_zorg >= 0;
-  if ((any || ssrc || sa.fs) && !merged) {
+  const bool work = any || ssrc || sa.fs;
+  if (h->use_tiled) {  // (the per-cell kernels below serve TTIFD_KERNEL=naive)
+    switch (c.variant) {
+    case TTI_COORDINATE: return adjoint_tiles<TTI_COORDINATE>(h, a, sa, work, slot);
+    case TTI_TENSOR: return adjoint_tiles<TTI_TENSOR>(h, a, sa, work, slot);
+    default: return adjoint_tiles<TTI_BOND>(h, a, sa, work, slot);
+    }
+  }
+  if (work) {
     GCK(h, launch_pdl(k_adj_surface, dim3((g.Nx + 3) / 4), dim3(128), 0, h->stream, sa));
     h->launches++;
   }
   h->launches += 3;
-  if (h->use_tiled) {  // TMA halo tiles (the per-cell kernels below serve TTIFD_KERNEL=naive)
-    // the stress-half adjoint stays one thread per cell: with the kept strain
-    // rates it has no stencil, only per-cell reads and writes
-    const int z0 = merged ? s->surf_zorg : 0;
-    const dim3 blk(BZ, BX), grd((g.Nz - z0 + BZ - 1) / BZ, (g.Nx + BX - 1) / BX);
-    if (merged) {
-      if (c.variant == TTI_BOND)
-        GCK(h, launch_pdl(k_adj_stress_local<TTI_BOND, true, true>, grd, blk, 0, h->stream, a, sa, z0, s->surf_zend));
-      else if (c.variant == TTI_TENSOR)
-        GCK(h, launch_pdl(k_adj_stress_local<TTI_TENSOR, true, true>, grd, blk, 0, h->stream, a, sa, z0, s->surf_zend));
-      else
-        GCK(h, launch_pdl(k_adj_stress_local<TTI_COORDINATE, true, true>, grd, blk, 0, h->stream, a, sa, z0, s->surf_zend));
-    } else {
-      if (c.variant == TTI_BOND)
-        GCK(h, launch_pdl(k_adj_stress_local<TTI_BOND, true, false>, grd, blk, 0, h->stream, a, sa, z0, s->surf_zend));
-      else if (c.variant == TTI_TENSOR)
-        GCK(h, launch_pdl(k_adj_stress_local<TTI_TENSOR, true, false>, grd, blk, 0, h->stream, a, sa, z0, s->surf_zend));
-      else
-        GCK(h, launch_pdl(k_adj_stress_local<TTI_COORDINATE, true, false>, grd, blk, 0, h->stream, a, sa, z0, s->surf_zend));
-    }
-    if (int rc = launch_vsource(h, a, it)) return rc;
-    AdjTile at;
-    memset(&at, 0, sizeof at);
-    at.a = a;
-    at.pk = packed::Packed{h->pk_cf, h->pk_vsc, h->pk_sc, h->pk_c4};
-    at.err = h->d_flag;
-    for (int k = 0; k < 4; ++k) at.map[k] = s->maps[k];
-    if (c.variant == TTI_COORDINATE)
-      GCK(h, launch_adj_tile(k_adj_velocity_tiled<TTI_COORDINATE>, at, 4, g.izStart, g, h->stream));
-    else  // tensor and Bond: no rotation at the velocity node
-      GCK(h, launch_adj_tile(k_adj_velocity_tiled<TTI_BOND>, at, 4, g.izStart, g, h->stream));
-    for (int k = 0; k < 6; ++k) at.map[k] = s->maps[4 + k];
-    GCK(h, launch_adj_tile(k_adj_vstencil_tiled, at, 4, a.z_lo, g, h->stream));
-    return TTI_OK;
-  }
   const dim3 blk(BZ, BX), grd((g.Nz + BZ - 1) / BZ, (g.Nx + BX - 1) / BX);
-  if (c.variant == TTI_BOND) k_adj_stress_local<TTI_BOND, false, false><<<grd, blk, 0, h->stream>>>(a, sa, 0, 0);
-  else if (c.variant == TTI_TENSOR) k_adj_stress_local<TTI_TENSOR, false, false><<<grd, blk, 0, h->stream>>>(a, sa, 0, 0);
-  else k_adj_stress_local<TTI_COORDINATE, false, false><<<grd, blk, 0, h->stream>>>(a, sa, 0, 0);
-  if (int rc = launch_vsource(h, a, it)) return rc;
+  if (c.variant == TTI_BOND) k_adj_stress_local<TTI_BOND><<<grd, blk, 0, h->stream>>>(a);
+  else if (c.variant == TTI_TENSOR) k_adj_stress_local<TTI_TENSOR><<<grd, blk, 0, h->stream>>>(a);
+  else k_adj_stress_local<TTI_COORDINATE><<<grd, blk, 0, h->stream>>>(a);
+  if (int rc = launch_vsource(h, a, sa.it)) return rc;
   if (c.variant == TTI_COORDINATE) k_adj_velocity<TTI_COORDINATE><<<grd, blk, 0, h->stream>>>(a);
   else k_adj_velocity<TTI_BOND><<<grd, blk, 0, h->stream>>>(a);  // tensor and Bond: no rotation at the velocity node
   k_adj_velocity_stencil<<<grd, blk, 0, h->stream>>>(a);
@@ -1344,6 +1490,12 @@ int grad_prepare(tti_handle *h, int slots, int seg, SourceTables *tab)
     s->ncheck = slots + 1;
     s->seg = seg;
     s->nkeep = nk;
+    if (h->use_tiled) {
+      int z_base, rows;
+      tiled::tiles(h->g, adj_z_lo(h), &z_base, &rows);
+      if (!tiled::encode_map3(s->maps + 8, h->g, s->keep, seg * nk, rows, WX))
+        return gerr(h, TTI_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    }
   }
   const int nt = c.nt;
   if (s->gsrc_n != h->nsrc * nt) {
@@ -1355,7 +1507,7 @@ int grad_prepare(tti_handle *h, int slots, int seg, SourceTables *tab)
   }
   handle_source_tables(h, tab);
   if ((rc = vsource_tables(h, *tab))) return rc;
-  return surface_origin(h, &s->surf_zorg, &s->surf_zend);
+  return surface_extent(h, &s->surf_merged, &s->surf_zend);
 }
 
 // Residuals d - dobs of every recorded component and J (read back into *J at
@@ -1379,7 +1531,8 @@ int grad_start_adjoint(tti_handle *h, double *J)
     if (p) GCK(h, cudaMemsetAsync(p, 0, n * sizeof(float), h->stream));
   for (auto p : s->T) GCK(h, cudaMemsetAsync(p, 0, n * sizeof(float), h->stream));
   if (s->gsrc) GCK(h, cudaMemsetAsync(s->gsrc, 0, sizeof(float) * (size_t)s->gsrc_n, h->stream));
-  for (auto p : s->TV) GCK(h, cudaMemsetAsync(p, 0, n * sizeof(float), h->stream));
+  for (auto p : s->TV)
+    if (p) GCK(h, cudaMemsetAsync(p, 0, n * sizeof(float), h->stream));
   return TTI_OK;
 }
 

@@ -564,21 +564,6 @@ int create_handle(tti_handle **out, const tti_config *cfg, int device, const tti
   if (share) {
     h->owner = share;
     for (int p = 0; p < TTI_P_COUNT; ++p) h->par[p] = share->par[p];
-    h->pk_cf = share->pk_cf;
-    h->pk_vsc = share->pk_vsc;
-    h->pk_sc = share->pk_sc;
-    h->pk_c4 = share->pk_c4;
-  } else if (h->use_tiled) {
-    auto palloc = [&](void *p, size_t bytes) {
-      return pool_alloc(static_cast<void **>(p), bytes, h->stream) == cudaSuccess;
-    };
-    bool okp = palloc(&h->pk_cf, g.n * sizeof(float2)) && palloc(&h->pk_sc, g.n * sizeof(float2)) &&
-               palloc(&h->pk_c4, g.n * sizeof(float4)) &&
-               (cfg->variant != TTI_COORDINATE || palloc(&h->pk_vsc, g.n * sizeof(float2)));
-    if (!okp) {
-      set_err(h, TTI_ERR_NOMEM, "device allocation of the packed parameters failed");
-      return fail(TTI_ERR_NOMEM);
-    }
   }
   for (int p = 0; p < TTI_P_COUNT && !share; ++p)
     if (param_used(cfg->variant, p) && (rc = alloc(&h->par[p]))) return fail(rc);
@@ -623,10 +608,6 @@ int tti_destroy(tti_handle *h)
   for (auto &p : h->fld) pool_free(p, fs);
   if (!h->owner) {
     for (auto &p : h->par) pool_free(p, fs);
-    pool_free(h->pk_cf, fs);
-    pool_free(h->pk_vsc, fs);
-    pool_free(h->pk_sc, fs);
-    pool_free(h->pk_c4, fs);
   }
   for (int k = 0; k < 3; ++k) {
     pool_free(h->d_rz[k], fs);  // with d_rzs, d_rid, d_rcol (one block)
@@ -777,19 +758,13 @@ static int upload_model(tti_handle *h, const float *const *src, bool physical)
   pool_free(raw_block, h->stream);
   pool_free(d_w, h->stream);
   if (rc == TTI_OK && h->use_tiled) {
-    packed::launch_pack(g, step_args(h).p, packed::Packed{h->pk_cf, h->pk_vsc, h->pk_sc, h->pk_c4}, c.variant,
-                       h->stream);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) rc = set_err(h, TTI_ERR_CUDA, "packing parameters: %s", cudaGetErrorString(e));
-  }
-  if (rc == TTI_OK && h->use_tiled) {
     // the tiled kernels skip coef1/coef2 loads where they are exactly 1 and
     // dt; verify that on the device instead of assuming the MEAL rim geometry
     int *cnt = nullptr;
     int bad = -1;
     if (pool_alloc(reinterpret_cast<void **>(&cnt), sizeof(int), h->stream) == cudaSuccess) {
       cudaMemsetAsync(cnt, 0, sizeof(int), h->stream);
-      packed::launch_check_undamped(g, h->par[TTI_P_COEF1], h->par[TTI_P_COEF2], c.dt, c.freesurface ? 0 : g.E, cnt,
+      launch_check_undamped(g, h->par[TTI_P_COEF1], h->par[TTI_P_COEF2], c.dt, c.freesurface ? 0 : g.E, cnt,
                                    h->stream);
       cudaMemcpyAsync(&bad, cnt, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
       pool_free(cnt, h->stream);

@@ -125,7 +125,7 @@ int build_tables(tti_batch *b)
     ha.invdx = h->invdx;
     ha.invdz = h->invdz;
     ha.dt = c.dt;
-    const dim3 gr = tiled::grid(h->g, &ha.z_base, &ha.tile_rows);
+    const dim3 gr = tiled::tiles(h->g, h->g.izStart, &ha.z_base, &ha.tile_rows);
     ha.x_base = NH;
     ha.undamped_ok = h->undamped_ok;
     ha.freesurface = c.freesurface;
@@ -344,7 +344,8 @@ int tti_batch_create(tti_batch **out, int nmodels, const tti_config *cfg, int ni
   b->nwork = 0;
   for (int i = 0; i < ninst; ++i) {
     int zb, rows;
-    const dim3 gr = tiled::grid(b->inst[i]->g, &zb, &rows);
+    const Grid &g = b->inst[i]->g;
+    const dim3 gr = tiled::tiles(g, g.izStart, &zb, &rows);
     b->nwork += (int)(gr.x * gr.y);
     b->max_nt = std::max(b->max_nt, b->inst[i]->cfg.nt);
     b->max_Nx = std::max(b->max_Nx, b->inst[i]->g.Nx);

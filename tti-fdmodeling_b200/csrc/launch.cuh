@@ -31,6 +31,10 @@ void launch_setup(const Grid &g, const SetupIn &in, const SetupOut &out, const M
 // dense padded [Nx][Nz] arrays (Nz * Nx floats apart), the E-wide rims filled
 // as padModel2d fills them on the host.
 void launch_expand_physical(const float *phys, float *pad, int na, int nz, int nx, int E, cudaStream_t st);
+// Counts cells of [E, Nx-E) x [zD, Nz-E) with coef1 != 1 or coef2 != dt; the
+// tiled kernels skip those loads where there are none.
+void launch_check_undamped(const Grid &g, const float *coef1, const float *coef2, float dt, int zD, int *count,
+                           cudaStream_t st);
 
 // ---------------- per-step ----------------
 // Source weight tables over the 11 x 11 window (offset (a, b) at a*11+b,

@@ -185,6 +185,21 @@ __global__ void k_expand_physical(const float *phys, float *pad, int na, int nz,
   for (int k = 0; k < na; ++k) pad[k * np + d] = phys[k * nq + s];
 }
 
+// one block per interior column: counts the rows [zD, Nz - E) where the MEAL
+// coefficients differ from the undamped values
+__global__ void k_check_undamped(Grid g, const float *__restrict__ c1, const float *__restrict__ c2, float dt,
+                                 int zD, int *count)
+{
+  const int ix = g.E + blockIdx.y;
+  int bad = 0;
+  for (int iz = zD + (int)threadIdx.x; iz < g.Nz - g.E; iz += blockDim.x) {
+    const size_t i = (size_t)ix * g.ldz + iz;
+    bad += (c1[i] != 1.0f) | (c2[i] != dt);
+  }
+  bad = __syncthreads_count(bad > 0);
+  if (threadIdx.x == 0 && bad) atomicAdd(count, bad);
+}
+
 }  // namespace
 
 void launch_setup(const Grid &g, const SetupIn &in, const SetupOut &out, const MealConst &mc, int variant,
@@ -199,6 +214,14 @@ void launch_expand_physical(const float *phys, float *pad, int na, int nz, int n
 {
   const int Nz = nz + 2 * E, Nx = nx + 2 * E;
   k_expand_physical<<<dim3((Nz + 127) / 128, Nx), 128, 0, st>>>(phys, pad, na, nz, nx, E);
+}
+
+void launch_check_undamped(const Grid &g, const float *coef1, const float *coef2, float dt, int zD, int *count,
+                           cudaStream_t st)
+{
+  const int nx = g.Nx - 2 * g.E;
+  if (nx <= 0) return;
+  k_check_undamped<<<dim3(1, nx), 256, 0, st>>>(g, coef1, coef2, dt, zD, count);
 }
 
 }  // namespace ttifd

@@ -1,21 +1,13 @@
 // Tiled half-step kernels (tiled_step.cu): velocity and stress updates in
-// place, each CTA loading its halo tile with one 2D TMA copy per field.
+// place, each CTA loading its halo tile with TMA copies.
 #pragma once
 
 #include <cuda.h>
 
-#include "pack.cuh"
+#include "launch.cuh"
 
 namespace ttifd {
 namespace tiled {
-
-constexpr int TX = 16;        // tile columns (x)
-constexpr int TZ = 128;       // tile rows (z)
-constexpr int BZ = TZ + 16;   // TMA box rows: [z0-8, z0+TZ+8), 16-byte aligned start
-constexpr int BX = TX + 9;    // TMA box columns: the tile plus the 10-point stencil's halo
-constexpr int NT = 512;       // threads per CTA: one row x TX/4 columns each (64 warps per SM at 4 CTAs)
-// floats per field region in shared memory, 128-byte aligned
-constexpr int FIELD = (BX * BZ * 4 + 127) / 128 * 128 / 4;
 
 // A handle's tensor maps: the halo boxes of vx vz sxx szz
 // sxz, then the tile inputs of the stress update (HalfArgs::in).
@@ -84,10 +76,13 @@ __host__ __device__ __forceinline__ bool tile_undamped(const HalfArgs &a, int z0
          z0 + a.tile_rows <= g.Nz - g.E;
 }
 
-// Encodes the 2D tensor map of one [Nx][ldz] field for the halo box.
-bool encode_map(CUtensorMap *map, const Grid &g, float *field, int box_rows = BZ, int box_cols = BX);
-// Tile grid; *z_base receives the first tile row, *tile_rows the height of a tile.
-dim3 grid(const Grid &g, int *z_base, int *tile_rows);
+// Encodes the 2D tensor map of one [Nx][ldz] field for boxes of box_rows x box_cols.
+bool encode_map(CUtensorMap *map, const Grid &g, float *field, int box_rows, int box_cols);
+// The same for `count` consecutive fields (3D; boxes of one field).
+bool encode_map3(CUtensorMap *map, const Grid &g, float *fields, int count, int box_rows, int box_cols);
+// Tile grid over rows z_first .. Nz - NH - 1: *z_base receives the first tile
+// row, *tile_rows the height of a tile.
+dim3 tiles(const Grid &g, int z_first, int *z_base, int *tile_rows);
 cudaError_t launch_velocity(const HalfArgs &a, int variant, bool exact, cudaStream_t st);
 cudaError_t launch_stress(const HalfArgs &a, int variant, bool exact, cudaStream_t st);
 // Batched: one launch over all instances' tiles (each instance's arguments
@@ -157,78 +152,14 @@ __device__ __forceinline__ void tma_load_2d(float *dst, const CUtensorMap *map, 
       : "memory");
 }
 
-static_assert((BZ * 4) % 16 == 0, "TMA inner box extent must be a multiple of 16 bytes");
-
-// Issues the TMA copies of the halo boxes of `n` fields (origin row z0 - 8,
-// column x0 - xoff); waited for by wait_tiles. With ph < 0 the barrier is
-// initialised here (a CTA that loads one tile); with ph >= 0 it is a barrier
-// the CTA initialised once, whose phase ph these copies complete (a CTA that
-// loads tile after tile: an mbarrier must not be initialised again while it
-// is valid).
-__device__ __forceinline__ void issue_tiles(const CUtensorMap *map, float *sm, unsigned long long *bar, int n, int z0,
-                                            int x0, int xoff, int ph = -1)
+__device__ __forceinline__ void tma_load_3d(float *dst, const CUtensorMap *map, int c0, int c1, int c2,
+                                            unsigned long long *bar)
 {
-  constexpr unsigned BOX_BYTES = BX * BZ * 4;
-  const int t = threadIdx.x;
-  if (t == 0 && ph < 0) {
-    mbar_init(bar, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();  // also: every thread is done with the boxes these copies replace
-  if (t == 0) {
-    mbar_arrive_expect_tx(bar, n * BOX_BYTES);
-    for (int f = 0; f < n; ++f) tma_load_2d(sm + f * FIELD, map + f, z0 - 8, x0 - xoff, bar);
-  }
-}
-
-// returns false (all threads) after a timed-out wait
-__device__ __forceinline__ bool wait_tiles(int *err, unsigned long long *bar, unsigned limit = WAIT_LIMIT,
-                                           unsigned parity = 0)
-{
-  const bool ok = mbar_wait(bar, parity, limit);
-  if (__syncthreads_or(!ok)) {
-    if (threadIdx.x == 0) {
-      atomicOr(err, 4);
-      mbar_wait(bar, parity, 1u << 16);  // give the copies in flight a bounded time
-    }
-    return false;
-  }
-  return true;
-}
-
-// The halo boxes of ng groups of `per` fields each, one barrier per group
-// (bars[0..ng)), so that a CTA can work on a group while the next is in flight.
-__device__ __forceinline__ void issue_groups(const CUtensorMap *map, float *sm, unsigned long long *bars, int ng,
-                                             int per, int z0, int x0, int xoff)
-{
-  constexpr unsigned BOX_BYTES = BX * BZ * 4;
-  const int t = threadIdx.x;
-  if (t == 0) {
-    for (int q = 0; q < ng; ++q) mbar_init(bars + q, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  if (t == 0)
-    for (int q = 0; q < ng; ++q) {
-      mbar_arrive_expect_tx(bars + q, per * BOX_BYTES);
-      for (int f = q * per; f < (q + 1) * per; ++f) tma_load_2d(sm + f * FIELD, map + f, z0 - 8, x0 - xoff, bars + q);
-    }
-}
-
-// Waits for group q of issue_groups (every thread of the CTA calls it); after a
-// timeout returns false to all threads, having given the groups from q on a
-// bounded time to land.
-__device__ __forceinline__ bool wait_group(int *err, unsigned long long *bars, int q, int ng)
-{
-  const bool ok = mbar_wait(bars + q, 0);
-  if (__syncthreads_or(!ok)) {
-    if (threadIdx.x == 0) {
-      atomicOr(err, 4);
-      for (int r = q; r < ng; ++r) mbar_wait(bars + r, 0, 1u << 16);
-    }
-    return false;
-  }
-  return true;
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          smem_u32(dst)),
+      "l"(reinterpret_cast<unsigned long long>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
+      : "memory");
 }
 
 }  // namespace tma

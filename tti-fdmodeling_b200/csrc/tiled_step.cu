@@ -538,7 +538,7 @@ cudaError_t launch_k(K kernel, const HalfArgs &a, int variant, bool velocity, cu
   cudaError_t e = prepare_kernel(kernel, bytes, &wave);
   if (e != cudaSuccess) return e;
   HalfArgs b = a;
-  const dim3 gr = grid(a.g, &b.z_base, &b.tile_rows);
+  const dim3 gr = tiles(a.g, a.g.izStart, &b.z_base, &b.tile_rows);
   if (gr.x == 0 || gr.y == 0) return cudaSuccess;
   return launch_pdl(kernel, gr, dim3(walk::NT), bytes, st, b);
 }
@@ -546,29 +546,47 @@ cudaError_t launch_k(K kernel, const HalfArgs &a, int variant, bool velocity, cu
 }  // namespace
 
 
-dim3 grid(const Grid &g, int *z_base, int *tile_rows)
+dim3 tiles(const Grid &g, int z_first, int *z_base, int *tile_rows)
 {
-  // from izStart rounded down to a 32-byte sector; tiles of equal height
-  *z_base = g.izStart & ~7;
+  // from z_first rounded down to a 32-byte sector; tiles of equal height
+  *z_base = z_first & ~7;
   const int nz = g.Nz - NH - *z_base, nx = g.Nx - 2 * NH;
   *tile_rows = walk::WZ;
   if (nz <= 0 || nx <= 0) return dim3(0, 0);
-  int nt = (nz + walk::WZ - 1) / walk::WZ;
+  const int nt = (nz + walk::WZ - 1) / walk::WZ;
   *tile_rows = ((nz + nt - 1) / nt + 7) & ~7;
   return dim3(nt, (nx + WX - 1) / WX);
 }
 
+static PFN_cuTensorMapEncodeTiled_v12000 encoder()
+{
+  static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+    cudaDriverEntryPointQueryResult q;
+    void *p = nullptr;
+    const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                    q == cudaDriverEntryPointSuccess;
+    return ok ? reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p) : nullptr;
+  }();
+  return fn;
+}
+
+bool encode_map3(CUtensorMap *map, const Grid &g, float *fields, int count, int box_rows, int box_cols)
+{
+  const auto encode = encoder();
+  if (!encode) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)g.ldz, (cuuint64_t)g.Nx, (cuuint64_t)count};
+  const cuuint64_t strides[2] = {(cuuint64_t)g.ldz * sizeof(float), (cuuint64_t)g.n * sizeof(float)};
+  const cuuint32_t box[3] = {(cuuint32_t)box_rows, (cuuint32_t)box_cols, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, fields, dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool encode_map(CUtensorMap *map, const Grid &g, float *field, int box_rows, int box_cols)
 {
-  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-  if (!encode) {
-    cudaDriverEntryPointQueryResult q;
-    void *fn = nullptr;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || !fn)
-      return false;
-    encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-  }
+  const auto encode = encoder();
+  if (!encode) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)g.ldz, (cuuint64_t)g.Nx};
   const cuuint64_t strides[1] = {(cuuint64_t)g.ldz * sizeof(float)};
   const cuuint32_t box[2] = {(cuuint32_t)box_rows, (cuuint32_t)box_cols};
@@ -586,7 +604,7 @@ bool encode_maps(CUtensorMap *map, const Grid &g, int variant, const Fields &f, 
                                     t ? p.s2 : b ? p.c15 : p.sn, t ? p.c2 : b ? p.c35 : p.cs,
                                     p.c11, p.c13, p.c33, p.c55, t ? p.s2t : p.c55};
   int z_base, rows;
-  grid(g, &z_base, &rows);
+  tiles(g, g.izStart, &z_base, &rows);
   for (int k = 0; k < HALO_MAPS; ++k)
     if (!encode_map(map + k, g, halo[k], walk::WB, walk::WBX)) return false;
   for (int k = 0; k < IN_MAPS; ++k)

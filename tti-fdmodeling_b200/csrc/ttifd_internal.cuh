@@ -152,8 +152,6 @@ struct tti_handle {
   void *tmaps = nullptr;   // host copy of the tensor maps (tiled::encode_maps), 64-byte aligned
   int undamped_ok = 0;  // coef1 == 1, coef2 == dt outside the absorbing rims (checked at upload)
   int *d_rcol[3] = {}, *d_rzs[3] = {}, *d_rid[3] = {};  // receivers grouped by column
-  float2 *pk_cf = nullptr, *pk_vsc = nullptr, *pk_sc = nullptr;  // packed parameters (pack.cuh)
-  float4 *pk_c4 = nullptr;
   float *par[TTI_P_COUNT] = {};
   float invdx = 0, invdz = 0, alpha_src = 0;
   // geometry

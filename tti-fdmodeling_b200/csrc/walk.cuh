@@ -21,6 +21,7 @@ namespace walk {
 constexpr int WX = 8;                        // tile columns: one warp each in the update
 constexpr int WZ = 120;                      // most tile rows: four per lane in the update, four warps of diagonals
 constexpr int WB = WZ + 16;                  // box rows (the box starts 8 rows above the tile)
+static_assert((WB * 4) % 16 == 0, "TMA inner box extent must be a multiple of 16 bytes");
 constexpr int WBX = WX + 9;                  // box columns
 constexpr int DP = (WZ + WX + 2 + 3) / 4 * 4;  // column pitch of a sum array (see d1_row, d2_row)
 constexpr int NT = 32 * WX;                  // threads per CTA
