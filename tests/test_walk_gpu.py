@@ -48,3 +48,34 @@ def test_tile_edges(variant, nz, nx, eal, fs, dz, monkeypatch, gpu_lib):
     for k, (a, b) in enumerate(zip(got, ref)):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (k, np.max(np.abs(a - b)))
     assert any(np.any(b != 0) for b in ref)
+
+
+# The column work (sources, free surface, receivers) runs in the tiles, in one
+# or two rows of tiles, or as launches of its own where a column lies outside
+# the updated ones or receivers spread over more rows.
+@pytest.mark.parametrize("where", ["surface", "two tiles", "all depths", "outside"])
+@pytest.mark.parametrize("stype", [1, 2, 3, 4, 5, 6, 7, 8])
+def test_column_work(where, stype, monkeypatch, gpu_lib):
+    import ttifd
+
+    nz, nx, nt, eal = 300, 40, 50, 0 if where == "outside" else 3
+    m = synthetic.layered_model(nz, nx, seed=8)
+    w = synthetic.ricker(nt, 0.0008, 30.0, delay=0.01)
+    gx = np.arange(nx)
+    sx, sz, gz = {"surface": ([20, 22], [2, 3], 2), "two tiles": ([20, 22], [112 - eal - 5, 105], 112),
+                  "all depths": ([20, 21], [140, 3], (gx * 7) % nz), "outside": ([0, nx], [nz, 2], 2)}[where]
+    out = []
+    for kernel in ("naive", "tiled"):
+        monkeypatch.setenv("TTIFD_EXACT", "1")
+        monkeypatch.setenv("TTIFD_KERNEL", kernel)
+        with ttifd.Modeling(variant=1, nz=nz, nx=nx, nt=nt, dx=10.0, dz=10.0, dt=0.0008, fpeak=30.0, ealThick=eal,
+                            freesurface=1, stype=stype, seistype=3, mt=2) as h:
+            h.upload_model(*synthetic.padded(m, eal))
+            h.set_source(sx, sz, np.stack([w, 0.5 * w]))
+            for k in (0, 1, 2):
+                h.set_receivers(k, gx, gz)
+            h.run()
+            out.append([h.fetch_traces(k) for k in (0, 1, 2)] + [h.fetch_field(f) for f in range(8)])
+    for k, (a, b) in enumerate(zip(*out)):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (k, np.max(np.abs(a - b)))
+    assert np.any(out[0][3] != 0)

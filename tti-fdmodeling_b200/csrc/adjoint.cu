@@ -1505,6 +1505,7 @@ int grad_prepare(tti_handle *h, int slots, int seg, SourceTables *tab)
     if (h->nsrc > 0) GCK(h, cudaMalloc(&s->gsrc, sizeof(float) * (size_t)h->nsrc * nt));
     s->gsrc_n = h->nsrc * nt;
   }
+  if ((rc = handle_columns(h))) return rc;
   handle_source_tables(h, tab);
   if ((rc = vsource_tables(h, *tab))) return rc;
   return surface_extent(h, &s->surf_merged, &s->surf_zend);
@@ -1538,7 +1539,7 @@ int grad_start_adjoint(tti_handle *h, double *J)
 
 // forward steps k0 .. k1-1 from the current state; `record`: what the adjoint
 // needs of each step goes to the kept segment (slot k - k0)
-int forward_steps(tti_handle *h, int k0, int k1, bool record, const SourceTables &tab)
+int forward_steps(tti_handle *h, int k0, int k1, bool record)
 {
   GradState *s = h->grad;
   const int nk = s->nkeep;
@@ -1546,7 +1547,7 @@ int forward_steps(tti_handle *h, int k0, int k1, bool record, const SourceTables
     float *keep[8] = {};
     if (record)
       for (int f = 0; f < nk; ++f) keep[f] = s->keep + ((size_t)(k - k0) * nk + f) * h->g.n;
-    const int rc = handle_step(h, tab, record ? keep : nullptr);
+    const int rc = handle_step(h, record ? keep : nullptr);
     if (rc) return rc;
   }
   return TTI_OK;
@@ -1767,7 +1768,7 @@ int tti_grad_run(tti_handle *h, int ncheck, double *misfit)
   for (int q = 0; q < nseg; ++q) {
     const bool last = q == nseg - 1;
     if (!last && (rc = store_state(h, q))) return rc;
-    if ((rc = forward_steps(h, q * seg, std::min(nt, (q + 1) * seg), last, tab))) return rc;
+    if ((rc = forward_steps(h, q * seg, std::min(nt, (q + 1) * seg), last))) return rc;
   }
   double J = 0.0;
   if ((rc = grad_start_adjoint(h, &J))) return rc;
@@ -1776,7 +1777,7 @@ int tti_grad_run(tti_handle *h, int ncheck, double *misfit)
     const int k0 = q * seg, k1 = std::min(nt, (q + 1) * seg);
     if (q < nseg - 1) {  // recompute the segment from its checkpoint
       if ((rc = restore_state(h, q, k0))) return rc;
-      if ((rc = forward_steps(h, k0, k1, true, tab))) return rc;
+      if ((rc = forward_steps(h, k0, k1, true))) return rc;
     }
     if ((rc = adjoint_steps(h, k0, k1, tab))) return rc;
   }
@@ -1802,10 +1803,10 @@ int tti_grad_run_binomial(tti_handle *h, int snapshots, int keep_steps, double *
   double J = 0.0;
   for (const Action &a : acts) {
     switch (a.kind) {
-    case Action::ADVANCE: rc = forward_steps(h, step_of(a.a), step_of(a.b), false, tab); break;
+    case Action::ADVANCE: rc = forward_steps(h, step_of(a.a), step_of(a.b), false); break;
     case Action::STORE: rc = store_state(h, a.slot); break;
     case Action::RESTORE: rc = restore_state(h, a.slot, step_of(a.a)); break;
-    case Action::RECORD: rc = forward_steps(h, step_of(a.a), step_of(a.b), true, tab); break;
+    case Action::RECORD: rc = forward_steps(h, step_of(a.a), step_of(a.b), true); break;
     case Action::START_ADJOINT: rc = grad_start_adjoint(h, &J); break;
     case Action::ADJOINT: rc = adjoint_steps(h, step_of(a.a), step_of(a.b), tab); break;
     }

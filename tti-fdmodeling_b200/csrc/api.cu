@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <numeric>
 
+#include "columns.cuh"
 #include "walk.cuh"
 
 using namespace ttifd;
@@ -123,18 +124,83 @@ int check_cfg(const tti_config *c)
 
 int current_it(const tti_handle *h) { return h->cfg.mode == 2 ? h->cfg.nt - 1 - h->step_index : h->step_index; }
 
+// Fills h->d_cols from the geometry, and decides where the column work runs.
+// The tiled kernels take it when every column it touches is in a tile
+// ([NH, Nx - NH)) and its rows fall in at most two rows of tiles: each warp of
+// such a tile then goes through its column's receivers once more, which for
+// receivers spread over all depths costs more than the launch it saves.
+int sync_columns(tti_handle *h)
+{
+  if (!h->cols_dirty) return TTI_OK;
+  const tti_config &c = h->cfg;
+  const Grid &g = h->g;
+  Columns w;
+  memset(&w, 0, sizeof w);
+  w.stype = h->nsrc > 0 ? c.stype : 0;
+  w.freesurface = c.freesurface == 1;
+  w.tensor = c.variant == TTI_TENSOR;
+  w.nt = c.nt;
+  w.mode2 = c.mode == 2;
+  w.mt = c.mt;
+  w.src = SourceSet{h->nsrc, h->d_sx, h->d_sz, h->d_src, c.nt};
+  source_tables(h, &w.t);
+  const bool want_v = c.seistype == 1 || c.seistype == 3, want_p = c.seistype == 2 || c.seistype == 3;
+  h->rec_at = Extent();
+  for (int k = 0; k < 3; ++k) {
+    const bool on = (k < 2 ? want_v : want_p) && h->nrec[k] > 0;
+    w.colptr[k] = on ? h->d_rcol[k] : nullptr;
+    w.rz[k] = h->d_rzs[k];
+    w.rid[k] = h->d_rid[k];
+    w.rec[k] = h->d_rec[k];
+    w.nrec[k] = h->nrec[k];
+    if (on) h->rec_at.add(h->rec_of[k]);
+  }
+  w.rec_on = h->rec_at.x1 > 0;
+  w.flag = h->d_flag;
+  Extent post = h->rec_at;
+  if (w.stype == 1) post.add(h->src_at);
+  if (w.freesurface) post.add(NH, g.Nx - NH, g.izStart - NH, g.izStart + NH + 1);
+  auto fold = [&](const Extent &e) {
+    if (!h->use_tiled) return false;
+    int z_base, rows;
+    const int nt = (int)tiled::tiles(g, g.izStart, &z_base, &rows).x;
+    auto tile = [&](int z) { return std::min(std::max((z - z_base) / rows, 0), nt - 1); };
+
+    return nt > 0 && e.x1 > 0 && e.x0 >= NH && e.x1 <= g.Nx - NH && tile(e.z1 - 1) - tile(e.z0) < 2;
+  };
+  h->fold_src = w.stype >= 2 && fold(h->src_at);
+  h->fold_post = fold(post);
+  if (!h->d_cols) CK(h, pool_alloc(reinterpret_cast<void **>(&h->d_cols), sizeof w, h->stream));
+  CK(h, cudaMemcpyAsync(h->d_cols, &w, sizeof w, cudaMemcpyHostToDevice, h->stream));
+  CK(h, cudaStreamSynchronize(h->stream));  // w goes out of scope
+  h->cols_dirty = false;
+  return TTI_OK;
+}
+
+// Rows of the column work after the stress update of a step that does or does
+// not record.
+Extent post_extent(const tti_handle *h, bool rec_now)
+{
+  const Grid &g = h->g;
+  Extent e;
+  if (rec_now) e = h->rec_at;
+  if (h->nsrc > 0 && h->cfg.stype == 1) e.add(h->src_at);
+  if (h->cfg.freesurface == 1) e.add(NH, g.Nx - NH, g.izStart - NH, g.izStart + NH + 1);
+  return e;
+}
+
 // Launches one time step (coord:611-926 body). With `ev` (5 events) the
 // phases are bracketed for tti_profile_steps: ev[0] | velocity | ev[1] |
-// velocity sources | ev[2] | stress | ev[3] | the rest | ev[4]. With `keep`
-// (5 device arrays, the gradient's recompute pass) vx, vz, sxx, szz, sxz are
-// copied there between the velocity sources and the stress update.
-int launch_one_step(tti_handle *h, const SourceTables &tab, cudaEvent_t *ev = nullptr, float *const *keep = nullptr)
+// velocity sources | ev[2] | stress | ev[3] | the rest | ev[4] (the sources
+// and the rest are empty where the half-step kernels do the column work). With
+// `keep` the gradient's forward pass keeps what the adjoint needs of the step.
+int launch_one_step(tti_handle *h, cudaEvent_t *ev = nullptr, float *const *keep = nullptr)
 {
   const tti_config &c = h->cfg;
-  const int it = current_it(h);
+  const int it = current_it(h), n = h->step_index;
   StepArgs a = step_args(h);
-  SourceSet s{h->nsrc, h->d_sx, h->d_sz, h->d_src, c.nt};
-  const bool vsrc = s.n > 0 && c.stype >= 2, ssrc = s.n > 0 && c.stype == 1;
+  const bool vsrc = h->nsrc > 0 && c.stype >= 2;
+  ColumnShot cs{h->g, a.f, h->d_cols, h->src_at.x0, h->src_at.x1};
   tiled::HalfArgs ha{};
   // What the gradient keeps of this step (keep_fields). Tiled kernels: the
   // stress kernel writes the strain rates vxx vxz vzx vzz (keep[0..3]) and for
@@ -144,27 +210,21 @@ int launch_one_step(tti_handle *h, const SourceTables &tab, cudaEvent_t *ev = nu
   // txx tzz txz) after the sources, from whose stencils the adjoint works.
   const bool keep_tiled = keep && h->use_tiled;
   if (h->use_tiled) {
-    ha.g = h->g;
-    ha.f = a.f;
-    ha.p = a.p;
-    ha.invdx = h->invdx;
-    ha.invdz = h->invdz;
-    ha.dt = c.dt;
-    ha.x_base = NH;
-    ha.undamped_ok = h->undamped_ok;
-    ha.freesurface = c.freesurface;
-    tiled::set_square(ha, h->exact);
-    ha.wait_limit = h->wait_limit;
-    ha.err = h->d_flag;
-    tiled::set_half(ha, static_cast<const CUtensorMap *>(h->tmaps), c.variant, true);
+    tiled::fill_args(ha, h, a);
+    ha.n = n;
+    if (h->fold_src) tiled::set_work(ha, h->src_at);
     if (keep_tiled && c.variant == TTI_COORDINATE)
       for (int k = 0; k < 4; ++k) ha.kd[k] = keep[4 + k];
   }
   if (ev) CK(h, cudaEventRecord(ev[0], h->stream));
-  if (h->use_tiled) CK(h, tiled::launch_velocity(ha, c.variant, h->exact, h->stream));
+  if (h->use_tiled) CK(h, tiled::launch_velocity(ha, h->tmaps, c.variant, h->exact, h->stream));
   else launch_velocity(a, h->stream);
+  h->launches++;
   if (ev) CK(h, cudaEventRecord(ev[1], h->stream));
-  if (vsrc) launch_sources(a, s, &tab, c.stype, 0, it, h->stream);
+  if (vsrc && !h->fold_src) {
+    CK(h, launch_sources(cs, n, h->stream));
+    h->launches++;
+  }
   if (keep && !keep_tiled) {  // v after the sources, and sigma or tau
     const bool t = c.variant == TTI_TENSOR;
     float *const src[5] = {h->fld[0], h->fld[1], h->fld[t ? 5 : 2], h->fld[t ? 6 : 3], h->fld[t ? 7 : 4]};
@@ -172,38 +232,22 @@ int launch_one_step(tti_handle *h, const SourceTables &tab, cudaEvent_t *ev = nu
     h->launches++;
   }
   if (ev) CK(h, cudaEventRecord(ev[2], h->stream));
+  // after the stress update: free surface, stress source and receivers
+  const Extent post = post_extent(h, it % c.mt == 0);
   if (h->use_tiled) {
-    tiled::set_half(ha, static_cast<const CUtensorMap *>(h->tmaps), c.variant, false);
     for (int k = 0; k < 4; ++k) ha.kd[k] = keep_tiled ? keep[k] : nullptr;
     for (int k = 0; k < 3; ++k) ha.kt[k] = keep_tiled && c.variant == TTI_TENSOR ? keep[4 + k] : nullptr;
-    CK(h, tiled::launch_stress(ha, c.variant, h->exact, h->stream));
+    tiled::set_work(ha, h->fold_post ? post : Extent());
+    CK(h, tiled::launch_stress(ha, h->tmaps, c.variant, h->exact, h->stream));
   } else {
     launch_stress(a, h->stream);
   }
+  h->launches++;
   if (ev) CK(h, cudaEventRecord(ev[3], h->stream));
-  h->launches += 2 + vsrc;
-  // free surface, stress source and receivers: one column-parallel launch
-  const bool rec_now = c.seistype > 0 && it % c.mt == 0 && h->nrec[0] + h->nrec[1] + h->nrec[2] > 0;
-  if (c.freesurface == 1 || ssrc || rec_now) {
-    PostArgs pa;
-    pa.freesurface = c.freesurface;
-    pa.stype = ssrc ? 1 : 0;
-    pa.tensor = c.variant == TTI_TENSOR;
-    pa.it = it;
-    pa.irec = rec_now ? it / c.mt : -1;
-    pa.src = s;
-    memcpy(pa.k1, tab.k1, sizeof pa.k1);
-    const bool want_v = c.seistype == 1 || c.seistype == 3, want_p = c.seistype == 2 || c.seistype == 3;
-    for (int k = 0; k < 3; ++k) {
-      const bool on = (k < 2 ? want_v : want_p) && h->nrec[k] > 0;
-      pa.colptr[k] = on ? h->d_rcol[k] : nullptr;
-      pa.rz[k] = h->d_rzs[k];
-      pa.rid[k] = h->d_rid[k];
-      pa.rec[k] = h->d_rec[k];
-      pa.nrec[k] = h->nrec[k];
-    }
-    pa.flag = h->d_flag;
-    launch_post(a, pa, h->stream);
+  if (post.x1 > 0 && !h->fold_post) {
+    cs.x0 = post.x0;
+    cs.x1 = post.x1;
+    CK(h, launch_post(cs, n, h->stream));
     h->launches++;
   }
   if (c.energy == 1) {
@@ -366,13 +410,13 @@ int do_snapshot(tti_handle *h, tti_snapshot_fn fn, void *user, int it)
 
 // The time loop of tti_run after the reset; device time between events
 // ev0 and ev1. A snapshot of the last snapshot step may still be in flight.
-int run_steps(tti_handle *h, const SourceTables &tab, tti_snapshot_fn snap, void *user)
+int run_steps(tti_handle *h, tti_snapshot_fn snap, void *user)
 {
   const tti_config &c = h->cfg;
   CK(h, cudaEventRecord(h->ev0, h->stream));
   for (int n = 0; n < c.nt; ++n) {
     const int it = current_it(h);
-    int rc = launch_one_step(h, tab);
+    int rc = launch_one_step(h);
     if (rc == TTI_OK && snap && c.wsave > 0 && it % c.snap_sample == 0) rc = do_snapshot(h, snap, user, it);
     if (rc) return rc;
   }
@@ -472,10 +516,9 @@ int keep_fields(const tti_handle *h)
 }
 StepArgs handle_step_args(const tti_handle *h) { return step_args(h); }
 void handle_source_tables(const tti_handle *h, SourceTables *t) { source_tables(h, t); }
-int handle_step(tti_handle *h, const SourceTables &tab, float *const *keep)
-{
-  return launch_one_step(h, tab, nullptr, keep);
-}
+int handle_step(tti_handle *h, float *const *keep) { return launch_one_step(h, nullptr, keep); }
+int handle_columns(tti_handle *h) { return sync_columns(h); }
+Extent handle_post_extent(const tti_handle *h) { return post_extent(h, true); }
 int handle_check_flag(tti_handle *h) { return check_flag(h); }
 int handle_error(tti_handle *h, int code, const char *msg) { return set_err(h, code, "%s", msg); }
 }  // namespace ttifd
@@ -625,6 +668,7 @@ int tti_destroy(tti_handle *h)
   }
   pool_free(h->d_snap, fs);
   pool_free(h->d_stage, fs);
+  pool_free(h->d_cols, fs);
   if (fs) cudaStreamSynchronize(fs);
   grad_release(h);
   free(h->h_snap);
@@ -821,11 +865,15 @@ int tti_set_source(tti_handle *h, int ntrace, const int *posx, const int *posz, 
   h->d_sx = h->d_sz = nullptr;
   h->d_src = nullptr;
   h->nsrc = 0;
+  h->cols_dirty = true;
+  h->src_at = Extent();
   if (ntrace == 0) return TTI_OK;
   std::vector<int> x(ntrace), z(ntrace);
   for (int i = 0; i < ntrace; ++i) {
     x[i] = posx[i] + h->g.E;
     z[i] = posz[i] + h->g.E;
+    h->src_at.add(std::max(0, x[i] - NH), std::min(h->g.Nx, x[i] + NH + 1), std::max(0, z[i] - NH),
+                  std::min(h->g.Nz, z[i] + NH + 1));
   }
   CK(h, pool_alloc(reinterpret_cast<void **>(&h->d_sx), sizeof(int) * ntrace, h->stream));
   CK(h, pool_alloc(reinterpret_cast<void **>(&h->d_sz), sizeof(int) * ntrace, h->stream));
@@ -861,6 +909,8 @@ int tti_set_receivers(tti_handle *h, int kind, int ntrace, const int *posx, cons
   h->d_rz[kind] = h->d_rzs[kind] = h->d_rid[kind] = h->d_rcol[kind] = nullptr;
   h->d_rec[kind] = nullptr;
   h->nrec[kind] = 0;
+  h->cols_dirty = true;
+  h->rec_of[kind] = Extent();
   if (ntrace == 0) return TTI_OK;
   const int Nx = h->g.Nx;
   std::vector<int> blk(3 * (size_t)ntrace + Nx + 1, 0), x(ntrace), order(ntrace);
@@ -868,6 +918,7 @@ int tti_set_receivers(tti_handle *h, int kind, int ntrace, const int *posx, cons
   for (int i = 0; i < ntrace; ++i) {
     x[i] = posx[i] + h->g.E;
     z[i] = posz[i] + h->g.E;
+    h->rec_of[kind].add(x[i], x[i] + 1, z[i], z[i] + 1);
   }
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return x[a] < x[b]; });
@@ -912,11 +963,10 @@ int tti_step(tti_handle *h, int nsteps)
   if (!h->have_model) return set_err(h, TTI_ERR_STATE, "model not uploaded");
   if (h->step_index + nsteps > h->cfg.nt) return set_err(h, TTI_ERR_STATE, "step past nt");
   CK(h, cudaSetDevice(h->device));
-  SourceTables tab;
-  source_tables(h, &tab);
+  if (int rc = sync_columns(h)) return rc;
   CK(h, cudaEventRecord(h->ev0, h->stream));
   for (int n = 0; n < nsteps; ++n) {
-    int rc = launch_one_step(h, tab);
+    int rc = launch_one_step(h);
     if (rc) return rc;
   }
   CK(h, cudaEventRecord(h->ev1, h->stream));
@@ -948,9 +998,8 @@ int tti_run(tti_handle *h, tti_snapshot_fn snap, void *user)
   if (!h->have_model) return set_err(h, TTI_ERR_STATE, "model not uploaded");
   int rc = tti_reset(h);
   if (rc) return rc;
-  SourceTables tab;
-  source_tables(h, &tab);
-  rc = run_steps(h, tab, snap, user);
+  if ((rc = sync_columns(h))) return rc;
+  rc = run_steps(h, snap, user);
   if (rc) {
     finish_snapshot(h, false);
     return rc;
@@ -967,11 +1016,10 @@ int tti_profile_steps(tti_handle *h, int nsteps, float ms[3])
   CK(h, cudaSetDevice(h->device));
   for (int k = 0; k < 5; ++k)
     if (!h->pev[k]) CK(h, cudaEventCreate(&h->pev[k]));
-  SourceTables tab;
-  source_tables(h, &tab);
+  if (int rc = sync_columns(h)) return rc;
   ms[0] = ms[1] = ms[2] = 0.0f;
   for (int n = 0; n < nsteps; ++n) {
-    int rc = launch_one_step(h, tab, h->pev);
+    int rc = launch_one_step(h, h->pev);
     if (rc) return rc;
     CK(h, cudaEventSynchronize(h->pev[4]));
     float t01, t12, t23, t34;

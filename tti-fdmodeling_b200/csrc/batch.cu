@@ -29,16 +29,16 @@ struct tti_batch {
   std::vector<tti_handle *> models;  // model m's handle is also its first instance
   std::vector<tti_handle *> inst;
   std::vector<int> model_of;
-  int max_nt = 0, max_Nx = 0;
-  bool any_vsrc = false;
+  int max_nt = 0;
   bool square = false;  // every instance uses the folded coefficients (FMA mode, dx == dz)
   // device tables (fixed addresses: a captured graph refers to them)
   tiled::HalfArgs *d_vel = nullptr, *d_str = nullptr;
   tiled::Work *d_work = nullptr;
   int nwork = 0;
-  BatchPost *d_post = nullptr;
-  BatchSrc *d_src = nullptr;
-  SourceTables *d_tab = nullptr;
+  tiled::VelocityMaps *d_vmaps = nullptr;
+  tiled::StressMaps *d_smaps = nullptr;
+  ColumnShot *d_post = nullptr, *d_src = nullptr;  // column work: instances that have some, after either half-step
+  int npost = 0, nsrc = 0, post_cols = 0, src_cols = 0;  // their number, their widest
   int *d_step = nullptr;
   int group = 0;  // work-table order: shots of a model interleaved tile by tile in groups of `group` (0: all)
   bool persistent = false;  // one resident wave of CTAs walks the work table (else one CTA per item)
@@ -106,72 +106,37 @@ int build_tables(tti_batch *b)
 {
   const int n = (int)b->inst.size(), nm = (int)b->models.size();
   std::vector<tiled::HalfArgs> vel(n), str(n);
-  std::vector<BatchPost> post(n);
-  std::vector<BatchSrc> src(n);
-  std::vector<SourceTables> tab(nm);
-  for (int m = 0; m < nm; ++m) handle_source_tables(b->models[m], &tab[m]);
+  std::vector<tiled::VelocityMaps> vmaps(n);
+  std::vector<tiled::StressMaps> smaps(n);
+  std::vector<ColumnShot> post, src;
+  const int cols0 = b->src_cols, cols1 = b->post_cols;
+  b->src_cols = b->post_cols = 0;
   std::vector<dim3> tiles(n);
   bool all_square = true;
   sync_instances(b);
   for (int i = 0; i < n; ++i) {
     tti_handle *h = b->inst[i];
-    const tti_config &c = h->cfg;
+    if (const int rc = handle_columns(h)) return berr(b, rc, "%s", h->err.c_str());
     const StepArgs a = handle_step_args(h);
-    tiled::HalfArgs ha{};
-    memset(&ha, 0, sizeof ha);
-    ha.g = h->g;
-    ha.f = a.f;
-    ha.p = a.p;
-    ha.invdx = h->invdx;
-    ha.invdz = h->invdz;
-    ha.dt = c.dt;
-    const dim3 gr = tiled::tiles(h->g, h->g.izStart, &ha.z_base, &ha.tile_rows);
-    ha.x_base = NH;
-    ha.undamped_ok = h->undamped_ok;
-    ha.freesurface = c.freesurface;
+    tiled::HalfArgs ha;
+    tiled::fill_args(ha, h, a);
     tiled::set_square(ha, b->exact);
     all_square = all_square && ha.square;
-    ha.wait_limit = h->wait_limit;
-    ha.err = h->d_flag;
-    tiles[i] = gr;
+    int z_base, rows;
+    tiles[i] = tiled::tiles(h->g, h->g.izStart, &z_base, &rows);
     vel[i] = ha;
     str[i] = ha;
-    tiled::set_half(vel[i], static_cast<const CUtensorMap *>(h->tmaps), c.variant, true);
-    tiled::set_half(str[i], static_cast<const CUtensorMap *>(h->tmaps), c.variant, false);
-    SourceSet s{h->nsrc, h->d_sx, h->d_sz, h->d_src, c.nt};
-    BatchPost &bp = post[i];
-    memset(&bp, 0, sizeof bp);
-    bp.g = h->g;
-    bp.f = a.f;
-    bp.p.freesurface = c.freesurface;
-    bp.p.stype = s.n > 0 && c.stype == 1 ? 1 : 0;
-    bp.p.tensor = c.variant == TTI_TENSOR;
-    bp.p.src = s;
-    memcpy(bp.p.k1, tab[b->model_of[i]].k1, sizeof bp.p.k1);
-    const bool want_v = c.seistype == 1 || c.seistype == 3, want_p = c.seistype == 2 || c.seistype == 3;
-    for (int k = 0; k < 3; ++k) {
-      const bool on = (k < 2 ? want_v : want_p) && h->nrec[k] > 0;
-      bp.p.colptr[k] = on ? h->d_rcol[k] : nullptr;
-      bp.p.rz[k] = h->d_rzs[k];
-      bp.p.rid[k] = h->d_rid[k];
-      bp.p.rec[k] = h->d_rec[k];
-      bp.p.nrec[k] = h->nrec[k];
+    tiled::velocity_maps(vmaps[i], h->tmaps);
+    tiled::stress_maps(smaps[i], h->tmaps);
+    const Extent &se = h->src_at, pe = handle_post_extent(h);
+    if (h->nsrc > 0 && h->cfg.stype >= 2) {
+      src.push_back(ColumnShot{h->g, a.f, h->d_cols, se.x0, se.x1});
+      b->src_cols = std::max(b->src_cols, se.x1 - se.x0);
     }
-    bp.p.flag = h->d_flag;
-    bp.nt = c.nt;
-    bp.mode2 = c.mode == 2;
-    bp.mt = c.mt;
-    bp.rec_on = c.seistype > 0 && h->nrec[0] + h->nrec[1] + h->nrec[2] > 0;
-    BatchSrc &bs = src[i];
-    memset(&bs, 0, sizeof bs);
-    bs.g = h->g;
-    bs.f = a.f;
-    bs.s = s;
-    bs.tab = b->d_tab + b->model_of[i];
-    bs.variant = c.variant;
-    bs.stype = c.stype >= 2 ? c.stype : 0;
-    bs.nt = c.nt;
-    bs.mode2 = c.mode == 2;
+    if (pe.x1 > 0) {
+      post.push_back(ColumnShot{h->g, a.f, h->d_cols, pe.x0, pe.x1});
+      b->post_cols = std::max(b->post_cols, pe.x1 - pe.x0);
+    }
   }
   // work table: per model, per group of its instances, tile by tile
   std::vector<tiled::Work> work;
@@ -192,18 +157,24 @@ int build_tables(tti_batch *b)
         }
   }
   if ((int)work.size() != b->nwork) return berr(b, TTI_ERR_STATE, "work table size changed");
-  if (all_square != b->square && b->exec) {  // the captured launches select the kernels
+  if ((all_square != b->square || (int)post.size() != b->npost || (int)src.size() != b->nsrc || cols0 != b->src_cols ||
+       cols1 != b->post_cols) && b->exec) {  // the captured launches select the kernels and their grids
     cudaGraphExecDestroy(b->exec);
     cudaGraphDestroy(b->graph);
     b->exec = nullptr;
     b->graph = nullptr;
   }
   b->square = all_square;
+  b->npost = (int)post.size();
+  b->nsrc = (int)src.size();
   BCK(b, cudaMemcpyAsync(b->d_vel, vel.data(), sizeof(tiled::HalfArgs) * n, cudaMemcpyHostToDevice, b->stream));
   BCK(b, cudaMemcpyAsync(b->d_str, str.data(), sizeof(tiled::HalfArgs) * n, cudaMemcpyHostToDevice, b->stream));
-  BCK(b, cudaMemcpyAsync(b->d_post, post.data(), sizeof(BatchPost) * n, cudaMemcpyHostToDevice, b->stream));
-  BCK(b, cudaMemcpyAsync(b->d_src, src.data(), sizeof(BatchSrc) * n, cudaMemcpyHostToDevice, b->stream));
-  BCK(b, cudaMemcpyAsync(b->d_tab, tab.data(), sizeof(SourceTables) * nm, cudaMemcpyHostToDevice, b->stream));
+  BCK(b, cudaMemcpyAsync(b->d_vmaps, vmaps.data(), sizeof(vmaps[0]) * n, cudaMemcpyHostToDevice, b->stream));
+  BCK(b, cudaMemcpyAsync(b->d_smaps, smaps.data(), sizeof(smaps[0]) * n, cudaMemcpyHostToDevice, b->stream));
+  if (!post.empty())
+    BCK(b, cudaMemcpyAsync(b->d_post, post.data(), sizeof(post[0]) * post.size(), cudaMemcpyHostToDevice, b->stream));
+  if (!src.empty())
+    BCK(b, cudaMemcpyAsync(b->d_src, src.data(), sizeof(src[0]) * src.size(), cudaMemcpyHostToDevice, b->stream));
   BCK(b, cudaMemcpyAsync(b->d_work, work.data(), sizeof(tiled::Work) * work.size(), cudaMemcpyHostToDevice,
                          b->stream));
   BCK(b, cudaStreamSynchronize(b->stream));
@@ -213,7 +184,7 @@ int build_tables(tti_batch *b)
 // Launch description of a half-step (`vel`: the velocity tables, else the stress ones).
 tiled::BatchLaunch batch_launch(const tti_batch *b, bool vel, int offset)
 {
-  return tiled::BatchLaunch{vel ? b->d_vel : b->d_str, b->d_work, b->nwork, b->d_step, offset, b->variant, b->exact,
+  return tiled::BatchLaunch{vel ? b->d_vel : b->d_str, vel ? (const void *)b->d_vmaps : b->d_smaps, b->d_work, b->nwork, b->d_step, offset, b->variant, b->exact,
                             b->square, b->inst[0]->wait_limit, b->persistent};
 }
 
@@ -221,19 +192,18 @@ tiled::BatchLaunch batch_launch(const tti_batch *b, bool vel, int offset)
 // step's offset to the device counter, which moves on once at the end.
 int launch_steps(tti_batch *b, int n)
 {
-  const int ni = (int)b->inst.size();
   for (int k = 0; k < n; ++k) {
     BCK(b, tiled::launch_velocity_batch(batch_launch(b, true, k), b->stream));
-    if (b->any_vsrc) BCK(b, launch_sources_batch(b->d_src, ni, b->d_step, k, b->stream));
+    if (b->nsrc) BCK(b, launch_sources_batch(b->d_src, b->nsrc, b->src_cols, b->d_step, k, b->stream));
     BCK(b, tiled::launch_stress_batch(batch_launch(b, false, k), b->stream));
-    BCK(b, launch_post_batch(b->d_post, ni, b->max_Nx, b->d_step, k, b->stream));
+    if (b->npost) BCK(b, launch_post_batch(b->d_post, b->npost, b->post_cols, b->d_step, k, b->stream));
   }
   BCK(b, launch_advance(b->d_step, n, b->stream));
   return TTI_OK;
 }
 
 // kernels of launch_steps(n)
-int launches_of(const tti_batch *b, int n) { return n * (3 + (b->any_vsrc ? 1 : 0)) + 1; }
+int launches_of(const tti_batch *b, int n) { return n * (2 + (b->nsrc > 0) + (b->npost > 0)) + 1; }
 
 int ensure_graph(tti_batch *b)
 {
@@ -283,7 +253,8 @@ int tti_batch_destroy(tti_batch *b)
   cudaFree(b->d_work);
   cudaFree(b->d_post);
   cudaFree(b->d_src);
-  cudaFree(b->d_tab);
+  cudaFree(b->d_vmaps);
+  cudaFree(b->d_smaps);
   cudaFree(b->d_step);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
@@ -348,14 +319,13 @@ int tti_batch_create(tti_batch **out, int nmodels, const tti_config *cfg, int ni
     const dim3 gr = tiled::tiles(g, g.izStart, &zb, &rows);
     b->nwork += (int)(gr.x * gr.y);
     b->max_nt = std::max(b->max_nt, b->inst[i]->cfg.nt);
-    b->max_Nx = std::max(b->max_Nx, b->inst[i]->g.Nx);
-    b->any_vsrc = b->any_vsrc || b->inst[i]->cfg.stype >= 2;
   }
   const bool ok = cudaMalloc(&b->d_vel, sizeof(tiled::HalfArgs) * ninst) == cudaSuccess &&
                   cudaMalloc(&b->d_str, sizeof(tiled::HalfArgs) * ninst) == cudaSuccess &&
-                  cudaMalloc(&b->d_post, sizeof(BatchPost) * ninst) == cudaSuccess &&
-                  cudaMalloc(&b->d_src, sizeof(BatchSrc) * ninst) == cudaSuccess &&
-                  cudaMalloc(&b->d_tab, sizeof(SourceTables) * nmodels) == cudaSuccess &&
+                  cudaMalloc(&b->d_vmaps, sizeof(tiled::VelocityMaps) * ninst) == cudaSuccess &&
+                  cudaMalloc(&b->d_smaps, sizeof(tiled::StressMaps) * ninst) == cudaSuccess &&
+                  cudaMalloc(&b->d_post, sizeof(ColumnShot) * ninst) == cudaSuccess &&
+                  cudaMalloc(&b->d_src, sizeof(ColumnShot) * ninst) == cudaSuccess &&
                   cudaMalloc(&b->d_work, sizeof(tiled::Work) * (size_t)std::max(1, b->nwork)) == cudaSuccess &&
                   cudaMalloc(&b->d_step, sizeof(int)) == cudaSuccess;
   if (!ok) {

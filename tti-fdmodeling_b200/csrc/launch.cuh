@@ -60,43 +60,33 @@ struct StepArgs {
 
 void launch_velocity(const StepArgs &a, cudaStream_t st);
 void launch_stress(const StepArgs &a, cudaStream_t st);
-void launch_free_surface(const StepArgs &a, cudaStream_t st);
-// stage 0: velocity sources (stype 2..8), stage 1: stress source (stype 1)
-void launch_sources(const StepArgs &a, const SourceSet &s, const SourceTables *tab, int stype, int stage, int it,
-                    cudaStream_t st);
-void launch_receivers(const StepArgs &a, const ReceiverSet &r, int seistype, int irec, int *flag, cudaStream_t st);
 void launch_energy(const StepArgs &a, int nz, int nx, double *out2, cudaStream_t st);
-// free surface + stress source (stype 1) + receiver samples, one thread per column
-struct PostArgs {
-  int freesurface, stype, tensor, it, irec;
+
+// A shot's sources, receivers and the rest of its column work (columns.cuh),
+// in device memory; rebuilt when its geometry changes.
+struct Columns {
+  int stype;  // 0: no sources
+  int freesurface, tensor, nt, mode2, mt, rec_on;
   SourceSet src;
-  float k1[121];
+  SourceTables t;
   const int *colptr[3], *rz[3], *rid[3];  // receivers grouped by column (null: component off)
   float *rec[3];
   int nrec[3];
   int *flag;
 };
-void launch_post(const StepArgs &a, const PostArgs &p, cudaStream_t st);
-
-// ---------------- batched (many instances per launch) ----------------
-// Per-instance arguments in device memory; the time index comes from the
-// shared step counter `step` plus the launch's offset (it = that, or nt - 1 -
-// that for mode 2), and an instance whose nt has been reached does nothing.
-struct BatchPost {
+// One shot's column work as launches of their own (batched shots, and where
+// the tiles do not cover it): one warp per column of [x0, x1), step n (batched:
+// *step + n, shots past their nt do nothing, at most `cols` columns each).
+struct ColumnShot {
   Grid g;
   Fields f;
-  PostArgs p;  // it / irec unused
-  int nt, mode2, mt, rec_on;
+  const Columns *c;
+  int x0, x1;
 };
-struct BatchSrc {
-  Grid g;
-  Fields f;
-  SourceSet s;
-  const SourceTables *tab;  // device
-  int variant, stype, nt, mode2;
-};
-cudaError_t launch_post_batch(const BatchPost *d, int n, int maxNx, const int *step, int offset, cudaStream_t st);
-cudaError_t launch_sources_batch(const BatchSrc *d, int n, const int *step, int offset, cudaStream_t st);
+cudaError_t launch_post(const ColumnShot &s, int n, cudaStream_t st);
+cudaError_t launch_sources(const ColumnShot &s, int n, cudaStream_t st);
+cudaError_t launch_post_batch(const ColumnShot *d, int ns, int cols, const int *step, int n, cudaStream_t st);
+cudaError_t launch_sources_batch(const ColumnShot *d, int ns, int cols, const int *step, int n, cudaStream_t st);
 cudaError_t launch_advance(int *step, int n, cudaStream_t st);
 // dst[f][0..n) = src[f][0..n), f < 5 (n a multiple of 4, 16-byte aligned arrays)
 // the first nf (<= 5) of the arrays src[] into dst[], n floats each, one launch
@@ -113,7 +103,10 @@ void handle_source_tables(const tti_handle *h, SourceTables *t);
 int handle_check_flag(tti_handle *h);
 // one time step; `keep` (5 device arrays or null) receives vx vz sxx szz sxz
 // between the velocity sources and the stress update
-int handle_step(tti_handle *h, const SourceTables &tab, float *const *keep);  // keep: 8 pointers or null
+int handle_step(tti_handle *h, float *const *keep);  // keep: 8 pointers or null
+// brings the handle's Columns on the device up to date with its geometry
+int handle_columns(tti_handle *h);
+Extent handle_post_extent(const tti_handle *h);  // the cells of its work after the stress update
 // Fields of one kept step of the gradient (the arrays `keep` of handle_step
 // points at). Tiled kernels: the strain rates vxx vxz vzx vzz, then for the
 // coordinate rotation the stress derivative combinations P Q R S (8 fields),

@@ -1,9 +1,8 @@
 // Per-step kernels of the RSG time loop: velocity and stress updates along
-// the two grid diagonals, free surface, sources, receivers, energy, snapshot
-// packing.
+// the two grid diagonals, the column work, energy, snapshot packing.
 #include <algorithm>
 
-#include "launch.cuh"
+#include "columns.cuh"
 
 namespace ttifd {
 
@@ -139,139 +138,10 @@ __global__ void __launch_bounds__(BZ *BX) k_stress(Grid g, Fields f, Params p, f
   }
 }
 
-// coord:847-863: stress image about row s = izStart
-__global__ void k_free_surface(Grid g, Fields f)
-{
-  const int ix = NH + blockIdx.x * blockDim.x + threadIdx.x;
-  if (ix >= g.Nx - NH) return;
-  const size_t c = (size_t)ix * g.ldz + g.izStart;
-  f.sxz[c] = 0.0f;
-  f.szz[c] = 0.0f;
-  const float sxx0 = f.sxx[c];
-#pragma unroll
-  for (int k = 1; k <= NH; ++k) {
-    f.sxx[c - k] = __fsub_rn(__fmul_rn(2.0f, sxx0), f.sxx[c + k]);
-    f.szz[c - k] = -f.szz[c + k];
-    f.sxz[c - k] = -f.sxz[c + k];
-  }
-}
-
-__device__ __forceinline__ void acc(float *p, float k, float a) { *p = __fadd_rn(*p, __fmul_rn(k, a)); }
-__device__ __forceinline__ void dec(float *p, float k, float a) { *p = __fsub_rn(*p, __fmul_rn(k, a)); }
-
-// Sources over their 11 x 11 windows, one thread per window cell. Sources are
-// applied one after another (a barrier between them) so overlapping windows
-// accumulate in the reference's order; stype 8 runs on one thread.
-__device__ void sources_block(const Grid &g, const Fields &f, const SourceSet &s, const SourceTables &t, int variant,
-                              int stype, int stage, int it)
-{
-  const int tid = threadIdx.x;
-  if (stage == 0 && stype == 8) {
-    if (tid != 0) return;
-    for (int n = 0; n < s.n; ++n) {
-      const size_t c = (size_t)s.x[n] * g.ldz + s.z[n];
-      const float a = s.w[(size_t)n * s.nt + it];
-      const size_t L = g.ldz;
-      dec(f.vx + c, t.q8, a);
-      acc(f.vz + c, t.q8, a);
-      dec(f.vx + c - L, t.q8, a);
-      dec(f.vz + c - L, t.q8, a);
-      acc(f.vx + c - L - 1, t.q8, a);
-      dec(f.vz + c - L - 1, t.q8, a);
-      acc(f.vx + c - 1, t.q8, a);
-      acc(f.vz + c - 1, t.q8, a);
-    }
-    return;
-  }
-  int passes[2], np = 0;
-  if (stage == 0) {
-    if (stype == 2 || stype == 4) passes[np++] = 2;
-    if (stype == 3 || stype == 4) passes[np++] = 3;
-    if (stype >= 5 && stype <= 7) passes[np++] = stype;
-  } else if (stype == 1) {
-    passes[np++] = 1;
-  }
-  const int oa = tid / 11, ob = tid % 11;
-  for (int pidx = 0; pidx < np; ++pidx) {
-    const int kind = passes[pidx];
-    for (int n = 0; n < s.n; ++n) {
-      if (tid < 121) {
-        const int ix = s.x[n] + oa - NH, iz = s.z[n] + ob - NH;
-        if (ix >= 0 && ix < g.Nx && iz >= 0 && iz < g.Nz) {
-          const size_t c = (size_t)ix * g.ldz + iz;
-          const float a = s.w[(size_t)n * s.nt + it];
-          switch (kind) {
-          case 1:
-            acc(f.sxx + c, t.k1[tid], a);
-            acc(f.szz + c, t.k1[tid], a);
-            if (variant == TTI_TENSOR) {
-              acc(f.txx + c, t.k1[tid], a);
-              acc(f.tzz + c, t.k1[tid], a);
-            }
-            break;
-          case 2:
-            acc(f.vx + c, t.kx[tid], a);
-            acc(f.vz + c, t.kz[tid], a);
-            break;
-          case 3:
-            dec(f.vx + c, t.kz[tid], a);
-            acc(f.vz + c, t.kx[tid], a);
-            break;
-          case 5:
-            acc(f.vx + c, t.k5[tid], a);
-            break;
-          case 6:
-            acc(f.vz + c, t.k5[tid], a);
-            break;
-          case 7:
-            acc(f.vx + c, t.k7[tid], a);
-            acc(f.vz + c, t.k7[tid], a);
-            break;
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-__global__ void k_sources(Grid g, Fields f, SourceSet s, const __grid_constant__ SourceTables t, int variant, int stype,
-                          int stage, int it)
-{
-  pdl_sync();
-  sources_block(g, f, s, t, variant, stype, stage, it);
-}
-
-// Batched velocity sources: one block per instance, time index from the step counter.
-__global__ void k_sources_batch(const BatchSrc *bs, const int *step, int offset)
-{
-  const BatchSrc &b = bs[blockIdx.x];
-  pdl_sync();
-  const int n = *step + offset;
-  if (n >= b.nt || b.s.n == 0) return;
-  sources_block(b.g, b.f, b.s, *b.tab, b.variant, b.stype, 0, b.mode2 ? b.nt - 1 - n : n);
-}
-
 __global__ void k_advance(int *step, int n)
 {
   pdl_sync();
   *step += n;
-}
-
-// isoelastic.c:103-144; recorded time-major on the device ([irec][trace]).
-__global__ void k_receivers(Grid g, Fields f, ReceiverSet r, int want_v, int want_p, int irec, int *flag)
-{
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int k = blockIdx.y;
-  if (t >= r.n[k]) return;
-  if ((k < 2 && !want_v) || (k == 2 && !want_p)) return;
-  const size_t c = (size_t)r.x[k][t] * g.ldz + r.z[k][t];
-  float v;
-  if (k == TTI_REC_VX) v = f.vx[c];
-  else if (k == TTI_REC_VZ) v = f.vz[c];
-  else v = __fmul_rn(0.5f, __fadd_rn(f.sxx[c], f.szz[c]));
-  r.rec[k][(size_t)irec * r.n[k] + t] = v;
-  if (!isfinite(v)) atomicOr(flag, 1);
 }
 
 // coord:898-924, accumulated in double per step
@@ -302,131 +172,37 @@ __global__ void k_energy(Grid g, Fields f, Params p, int nz, int nx, double *out
   }
 }
 
-// After the stress update, one warp per padded-grid column applies, in the
-// reference's order for that column: the free-surface image (coord:847-863;
-// lanes 1-5 take the mirrored rows), the stress source stype 1 of each source
-// in turn (coord:865-886, tensor:871-895 also adds to tau; lanes over the 11
-// rows of the window), and the receiver samples (isoelastic.c:103-144; lanes
-// over the column's receivers). Columns do not interact, so one launch
-// replaces three; the warp makes each phase one memory round trip.
-// PDL: the warp reads the column's receiver geometry (static since the
-// receivers were set) before waiting for the previous kernel, so those loads
-// overlap its tail.
-__device__ void post_column(const Grid &g, const Fields &f, const PostArgs &p, int ix, int it, int irec,
-                            bool pdl = false)
+__device__ __forceinline__ int warp_column(const ColumnShot &s)
 {
-  const int lane = threadIdx.x & 31;
-  const size_t col = (size_t)ix * g.ldz;
-  // the first 32 receivers of each component in this column, one per lane
-  int rb[3] = {0, 0, 0}, re[3] = {0, 0, 0}, rzl[3] = {0, 0, 0}, ridl[3] = {0, 0, 0};
-  if (irec >= 0) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      if (p.colptr[k]) {
-        rb[k] = p.colptr[k][ix];
-        re[k] = p.colptr[k][ix + 1];
-      }
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      if (rb[k] + lane < re[k]) {
-        rzl[k] = p.rz[k][rb[k] + lane];
-        ridl[k] = p.rid[k][rb[k] + lane];
-      }
-  }
-  if (pdl) pdl_sync();
-  if (p.freesurface && ix >= NH && ix < g.Nx - NH) {
-    const size_t c = col + g.izStart;
-    const float sxx0 = f.sxx[c];
-    float xx = 0.0f, zz = 0.0f, xz = 0.0f;
-    if (lane >= 1 && lane <= NH) {
-      xx = f.sxx[c + lane];
-      zz = f.szz[c + lane];
-      xz = f.sxz[c + lane];
-    }
-    __syncwarp();
-    if (lane >= 1 && lane <= NH) {
-      f.sxx[c - lane] = __fsub_rn(__fmul_rn(2.0f, sxx0), xx);
-      f.szz[c - lane] = -zz;
-      f.sxz[c - lane] = -xz;
-    } else if (lane == 0) {
-      f.sxz[c] = 0.0f;
-      f.szz[c] = 0.0f;
-    }
-    __syncwarp();
-  }
-  if (p.stype == 1) {
-    for (int n = 0; n < p.src.n; ++n) {
-      const int dx = ix - p.src.x[n];
-      if (dx < -NH || dx > NH) continue;
-      const int iz = p.src.z[n] + lane - NH;
-      if (lane <= 2 * NH && iz >= 0 && iz < g.Nz) {
-        const float a = p.src.w[(size_t)n * p.src.nt + it];
-        const float ws = __fmul_rn(p.k1[(dx + NH) * 11 + lane], a);
-        const size_t c = col + iz;
-        f.sxx[c] = __fadd_rn(f.sxx[c], ws);
-        f.szz[c] = __fadd_rn(f.szz[c], ws);
-        if (p.tensor) {
-          f.txx[c] = __fadd_rn(f.txx[c], ws);
-          f.tzz[c] = __fadd_rn(f.tzz[c], ws);
-        }
-      }
-      __syncwarp();
-    }
-  }
-  if (irec >= 0) {
-    // all three components' samples loaded before any is stored
-    float v[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      if (rb[k] + lane >= re[k]) continue;
-      const size_t c = col + rzl[k];
-      if (k == TTI_REC_VX) v[k] = f.vx[c];
-      else if (k == TTI_REC_VZ) v[k] = f.vz[c];
-      else v[k] = __fmul_rn(0.5f, __fadd_rn(f.sxx[c], f.szz[c]));
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      if (rb[k] + lane >= re[k]) continue;
-      p.rec[k][(size_t)irec * p.nrec[k] + ridl[k]] = v[k];
-      if (!isfinite(v[k])) atomicOr(p.flag, 1);
-    }
-    // columns with more than 32 receivers of a component
-    for (int k = 0; k < 3; ++k)
-      for (int j = rb[k] + 32 + lane; j < re[k]; j += 32) {
-        const size_t c = col + p.rz[k][j];
-        float w;
-        if (k == TTI_REC_VX) w = f.vx[c];
-        else if (k == TTI_REC_VZ) w = f.vz[c];
-        else w = __fmul_rn(0.5f, __fadd_rn(f.sxx[c], f.szz[c]));
-        p.rec[k][(size_t)irec * p.nrec[k] + p.rid[k][j]] = w;
-        if (!isfinite(w)) atomicOr(p.flag, 1);
-      }
-  }
+  return s.x0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
 }
 
-__global__ void k_post(Grid g, Fields f, PostArgs p)
+__global__ void k_post(ColumnShot s, int n)
 {
-  const int ix = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (ix >= g.Nx) {
-    pdl_sync();
-    return;
-  }
-  post_column(g, f, p, ix, p.it, p.irec, true);
+  const int ix = warp_column(s);
+  if (ix < s.x1) column_post(s.g, s.f, *s.c, ix, n, 0, s.g.Nz, true);
+  else pdl_sync();
 }
-
-// Batched: blockIdx.y = instance; time index and receiver slot from the step counter.
-__global__ void k_post_batch(const BatchPost *bp, const int *step, int offset)
+__global__ void k_sources(ColumnShot s, int n)
 {
-  const BatchPost &b = bp[blockIdx.y];
   pdl_sync();
-  const int n = *step + offset;
-  if (n >= b.nt) return;
-  const int it = b.mode2 ? b.nt - 1 - n : n;
-  const int irec = b.rec_on && it % b.mt == 0 ? it / b.mt : -1;
-  if (!b.p.freesurface && b.p.stype != 1 && irec < 0) return;
-  const int ix = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (ix >= b.g.Nx) return;
-  post_column(b.g, b.f, b.p, ix, it, irec);
+  const int ix = warp_column(s);
+  if (ix < s.x1) column_sources(s.g, s.f, *s.c, ix, n, 0, s.g.Nz);
+}
+// Batched: blockIdx.y = shot.
+__global__ void k_post_batch(const ColumnShot *d, const int *step, int n)
+{
+  const ColumnShot &s = d[blockIdx.y];
+  pdl_sync();
+  const int k = *step + n, ix = warp_column(s);
+  if (k < s.c->nt && ix < s.x1) column_post(s.g, s.f, *s.c, ix, k, 0, s.g.Nz);
+}
+__global__ void k_sources_batch(const ColumnShot *d, const int *step, int n)
+{
+  const ColumnShot &s = d[blockIdx.y];
+  pdl_sync();
+  const int k = *step + n, ix = warp_column(s);
+  if (k < s.c->nt && ix < s.x1) column_sources(s.g, s.f, *s.c, ix, k, 0, s.g.Nz);
 }
 
 __global__ void k_snapshot(Grid g, Fields f, int kind, int x0, int z0, int nzo, int nxo, float *dst)
@@ -468,49 +244,26 @@ static dim3 interior_grid(const Grid &g)
 void launch_velocity(const StepArgs &a, cudaStream_t st) { TTI_DISPATCH(k_velocity, a, st); }
 void launch_stress(const StepArgs &a, cudaStream_t st) { TTI_DISPATCH(k_stress, a, st); }
 
-void launch_free_surface(const StepArgs &a, cudaStream_t st)
-{
-  const int n = a.g.Nx - 2 * NH;
-  if (n <= 0) return;
-  k_free_surface<<<(n + 127) / 128, 128, 0, st>>>(a.g, a.f);
-}
-
-void launch_sources(const StepArgs &a, const SourceSet &s, const SourceTables *tab, int stype, int stage, int it,
-                    cudaStream_t st)
-{
-  if (s.n <= 0) return;
-  if (stage == 0 && (stype < 2 || stype > 8)) return;
-  if (stage == 1 && stype != 1) return;
-  launch_pdl(k_sources, dim3(1), dim3(128), 0, st, a.g, a.f, s, *tab, a.variant, stype, stage, it);
-}
-
-void launch_receivers(const StepArgs &a, const ReceiverSet &r, int seistype, int irec, int *flag, cudaStream_t st)
-{
-  const int want_v = seistype == 1 || seistype == 3, want_p = seistype == 2 || seistype == 3;
-  int nmax = 0;
-  for (int k = 0; k < 3; ++k) nmax = r.n[k] > nmax ? r.n[k] : nmax;
-  if (nmax == 0) return;
-  k_receivers<<<dim3((nmax + 127) / 128, 3), 128, 0, st>>>(a.g, a.f, r, want_v, want_p, irec, flag);
-}
-
 void launch_energy(const StepArgs &a, int nz, int nx, double *out2, cudaStream_t st)
 {
   k_energy<<<296, 256, 0, st>>>(a.g, a.f, a.p, nz, nx, out2);
 }
 
-void launch_post(const StepArgs &a, const PostArgs &p, cudaStream_t st)
+cudaError_t launch_post(const ColumnShot &s, int n, cudaStream_t st)
 {
-  launch_pdl(k_post, dim3((a.g.Nx + 3) / 4), dim3(128), 0, st, a.g, a.f, p);  // 4 columns (warps) per block
+  return launch_pdl(k_post, dim3((s.x1 - s.x0 + 3) / 4), dim3(128), 0, st, s, n);  // 4 columns (warps) per block
 }
-
-cudaError_t launch_post_batch(const BatchPost *d, int n, int maxNx, const int *step, int offset, cudaStream_t st)
+cudaError_t launch_sources(const ColumnShot &s, int n, cudaStream_t st)
 {
-  return launch_pdl(k_post_batch, dim3((maxNx + 3) / 4, n), dim3(128), 0, st, d, step, offset);
+  return launch_pdl(k_sources, dim3((s.x1 - s.x0 + 3) / 4), dim3(128), 0, st, s, n);
 }
-
-cudaError_t launch_sources_batch(const BatchSrc *d, int n, const int *step, int offset, cudaStream_t st)
+cudaError_t launch_post_batch(const ColumnShot *d, int ns, int cols, const int *step, int n, cudaStream_t st)
 {
-  return launch_pdl(k_sources_batch, dim3(n), dim3(128), 0, st, d, step, offset);
+  return launch_pdl(k_post_batch, dim3((cols + 3) / 4, ns), dim3(128), 0, st, d, step, n);
+}
+cudaError_t launch_sources_batch(const ColumnShot *d, int ns, int cols, const int *step, int n, cudaStream_t st)
+{
+  return launch_pdl(k_sources_batch, dim3((cols + 3) / 4, ns), dim3(128), 0, st, d, step, n);
 }
 
 // up to five state arrays copied in one launch (the gradient's kept states)

@@ -9,17 +9,21 @@
 namespace ttifd {
 namespace tiled {
 
-// A handle's tensor maps: the halo boxes of vx vz sxx szz
-// sxz, then the tile inputs of the stress update (HalfArgs::in).
+// A handle's tensor maps: the halo boxes of vx vz sxx szz sxz, then the tile
+// inputs of the stress update: coordinate sxx szz sxz sin cos c11 c13 c33 c55;
+// tensor txx tzz txz sin^2 cos^2 c11 c13 c33 c55 sin2theta; Bond sxx szz sxz
+// c15 c35 c11 c13 c33 c55.
 constexpr int HALO_MAPS = 5, IN_MAPS = 10, MAPS = HALO_MAPS + IN_MAPS;
+struct alignas(64) VelocityMaps {
+  CUtensorMap box[3];  // sxx szz sxz
+};
+struct alignas(64) StressMaps {
+  CUtensorMap box[2];  // vx vz
+  CUtensorMap in[IN_MAPS];
+};
 constexpr int AHEAD = 7;  // entries of HalfArgs::ahead
 
-struct alignas(64) HalfArgs {
-  CUtensorMap map[3];  // velocity update: sxx szz sxz; stress update: vx vz
-  // The stress update's own inputs. Coordinate sxx szz sxz sin cos c11 c13 c33
-  // c55; tensor txx tzz txz sin^2 cos^2 c11 c13 c33 c55 sin2theta; Bond sxx szz
-  // sxz c15 c35 c11 c13 c33 c55.
-  CUtensorMap in[IN_MAPS];
+struct alignas(16) HalfArgs {
   Grid g;
   Fields f;
   Params p;
@@ -45,13 +49,13 @@ struct alignas(64) HalfArgs {
   // invrho, coordinate also sin cos of theta_v, coef1, coef2
   const float *ahead[AHEAD];
   int nahead;
+  // Column work in the tiles: rows [work_z0, work_z1) have some (none: empty).
+  // After the velocity update the velocity sources, after the stress update the
+  // rest (columns.cuh), of step n (batched launches: from the step counter).
+  const Columns *cols;
+  int work_z0, work_z1;
+  int n;
 };
-
-// Encodes a handle's MAPS tensor maps.
-bool encode_maps(CUtensorMap *map, const Grid &g, int variant, const Fields &f, const Params &p);
-// Fills map, in and ahead for the velocity or the stress update from a handle's
-// maps (f and p set).
-void set_half(HalfArgs &a, const CUtensorMap *maps, int variant, bool velocity);
 
 // Sets square / hc for FMA-mode launches on grids with dx == dz.
 inline void set_square(HalfArgs &a, bool exact)
@@ -59,6 +63,18 @@ inline void set_square(HalfArgs &a, bool exact)
   a.square = !exact && a.invdx == a.invdz;
   for (int k = 0; k < 5; ++k) a.hc[k] = 0.5f * a.invdx * rsg(k);
   a.nzero = -0.0f;
+}
+
+// Encodes a handle's MAPS tensor maps.
+bool encode_maps(CUtensorMap *map, const Grid &g, int variant, const Fields &f, const Params &p);
+// The arguments of h's half-steps (a: handle_step_args), without column work.
+void fill_args(HalfArgs &ha, const tti_handle *h, const StepArgs &a);
+void velocity_maps(VelocityMaps &m, const void *maps);  // from a handle's maps
+void stress_maps(StressMaps &m, const void *maps);
+inline void set_work(HalfArgs &ha, const Extent &e)
+{
+  ha.work_z0 = e.x1 > 0 ? e.z0 : 0;
+  ha.work_z1 = e.x1 > 0 ? e.z1 : 0;
 }
 
 // One item of a batched launch: instance, tile origin (x0 with the UNDAMPED
@@ -83,12 +99,14 @@ bool encode_map3(CUtensorMap *map, const Grid &g, float *fields, int count, int 
 // Tile grid over rows z_first .. Nz - NH - 1: *z_base receives the first tile
 // row, *tile_rows the height of a tile.
 dim3 tiles(const Grid &g, int z_first, int *z_base, int *tile_rows);
-cudaError_t launch_velocity(const HalfArgs &a, int variant, bool exact, cudaStream_t st);
-cudaError_t launch_stress(const HalfArgs &a, int variant, bool exact, cudaStream_t st);
+// (maps: the handle's)
+cudaError_t launch_velocity(const HalfArgs &a, const void *maps, int variant, bool exact, cudaStream_t st);
+cudaError_t launch_stress(const HalfArgs &a, const void *maps, int variant, bool exact, cudaStream_t st);
 // Batched: one launch over all instances' tiles (each instance's arguments
 // with z_base set), driven by the work table.
 struct BatchLaunch {
-  const HalfArgs *inst;  // device: each instance's arguments (velocity or stress maps)
+  const HalfArgs *inst;  // device: each instance's arguments
+  const void *maps;      // device: each instance's VelocityMaps or StressMaps
   const Work *work;      // device: the CTA -> (instance, tile) table
   int nwork;
   const int *step;       // device: the shared step counter

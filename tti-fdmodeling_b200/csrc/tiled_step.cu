@@ -26,11 +26,11 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
-#include <cstddef>
 #include <cstring>
 #include <mutex>
 #include <vector>
 
+#include "columns.cuh"
 #include "walk.cuh"
 
 namespace ttifd {
@@ -41,6 +41,7 @@ namespace {
 // arguments of a batched half-step launch
 struct BatchArgs {
   const HalfArgs *inst;  // each instance's arguments
+  const void *maps;      // each instance's VelocityMaps or StressMaps
   const Work *work;      // the work table
   const int *step;       // the shared step counter
   int nwork, offset;     // offset: steps past the counter
@@ -205,11 +206,23 @@ __device__ __forceinline__ void read_sums(const Cells &c, const float *sums, F4 
   }
 }
 
+// Column work in the tiles instead of a launch between the half-steps: us a
+// step with and without, 60 x 80 9.1 / 9.8, 200 x 400 11.6 / 14.3, 600 x 1200
+// 19.2 / 20.2, 1126 x 7872 147.1 / 150.6.
+// The rows whose column work a tile does: its own, the first and the last tile
+// also those above and below all tiles.
+__device__ __forceinline__ bool tile_work(const HalfArgs &a, const Cells &c, int &r0, int &r1)
+{
+  r0 = c.z0 == a.z_base ? 0 : c.z0;
+  r1 = c.z0 + a.tile_rows >= a.g.Nz - NH ? a.g.Nz : c.z0 + a.tile_rows;
+  return r0 < a.work_z1 && r1 > a.work_z0;
+}
+
 // Velocity update of a tile whose boxes (sxx, szz, sxz) have arrived: one warp
 // per field and 32 diagonals, then one per column.
 template <int V, bool X, bool Q, bool K>
 __device__ __forceinline__ void velocity_tile(const HalfArgs &a, const Cells &c, bool und, const walk::Coefs &k,
-                                              float *sm)
+                                              float *sm, int n)
 {
   const int gr = walk::groups(a.tile_rows);
   float *sums = sm + V_SUMS;
@@ -230,6 +243,11 @@ __device__ __forceinline__ void velocity_tile(const HalfArgs &a, const Cells &c,
     F4 ds[3][2];
     read_sums(c, sums, ds);
     velocity_rows<V, X, Q, K>(a, c, gi, ds, p, k.nz);
+  }
+  int r0, r1;
+  if (tile_work(a, c, r0, r1)) {  // this warp's column
+    __syncwarp();
+    if (c.x < a.g.Nx - NH) column_sources(a.g, a.f, *a.cols, c.x, n, r0, r1);
   }
 }
 
@@ -343,7 +361,7 @@ __device__ __forceinline__ void stress_rows(const HalfArgs &a, const Cells &c, s
 // Stress update of a tile whose boxes (vx, vz) and inputs have arrived
 template <int V, bool X, bool Q, bool K>
 __device__ __forceinline__ void stress_tile(const HalfArgs &a, const Cells &c, bool und, const walk::Coefs &k,
-                                            float *sm)
+                                            float *sm, int n)
 {
   const int gr = walk::groups(a.tile_rows), t = threadIdx.x >> 5, f = t >= gr;
   const int d = (t - f * gr) * 32 + (threadIdx.x & 31);
@@ -365,23 +383,29 @@ __device__ __forceinline__ void stress_tile(const HalfArgs &a, const Cells &c, b
     load_scells<V>(a, und, c, gi, sm, p);
     stress_rows<V, X, Q, K>(a, c, gi, ds, p, k.nz);
   }
+  int r0, r1;
+  if (tile_work(a, c, r0, r1)) {  // this warp's column
+    __syncwarp();
+    if (c.x < a.g.Nx - NH) column_post(a.g, a.f, *a.cols, c.x, n, r0, r1);
+  }
 }
 
 // Single-shot launches, one tile per CTA.
 template <int V, bool X, bool Q, bool K = false>
-__global__ void __launch_bounds__(walk::NT, 4) k_velocity_tiled(const __grid_constant__ HalfArgs a)
+__global__ void __launch_bounds__(walk::NT, 4) k_velocity_tiled(const __grid_constant__ HalfArgs a,
+                                                                const __grid_constant__ VelocityMaps m)
 {
   extern __shared__ __align__(128) float sm[];
   unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + V_BAR);
   const int z0 = a.z_base + blockIdx.x * a.tile_rows, x0 = a.x_base + blockIdx.y * WX;
   walk::init_bar(bar);
   pdl_sync();
-  walk::issue_tile(a.map, 3, 4, nullptr, 0, 0, sm, 0, bar, z0, x0);
+  walk::issue_tile(m.box, 3, 4, nullptr, 0, 0, sm, 0, bar, z0, x0);
   const bool und = tile_undamped(a, z0, x0, WX);
   prefetch_velocity(a, und, z0, x0);
   const walk::Coefs k = coefs<Q>(a, a.nzero);
   if (!walk::wait_boxes(a.err, bar, a.wait_limit, 0)) return;
-  velocity_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm);
+  velocity_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, a.n);
 }
 
 // The stress update walks the tiles in the opposite order, so that it starts
@@ -389,7 +413,8 @@ __global__ void __launch_bounds__(walk::NT, 4) k_velocity_tiled(const __grid_con
 // in L2 (and the next velocity update starts where this one ended): 67.7
 // against 70.3 us a step at 1126 x 3000, 160.3 against 162.7 at 1126 x 7872.
 template <int V, bool X, bool Q, bool K = false>
-__global__ void __launch_bounds__(walk::NT, K ? 3 : 4) k_stress_tiled(const __grid_constant__ HalfArgs a)
+__global__ void __launch_bounds__(walk::NT, K ? 3 : 4) k_stress_tiled(const __grid_constant__ HalfArgs a,
+                                                                      const __grid_constant__ StressMaps m)
 {
   extern __shared__ __align__(128) float sm[];
   unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + s_bar(V));
@@ -397,30 +422,26 @@ __global__ void __launch_bounds__(walk::NT, K ? 3 : 4) k_stress_tiled(const __gr
   const int x0 = a.x_base + (gridDim.y - 1 - blockIdx.y) * WX;
   walk::init_bar(bar);
   pdl_sync();
-  walk::issue_tile(a.map, 2, 5, a.in, s_inputs(V), a.tile_rows, sm, S_IN, bar, z0, x0);
+  walk::issue_tile(m.box, 2, 5, m.in, s_inputs(V), a.tile_rows, sm, S_IN, bar, z0, x0);
   const bool und = tile_undamped(a, z0, x0, WX);
   prefetch_stress(a, und, z0, x0);
   const walk::Coefs k = coefs<Q>(a, a.nzero);
   if (!walk::wait_boxes(a.err, bar, a.wait_limit, 0)) return;
-  stress_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm);
+  stress_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, a.n);
 }
 
-// Batched launches copy the instance's arguments (less the tensor maps, which
-// TMA reads from global memory) into shared memory: the fields are then uniform shared loads that the in-place global stores cannot alias.
+// Batched launches copy the instance's arguments into shared memory: the fields
+// are then uniform shared loads that the in-place global stores cannot alias.
 // The copy runs while the boxes are in flight and is complete after the block
 // barrier of wait_boxes.
-constexpr size_t ARGS_HEAD = offsetof(HalfArgs, g);  // the tensor maps come first
-constexpr size_t ARGS_BYTES = sizeof(HalfArgs) - ARGS_HEAD;
-static_assert(ARGS_BYTES % 16 == 0 && ARGS_HEAD % 16 == 0, "HalfArgs must be whole 16-byte words");
+static_assert(sizeof(HalfArgs) % 16 == 0, "HalfArgs must be whole 16-byte words");
 
 __device__ __forceinline__ const HalfArgs &stage_args(const HalfArgs *src, void *dst)
 {
-  // the copy's (absent) tensor maps would start this far before the copied words
-  char *base = static_cast<char *>(dst) - ARGS_HEAD;
   const int4 *s4 = reinterpret_cast<const int4 *>(src);
-  int4 *d4 = reinterpret_cast<int4 *>(base);
-  for (int i = ARGS_HEAD / 16 + threadIdx.x; i < (int)(sizeof(HalfArgs) / 16); i += walk::NT) d4[i] = __ldg(s4 + i);
-  return *reinterpret_cast<const HalfArgs *>(base);
+  int4 *d4 = static_cast<int4 *>(dst);
+  for (int i = threadIdx.x; i < (int)(sizeof(HalfArgs) / 16); i += walk::NT) d4[i] = __ldg(s4 + i);
+  return *static_cast<const HalfArgs *>(dst);
 }
 
 // One work item: the copies need only the item (its tile origin) and the
@@ -436,10 +457,10 @@ __device__ __forceinline__ bool work_item(const BatchArgs &b, int i, int n, unsi
   const HalfArgs *src = b.inst + w.x;
   const int x0 = w.z & ~Work::UNDAMPED;
   const bool und = w.z & Work::UNDAMPED;
-  issue(*src, und, w.y, x0);
+  issue(*src, w.x, und, w.y, x0);
   const HalfArgs &a = stage_args(src, bar + 2);
   if (!walk::wait_boxes(src->err, bar, b.wait_limit, ph)) return false;
-  f(a, cells_of(a, w.y, x0), und);
+  f(a, cells_of(a, w.y, x0), und, n);
   ph ^= 1;
   return true;
 }
@@ -473,12 +494,12 @@ __global__ void __launch_bounds__(walk::NT, 4) k_velocity_batch(const __grid_con
   unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + V_BAR);
   for_work<LOOP>(
       b, false, bar,
-      [&](const HalfArgs &a, bool und, int z0, int x0) {
-        walk::issue_tile(a.map, 3, 4, nullptr, 0, 0, sm, 0, bar, z0, x0);
+      [&](const HalfArgs &a, int inst, bool und, int z0, int x0) {
+        walk::issue_tile(static_cast<const VelocityMaps *>(b.maps)[inst].box, 3, 4, nullptr, 0, 0, sm, 0, bar, z0, x0);
         prefetch_velocity(a, und, z0, x0);
       },
-      [&](const HalfArgs &a, const Cells &c, bool und) {
-        velocity_tile<V, X, Q, false>(a, c, und, coefs<Q>(a, b.nzero), sm);
+      [&](const HalfArgs &a, const Cells &c, bool und, int n) {
+        velocity_tile<V, X, Q, false>(a, c, und, coefs<Q>(a, b.nzero), sm, n);
       });
 }
 
@@ -489,12 +510,13 @@ __global__ void __launch_bounds__(walk::NT, 4) k_stress_batch(const __grid_const
   unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + s_bar(V));
   for_work<LOOP>(
       b, true, bar,
-      [&](const HalfArgs &a, bool und, int z0, int x0) {
-        walk::issue_tile(a.map, 2, 5, a.in, s_inputs(V), a.tile_rows, sm, S_IN, bar, z0, x0);
+      [&](const HalfArgs &a, int inst, bool und, int z0, int x0) {
+        const StressMaps &m = static_cast<const StressMaps *>(b.maps)[inst];
+        walk::issue_tile(m.box, 2, 5, m.in, s_inputs(V), threadIdx.x ? 0 : a.tile_rows, sm, S_IN, bar, z0, x0);
         prefetch_stress(a, und, z0, x0);
       },
-      [&](const HalfArgs &a, const Cells &c, bool und) {
-        stress_tile<V, X, Q, false>(a, c, und, coefs<Q>(a, b.nzero), sm);
+      [&](const HalfArgs &a, const Cells &c, bool und, int n) {
+        stress_tile<V, X, Q, false>(a, c, und, coefs<Q>(a, b.nzero), sm, n);
       });
 }
 
@@ -530,17 +552,16 @@ cudaError_t prepare_kernel(K kernel, size_t bytes, int *wave)
   return cudaSuccess;
 }
 
-template <typename K>
-cudaError_t launch_k(K kernel, const HalfArgs &a, int variant, bool velocity, cudaStream_t st)
+template <typename M>
+cudaError_t launch_k(void (*kernel)(HalfArgs, M), const HalfArgs &a, const M &m, size_t smem, cudaStream_t st)
 {
-  const size_t bytes = (size_t)((velocity ? V_BAR : s_bar(variant)) + 16) * sizeof(float);
   int wave = 0;
-  cudaError_t e = prepare_kernel(kernel, bytes, &wave);
+  const cudaError_t e = prepare_kernel(kernel, smem, &wave);
   if (e != cudaSuccess) return e;
-  HalfArgs b = a;
-  const dim3 gr = tiles(a.g, a.g.izStart, &b.z_base, &b.tile_rows);
+  int z_base, rows;
+  const dim3 gr = tiles(a.g, a.g.izStart, &z_base, &rows);
   if (gr.x == 0 || gr.y == 0) return cudaSuccess;
-  return launch_pdl(kernel, gr, dim3(walk::NT), bytes, st, b);
+  return launch_pdl(kernel, gr, dim3(walk::NT), smem, st, a, m);
 }
 
 }  // namespace
@@ -612,57 +633,84 @@ bool encode_maps(CUtensorMap *map, const Grid &g, int variant, const Fields &f, 
   return true;
 }
 
-void set_half(HalfArgs &a, const CUtensorMap *maps, int variant, bool velocity)
+void fill_args(HalfArgs &ha, const tti_handle *h, const StepArgs &a)
 {
-  std::copy_n(maps + (velocity ? 2 : 0), 3, a.map);
-  std::copy_n(maps + HALO_MAPS, IN_MAPS, a.in);
-  const Params &p = a.p;
-  std::vector<const float *> v;
-  if (velocity) {
-    v = {a.f.vx, a.f.vz, p.invrho};
-    if (variant == TTI_COORDINATE) v.insert(v.end(), {p.snv, p.csv});
-    v.insert(v.end(), {p.coef1, p.coef2});
-  }
-  a.nahead = (int)v.size();
-  for (int k = 0; k < AHEAD; ++k) a.ahead[k] = k < a.nahead ? v[k] : nullptr;
+  const tti_config &c = h->cfg;
+  ha = HalfArgs{};
+  ha.g = h->g;
+  ha.f = a.f;
+  ha.p = a.p;
+  ha.invdx = h->invdx;
+  ha.invdz = h->invdz;
+  ha.dt = c.dt;
+  tiles(h->g, h->g.izStart, &ha.z_base, &ha.tile_rows);
+  ha.x_base = NH;
+  ha.undamped_ok = h->undamped_ok;
+  ha.freesurface = c.freesurface;
+  set_square(ha, h->exact);
+  ha.wait_limit = h->wait_limit;
+  ha.err = h->d_flag;
+  ha.cols = h->d_cols;
+  for (const float *q : {(const float *)a.f.vx, (const float *)a.f.vz, a.p.invrho}) ha.ahead[ha.nahead++] = q;
+  if (c.variant == TTI_COORDINATE)
+    for (const float *q : {a.p.snv, a.p.csv}) ha.ahead[ha.nahead++] = q;
+  for (const float *q : {a.p.coef1, a.p.coef2}) ha.ahead[ha.nahead++] = q;
+}
+
+void velocity_maps(VelocityMaps &m, const void *maps)
+{
+  std::copy_n(static_cast<const CUtensorMap *>(maps) + 2, 3, m.box);
+}
+void stress_maps(StressMaps &m, const void *maps)
+{
+  const CUtensorMap *t = static_cast<const CUtensorMap *>(maps);
+  std::copy_n(t, 2, m.box);
+  std::copy_n(t + HALO_MAPS, IN_MAPS, m.in);
 }
 
 template <bool X, bool Q>
-cudaError_t velocity_xq(const HalfArgs &a, int variant, cudaStream_t st)
+cudaError_t velocity_xq(const HalfArgs &a, const VelocityMaps &m, int variant, cudaStream_t st)
 {
-  if (variant == TTI_COORDINATE && a.kd[0]) return launch_k(k_velocity_tiled<TTI_COORDINATE, X, Q, true>, a, variant, true, st);
-  if (variant == TTI_COORDINATE) return launch_k(k_velocity_tiled<TTI_COORDINATE, X, Q>, a, variant, true, st);
-  if (variant == TTI_TENSOR) return launch_k(k_velocity_tiled<TTI_TENSOR, X, Q>, a, variant, true, st);
-  return launch_k(k_velocity_tiled<TTI_BOND, X, Q>, a, variant, true, st);
-}
-
-template <bool X, bool Q>
-cudaError_t stress_xq(const HalfArgs &a, int variant, cudaStream_t st)
-{
-  const bool k = a.kd[0] != nullptr;
+  constexpr size_t smem = (size_t)(V_BAR + 16) * sizeof(float);
   if (variant == TTI_COORDINATE)
-    return k ? launch_k(k_stress_tiled<TTI_COORDINATE, X, Q, true>, a, variant, false, st)
-             : launch_k(k_stress_tiled<TTI_COORDINATE, X, Q>, a, variant, false, st);
-  if (variant == TTI_TENSOR)
-    return k ? launch_k(k_stress_tiled<TTI_TENSOR, X, Q, true>, a, variant, false, st)
-             : launch_k(k_stress_tiled<TTI_TENSOR, X, Q>, a, variant, false, st);
-  return k ? launch_k(k_stress_tiled<TTI_BOND, X, Q, true>, a, variant, false, st) : launch_k(k_stress_tiled<TTI_BOND, X, Q>, a, variant, false, st);
+    return a.kd[0] ? launch_k(k_velocity_tiled<TTI_COORDINATE, X, Q, true>, a, m, smem, st)
+                   : launch_k(k_velocity_tiled<TTI_COORDINATE, X, Q>, a, m, smem, st);
+  if (variant == TTI_TENSOR) return launch_k(k_velocity_tiled<TTI_TENSOR, X, Q>, a, m, smem, st);
+  return launch_k(k_velocity_tiled<TTI_BOND, X, Q>, a, m, smem, st);
 }
 
-cudaError_t launch_velocity(const HalfArgs &a, int variant, bool exact, cudaStream_t st)
+template <int V, bool X, bool Q>
+cudaError_t stress_vxq(const HalfArgs &a, const StressMaps &m, cudaStream_t st)
 {
-  if (exact) return velocity_xq<true, false>(a, variant, st);
-  return a.square ? velocity_xq<false, true>(a, variant, st) : velocity_xq<false, false>(a, variant, st);
+  constexpr size_t smem = (size_t)(s_bar(V) + 16) * sizeof(float);
+  return a.kd[0] ? launch_k(k_stress_tiled<V, X, Q, true>, a, m, smem, st)
+                 : launch_k(k_stress_tiled<V, X, Q>, a, m, smem, st);
+}
+template <bool X, bool Q>
+cudaError_t stress_xq(const HalfArgs &a, const StressMaps &m, int variant, cudaStream_t st)
+{
+  if (variant == TTI_COORDINATE) return stress_vxq<TTI_COORDINATE, X, Q>(a, m, st);
+  return variant == TTI_TENSOR ? stress_vxq<TTI_TENSOR, X, Q>(a, m, st) : stress_vxq<TTI_BOND, X, Q>(a, m, st);
 }
 
-cudaError_t launch_stress(const HalfArgs &a, int variant, bool exact, cudaStream_t st)
+cudaError_t launch_velocity(const HalfArgs &a, const void *maps, int variant, bool exact, cudaStream_t st)
 {
-  if (exact) return stress_xq<true, false>(a, variant, st);
-  return a.square ? stress_xq<false, true>(a, variant, st) : stress_xq<false, false>(a, variant, st);
+  VelocityMaps m;
+  velocity_maps(m, maps);
+  if (exact) return velocity_xq<true, false>(a, m, variant, st);
+  return a.square ? velocity_xq<false, true>(a, m, variant, st) : velocity_xq<false, false>(a, m, variant, st);
+}
+
+cudaError_t launch_stress(const HalfArgs &a, const void *maps, int variant, bool exact, cudaStream_t st)
+{
+  StressMaps m;
+  stress_maps(m, maps);
+  if (exact) return stress_xq<true, false>(a, m, variant, st);
+  return a.square ? stress_xq<false, true>(a, m, variant, st) : stress_xq<false, false>(a, m, variant, st);
 }
 
 // shared memory of a batched kernel whose barrier is at float `bar`
-constexpr size_t batch_smem(int bar) { return (size_t)(bar + 4) * sizeof(float) + ARGS_BYTES; }
+constexpr size_t batch_smem(int bar) { return (size_t)(bar + 4) * sizeof(float) + sizeof(HalfArgs); }
 
 // One CTA per work item, or (persistent) one resident wave of CTAs that walks
 // the table: the SM count times the kernel's CTAs per SM at its shared memory.
@@ -673,7 +721,7 @@ cudaError_t launch_batch_k(K one, K loop, size_t smem, const BatchLaunch &l, cud
   int wave = 0;
   cudaError_t e = prepare_kernel(kernel, smem, &wave);
   if (e != cudaSuccess || l.nwork == 0) return e;
-  const BatchArgs b{l.inst, l.work, l.step, l.nwork, l.offset, -0.0f, l.wait_limit};
+  const BatchArgs b{l.inst, l.maps, l.work, l.step, l.nwork, l.offset, -0.0f, l.wait_limit};
   return launch_pdl(kernel, dim3(l.persistent ? std::min(l.nwork, wave) : l.nwork), dim3(walk::NT), smem, st, b);
 }
 

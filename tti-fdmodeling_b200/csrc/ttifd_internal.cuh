@@ -128,11 +128,23 @@ constexpr size_t PIN_CHUNK = (size_t)4 << 20;
 float *pinned_chunk();
 void pinned_release(float *p);
 
-struct ReceiverSet {
-  int n[3];
-  const int *x[3], *z[3];  // padded-grid cells
-  float *rec[3];           // time-major on the device: [nts][n]
+// columns [x0, x1) and rows [z0, z1) of the padded grid that something touches
+struct Extent {
+  int x0 = 1 << 30, x1 = 0, z0 = 1 << 30, z1 = 0;
+  void add(int xa, int xb, int za, int zb)
+  {
+    x0 = xa < x0 ? xa : x0;
+    x1 = xb > x1 ? xb : x1;
+    z0 = za < z0 ? za : z0;
+    z1 = zb > z1 ? zb : z1;
+  }
+  void add(const Extent &e)
+  {
+    if (e.x1 > 0) add(e.x0, e.x1, e.z0, e.z1);
+  }
 };
+
+struct Columns;
 
 }  // namespace ttifd
 
@@ -162,6 +174,11 @@ struct tti_handle {
   int *d_rz[3] = {};  // receiver rows in the caller's order; owns the block d_rzs, d_rid, d_rcol point into
   float *d_rec[3] = {};
   int nts = 0;
+  ttifd::Columns *d_cols = nullptr;  // sources and receivers for the column work
+  bool cols_dirty = true;            // the geometry changed since d_cols was filled
+  ttifd::Extent src_at, rec_at;      // cells of the source windows; of the receivers (handle_columns)
+  ttifd::Extent rec_of[3];           // receivers by component
+  bool fold_src = false, fold_post = false;  // the tiled kernels do the column work (else launches of its own)
   double *d_energy = nullptr;  // [nt][2]
   int *d_flag = nullptr;       // nonfinite watchdog
   float *d_snap = nullptr;      // packed snapshot kinds of one step, snap_cap floats
