@@ -1542,15 +1542,9 @@ int grad_start_adjoint(tti_handle *h, double *J)
 int forward_steps(tti_handle *h, int k0, int k1, bool record)
 {
   GradState *s = h->grad;
-  const int nk = s->nkeep;
-  for (int k = k0; k < k1; ++k) {
-    float *keep[8] = {};
-    if (record)
-      for (int f = 0; f < nk; ++f) keep[f] = s->keep + ((size_t)(k - k0) * nk + f) * h->g.n;
-    const int rc = handle_step(h, record ? keep : nullptr);
-    if (rc) return rc;
-  }
-  return TTI_OK;
+  float *keep[8] = {};
+  for (int f = 0; f < s->nkeep; ++f) keep[f] = s->keep + f * h->g.n;
+  return handle_steps(h, k1, record ? keep : nullptr, s->nkeep * h->g.n);
 }
 
 int adjoint_steps(tti_handle *h, int k0, int k1, const SourceTables &tab)

@@ -104,6 +104,16 @@ void source_tables(const tti_handle *h, SourceTables *t)
   t->q8 = 0.125f * sqrtf(2.0f);
 }
 
+// A single shot's steps go out as replays of a graph of GRAPH_STEPS steps where
+// the grid is one wave of tiles (4 a SM on 148 SMs) or less: there the kernels
+// are shorter than the host's launches or little longer, and the gaps between
+// them show. us a step by replays / by launches: 60 x 80 8.05 / 9.2, 200 x 400
+// 10.8 / 12.0, 300 x 600 12.3 / 13.3, 400 x 800 (440 tiles) 13.7 / 14.4. Above,
+// a replay is hardly faster (600 x 1200, 960 tiles, 18.9 / 19.1) and the first
+// run, which captures, slower (19.7 / 19.4). The capture costs what replays
+// save over 60 to 250 steps, so runs of fewer steps do without.
+constexpr int GRAPH_TILES = 4 * 148, GRAPH_NT = 200;
+
 int check_cfg(const tti_config *c)
 {
   if (c->variant < 0 || c->variant > 2) return set_err(nullptr, TTI_ERR_ARG, "variant must be 0, 1 or 2");
@@ -170,7 +180,6 @@ int sync_columns(tti_handle *h)
   };
   h->fold_src = w.stype >= 2 && fold(h->src_at);
   h->fold_post = fold(post);
-  if (!h->d_cols) CK(h, pool_alloc(reinterpret_cast<void **>(&h->d_cols), sizeof w, h->stream));
   CK(h, cudaMemcpyAsync(h->d_cols, &w, sizeof w, cudaMemcpyHostToDevice, h->stream));
   CK(h, cudaStreamSynchronize(h->stream));  // w goes out of scope
   h->cols_dirty = false;
@@ -189,59 +198,74 @@ Extent post_extent(const tti_handle *h, bool rec_now)
   return e;
 }
 
+// The arguments of one time step's tiled half-steps. What the gradient keeps
+// of a step (keep_fields): the stress kernel writes the strain rates vxx vxz
+// vzx vzz (keep[0..3]) and for the tensor rotation the tau it starts from
+// (keep[4..6]); the coordinate velocity kernel writes the stress derivative
+// combinations P Q R S (keep[4..7]).
+struct TiledStep {
+  tiled::HalfArgs v, s;
+};
+void tiled_step(const tti_handle *h, const Extent &post, float *const *keep, size_t stride, TiledStep &t)
+{
+  const int variant = h->cfg.variant;
+  memset(&t, 0, sizeof t);
+  tiled::fill_args(t.v, h, step_args(h));
+  t.v.n = t.v.k0 = h->step_index;
+  t.v.kstride = stride;
+  t.s = t.v;
+  if (h->fold_src) tiled::set_work(t.v, h->src_at);
+  if (h->fold_post) tiled::set_work(t.s, post);
+  if (!keep) return;
+  if (variant == TTI_COORDINATE)
+    for (int k = 0; k < 4; ++k) t.v.kd[k] = keep[4 + k];
+  for (int k = 0; k < 4; ++k) t.s.kd[k] = keep[k];
+  if (variant == TTI_TENSOR)
+    for (int k = 0; k < 3; ++k) t.s.kt[k] = keep[4 + k];
+}
+
 // Launches one time step (coord:611-926 body). With `ev` (5 events) the
 // phases are bracketed for tti_profile_steps: ev[0] | velocity | ev[1] |
 // velocity sources | ev[2] | stress | ev[3] | the rest | ev[4] (the sources
 // and the rest are empty where the half-step kernels do the column work). With
-// `keep` the gradient's forward pass keeps what the adjoint needs of the step.
-int launch_one_step(tti_handle *h, cudaEvent_t *ev = nullptr, float *const *keep = nullptr)
+// `keep` the gradient's forward pass keeps what the adjoint needs of the step
+// in slot step - k0; the per-cell kernels keep a copy of vx vz and sxx szz sxz
+// (tensor: txx tzz txz) after the sources, from whose stencils the adjoint
+// works.
+int launch_one_step(tti_handle *h, cudaEvent_t *ev = nullptr, float *const *keep = nullptr, size_t stride = 0,
+                    int k0 = 0)
 {
   const tti_config &c = h->cfg;
   const int it = current_it(h), n = h->step_index;
-  StepArgs a = step_args(h);
-  const bool vsrc = h->nsrc > 0 && c.stype >= 2;
+  const StepArgs a = step_args(h);
+  const Extent post = post_extent(h, it % c.mt == 0);
   ColumnShot cs{h->g, a.f, h->d_cols, h->src_at.x0, h->src_at.x1};
-  tiled::HalfArgs ha{};
-  // What the gradient keeps of this step (keep_fields). Tiled kernels: the
-  // stress kernel writes the strain rates vxx vxz vzx vzz (keep[0..3]) and for
-  // the tensor rotation the tau it starts from (keep[4..6]); the coordinate
-  // velocity kernel writes the stress derivative combinations P Q R S
-  // (keep[4..7]). Per-cell kernels: a copy of vx vz and sxx szz sxz (tensor:
-  // txx tzz txz) after the sources, from whose stencils the adjoint works.
-  const bool keep_tiled = keep && h->use_tiled;
+  TiledStep t;
   if (h->use_tiled) {
-    tiled::fill_args(ha, h, a);
-    ha.n = n;
-    if (h->fold_src) tiled::set_work(ha, h->src_at);
-    if (keep_tiled && c.variant == TTI_COORDINATE)
-      for (int k = 0; k < 4; ++k) ha.kd[k] = keep[4 + k];
+    tiled_step(h, post, keep, stride, t);
+    t.v.k0 = t.s.k0 = k0;
   }
   if (ev) CK(h, cudaEventRecord(ev[0], h->stream));
-  if (h->use_tiled) CK(h, tiled::launch_velocity(ha, h->tmaps, c.variant, h->exact, h->stream));
+  if (h->use_tiled) CK(h, tiled::launch_velocity(t.v, h->tmaps, c.variant, h->exact, h->stream));
   else launch_velocity(a, h->stream);
   h->launches++;
   if (ev) CK(h, cudaEventRecord(ev[1], h->stream));
-  if (vsrc && !h->fold_src) {
+  if (h->nsrc > 0 && c.stype >= 2 && !h->fold_src) {
     CK(h, launch_sources(cs, n, h->stream));
     h->launches++;
   }
-  if (keep && !keep_tiled) {  // v after the sources, and sigma or tau
-    const bool t = c.variant == TTI_TENSOR;
-    float *const src[5] = {h->fld[0], h->fld[1], h->fld[t ? 5 : 2], h->fld[t ? 6 : 3], h->fld[t ? 7 : 4]};
-    launch_copy5(src, keep, 5, h->g.n, h->stream);
+  if (keep && !h->use_tiled) {  // v after the sources, and sigma or tau
+    const bool ten = c.variant == TTI_TENSOR;
+    float *const src[5] = {h->fld[0], h->fld[1], h->fld[ten ? 5 : 2], h->fld[ten ? 6 : 3], h->fld[ten ? 7 : 4]};
+    float *dst[5];
+    for (int f = 0; f < 5; ++f) dst[f] = keep[f] + (size_t)(n - k0) * stride;
+    launch_copy5(src, dst, 5, h->g.n, h->stream);
     h->launches++;
   }
   if (ev) CK(h, cudaEventRecord(ev[2], h->stream));
   // after the stress update: free surface, stress source and receivers
-  const Extent post = post_extent(h, it % c.mt == 0);
-  if (h->use_tiled) {
-    for (int k = 0; k < 4; ++k) ha.kd[k] = keep_tiled ? keep[k] : nullptr;
-    for (int k = 0; k < 3; ++k) ha.kt[k] = keep_tiled && c.variant == TTI_TENSOR ? keep[4 + k] : nullptr;
-    tiled::set_work(ha, h->fold_post ? post : Extent());
-    CK(h, tiled::launch_stress(ha, h->tmaps, c.variant, h->exact, h->stream));
-  } else {
-    launch_stress(a, h->stream);
-  }
+  if (h->use_tiled) CK(h, tiled::launch_stress(t.s, h->tmaps, c.variant, h->exact, h->stream));
+  else launch_stress(a, h->stream);
   h->launches++;
   if (ev) CK(h, cudaEventRecord(ev[3], h->stream));
   if (post.x1 > 0 && !h->fold_post) {
@@ -257,6 +281,87 @@ int launch_one_step(tti_handle *h, cudaEvent_t *ev = nullptr, float *const *keep
   if (ev) CK(h, cudaEventRecord(ev[4], h->stream));
   CK(h, cudaGetLastError());
   h->step_index++;
+  return TTI_OK;
+}
+
+// Captures GRAPH_STEPS steps with the arguments t, whose step counters are on
+// the device; false when no graph could be made.
+bool capture_steps(tti_handle *h, StepGraph &g, TiledStep t)
+{
+  // relaxed for this thread: nothing here may spoil a capture that another
+  // thread has under way
+  struct Relaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  } relaxed;
+  if (g.exec) cudaGraphExecDestroy(g.exec);
+  g.exec = nullptr;
+  g.key.assign(reinterpret_cast<unsigned char *>(&t), reinterpret_cast<unsigned char *>(&t + 1));
+  if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; ++k) {
+    t.v.n = t.s.n = k;
+    e = tiled::launch_velocity(t.v, h->tmaps, h->cfg.variant, h->exact, h->stream);
+    if (e == cudaSuccess) e = tiled::launch_stress(t.s, h->tmaps, h->cfg.variant, h->exact, h->stream);
+  }
+  if (e == cudaSuccess) e = launch_advance(h->d_clk, GRAPH_STEPS, h->stream);
+  cudaGraph_t graph = nullptr;
+  const cudaError_t end = cudaStreamEndCapture(h->stream, &graph);
+  if (e == cudaSuccess) e = end;
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
+  if (graph) cudaGraphDestroy(graph);
+  if (e == cudaSuccess) return true;
+  cudaGetLastError();
+  g.exec = nullptr;
+  return false;
+}
+
+// As many whole graph replays as fit before step n1; the fields that are kept
+// belong to the segment from step k0. Where no graph can be made the handle
+// launches every step by itself from here on.
+int replay_steps(tti_handle *h, int n1, float *const *keep, size_t stride, int k0)
+{
+  const int n = h->step_index, steps = (n1 - n) / GRAPH_STEPS * GRAPH_STEPS;
+  if (steps == 0) return TTI_OK;
+  TiledStep t;
+  tiled_step(h, post_extent(h, true), keep, stride, t);
+  for (tiled::HalfArgs *a : {&t.v, &t.s}) {
+    a->clk = h->d_clk;
+    a->n = a->k0 = 0;
+  }
+  StepGraph &g = h->graph[keep != nullptr];
+  if (!g.exec || g.key.size() != sizeof t || memcmp(g.key.data(), &t, sizeof t) != 0)
+    if (!capture_steps(h, g, t)) {
+      h->use_graphs = false;
+      return TTI_OK;
+    }
+  const tiled::StepClock clk{n, k0};
+  CK(h, cudaMemcpyAsync(h->d_clk, &clk, sizeof clk, cudaMemcpyHostToDevice, h->stream));
+  for (int k = 0; k < steps; k += GRAPH_STEPS) CK(h, cudaGraphLaunch(g.exec, h->stream));
+  h->launches += 2 * steps + steps / GRAPH_STEPS;
+  h->step_index += steps;
+  return TTI_OK;
+}
+
+// Forward steps up to step n1 (see handle_steps): graph replays where the
+// handle uses them and every launch of a step is a half-step, single launches
+// for the rest. The first step of a run is never captured, so that its
+// kernels' attributes are set outside a capture.
+int run_forward(tti_handle *h, int n1, float *const *keep, size_t stride)
+{
+  const int k0 = h->step_index;
+  const bool whole = h->cfg.energy == 0 && (h->fold_post || post_extent(h, true).x1 == 0) &&
+                     (h->fold_src || h->nsrc == 0 || h->cfg.stype == 1);
+  while (h->step_index < n1) {
+    if (h->use_graphs && whole && h->step_index > k0)
+      if (const int rc = replay_steps(h, n1, keep, stride, k0)) return rc;
+    if (h->step_index < n1)
+      if (const int rc = launch_one_step(h, nullptr, keep, stride, k0)) return rc;
+  }
   return TTI_OK;
 }
 
@@ -414,10 +519,14 @@ int run_steps(tti_handle *h, tti_snapshot_fn snap, void *user)
 {
   const tti_config &c = h->cfg;
   CK(h, cudaEventRecord(h->ev0, h->stream));
-  for (int n = 0; n < c.nt; ++n) {
-    const int it = current_it(h);
-    int rc = launch_one_step(h);
-    if (rc == TTI_OK && snap && c.wsave > 0 && it % c.snap_sample == 0) rc = do_snapshot(h, snap, user, it);
+  const bool snaps = snap && c.wsave > 0;
+  while (h->step_index < c.nt) {
+    // up to and with the next step that has a snapshot
+    int n1 = snaps ? h->step_index : c.nt - 1;
+    auto it_of = [&](int n) { return c.mode == 2 ? c.nt - 1 - n : n; };
+    while (n1 < c.nt - 1 && it_of(n1) % c.snap_sample != 0) ++n1;
+    int rc = run_forward(h, n1 + 1, nullptr, 0);
+    if (rc == TTI_OK && snaps && it_of(n1) % c.snap_sample == 0) rc = do_snapshot(h, snap, user, it_of(n1));
     if (rc) return rc;
   }
   CK(h, cudaEventRecord(h->ev1, h->stream));
@@ -516,7 +625,7 @@ int keep_fields(const tti_handle *h)
 }
 StepArgs handle_step_args(const tti_handle *h) { return step_args(h); }
 void handle_source_tables(const tti_handle *h, SourceTables *t) { source_tables(h, t); }
-int handle_step(tti_handle *h, float *const *keep) { return launch_one_step(h, nullptr, keep); }
+int handle_steps(tti_handle *h, int n1, float *const *keep, size_t stride) { return run_forward(h, n1, keep, stride); }
 int handle_columns(tti_handle *h) { return sync_columns(h); }
 Extent handle_post_extent(const tti_handle *h) { return post_extent(h, true); }
 int handle_check_flag(tti_handle *h) { return check_flag(h); }
@@ -617,12 +726,18 @@ int create_handle(tti_handle **out, const tti_config *cfg, int device, const tti
       return fail(TTI_ERR_NOMEM);
     }
     const StepArgs a = step_args(h);
+    int z_base, rows;
+    const dim3 nt = tiled::tiles(g, g.izStart, &z_base, &rows);
+    const char *gs = getenv("TTIFD_GRAPH_STEPS");  // 0: every step by its own launches
+    h->use_graphs = (int)(nt.x * nt.y) <= GRAPH_TILES && cfg->nt >= GRAPH_NT && (!gs || atoi(gs) > 0);
     if (!tiled::encode_maps(static_cast<CUtensorMap *>(h->tmaps), g, cfg->variant, a.f, a.p)) {
       set_err(h, TTI_ERR_CUDA, "cuTensorMapEncodeTiled failed");
       return fail(TTI_ERR_CUDA);
     }
   }
-  if (pool_alloc(reinterpret_cast<void **>(&h->d_flag), sizeof(int), h->stream) != cudaSuccess ||
+  if (pool_alloc(reinterpret_cast<void **>(&h->d_clk), sizeof(tiled::StepClock), h->stream) != cudaSuccess ||
+      pool_alloc(reinterpret_cast<void **>(&h->d_cols), sizeof(Columns), h->stream) != cudaSuccess ||
+      pool_alloc(reinterpret_cast<void **>(&h->d_flag), sizeof(int), h->stream) != cudaSuccess ||
       pool_alloc(reinterpret_cast<void **>(&h->d_energy), sizeof(double) * 2 * (size_t)cfg->nt, h->stream) !=
           cudaSuccess) {
     set_err(h, TTI_ERR_NOMEM, "device allocation failed");
@@ -647,6 +762,8 @@ int tti_destroy(tti_handle *h)
   if (!h) return TTI_OK;
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
+  for (auto &g : h->graph)
+    if (g.exec) cudaGraphExecDestroy(g.exec);
   cudaStream_t fs = h->stream;  // pool blocks are released in stream order
   for (auto &p : h->fld) pool_free(p, fs);
   if (!h->owner) {
@@ -669,6 +786,7 @@ int tti_destroy(tti_handle *h)
   pool_free(h->d_snap, fs);
   pool_free(h->d_stage, fs);
   pool_free(h->d_cols, fs);
+  pool_free(h->d_clk, fs);
   if (fs) cudaStreamSynchronize(fs);
   grad_release(h);
   free(h->h_snap);
@@ -965,10 +1083,7 @@ int tti_step(tti_handle *h, int nsteps)
   CK(h, cudaSetDevice(h->device));
   if (int rc = sync_columns(h)) return rc;
   CK(h, cudaEventRecord(h->ev0, h->stream));
-  for (int n = 0; n < nsteps; ++n) {
-    int rc = launch_one_step(h);
-    if (rc) return rc;
-  }
+  if (const int rc = run_forward(h, h->step_index + nsteps, nullptr, 0)) return rc;
   CK(h, cudaEventRecord(h->ev1, h->stream));
   CK(h, cudaEventSynchronize(h->ev1));
   CK(h, cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));

@@ -101,9 +101,10 @@ void launch_snapshot(const StepArgs &a, int kind, int savew, float *dst, cudaStr
 StepArgs handle_step_args(const tti_handle *h);
 void handle_source_tables(const tti_handle *h, SourceTables *t);
 int handle_check_flag(tti_handle *h);
-// one time step; `keep` (5 device arrays or null) receives vx vz sxx szz sxz
-// between the velocity sources and the stress update
-int handle_step(tti_handle *h, float *const *keep);  // keep: 8 pointers or null
+// Steps [n0, n1) from the current state (the handle's step index is n0). With
+// `keep` what the adjoint needs of them goes to slot n - n0 of the kept steps:
+// keep[f] + slot * stride, f < keep_fields.
+int handle_steps(tti_handle *h, int n1, float *const *keep, size_t stride);
 // brings the handle's Columns on the device up to date with its geometry
 int handle_columns(tti_handle *h);
 Extent handle_post_extent(const tti_handle *h);  // the cells of its work after the stress update

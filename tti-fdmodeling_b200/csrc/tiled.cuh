@@ -42,7 +42,8 @@ struct alignas(16) HalfArgs {
   // rotation: per cell the stress derivative combinations the adjoint's
   // theta_v terms need (sxz_x - sxx_z, szz_x - sxz_z, sxx_x + sxz_z,
   // sxz_x + szz_z). Stress update: the strain rates vxx vxz vzx vzz (not
-  // rotated), and for the tensor rotation the tau it starts from (kt).
+  // rotated), and for the tensor rotation the tau it starts from (kt). Pointers
+  // to the first slot.
   float *kd[4];
   float *kt[3];
   // the arrays the velocity update reads per cell, for the L2 prefetch: vx vz
@@ -54,7 +55,18 @@ struct alignas(16) HalfArgs {
   // rest (columns.cuh), of step n (batched launches: from the step counter).
   const Columns *cols;
   int work_z0, work_z1;
-  int n;
+  // The step: n, or inside a graph clk[0] + n (StepClock). The gradient's kept
+  // steps: the slot of step k0 (graph: clk[1]) is kd and kt, the next ones
+  // kstride floats apart.
+  const int *clk;
+  int n, k0;
+  size_t kstride;
+};
+
+// A handle's device step counters for graphs of several steps: the step, and
+// the first step of the kept segment.
+struct StepClock {
+  int n, k0;
 };
 
 // Sets square / hc for FMA-mode launches on grids with dx == dz.

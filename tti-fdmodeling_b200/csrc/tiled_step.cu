@@ -120,6 +120,13 @@ static_assert(4 * walk::SUM <= 2 * walk::BOX, "the sums fit in place of the boxe
 constexpr int s_inputs(int V) { return V == TTI_TENSOR ? 10 : 9; }
 constexpr int s_bar(int V) { return S_IN + s_inputs(V) * walk::WZ * WX; }
 
+// this launch's step, and the offset of its slot among the kept steps
+__device__ __forceinline__ int step_of(const HalfArgs &a) { return a.clk ? a.clk[0] + a.n : a.n; }
+__device__ __forceinline__ size_t kept_at(const HalfArgs &a, int n)
+{
+  return (size_t)(n - (a.clk ? a.clk[1] : a.k0)) * a.kstride;
+}
+
 // per-cell inputs of the velocity update, four rows
 struct VCells {
   F4 vx, vz, c1, c2, ir, sv, cv;
@@ -142,7 +149,7 @@ __device__ __forceinline__ void load_vcells(const HalfArgs &a, bool und, size_t 
 // d2) of sxx, szz, sxz (coord:614-672, tensor:617-666, bond:654-703).
 template <int V, bool X, bool Q, bool K>
 __device__ __forceinline__ void velocity_rows(const HalfArgs &a, const Cells &c, size_t gi, const F4 (&d)[3][2],
-                                              const VCells &p, walk::u64 nz)
+                                              const VCells &p, walk::u64 nz, int n)
 {
   typedef walk::Rows<X> A;
   typedef typename A::T T;
@@ -189,9 +196,11 @@ __device__ __forceinline__ void velocity_rows(const HalfArgs &a, const Cells &c,
   const int lo = a.g.izStart, hi = min(a.g.Nz - NH, c.z0 + a.tile_rows);
   st4(a.f.vx + gi, vx, c.z, lo, hi);
   st4(a.f.vz + gi, vz, c.z, lo, hi);
-  if (K && V == TTI_COORDINATE)
+  if (K && V == TTI_COORDINATE) {
+    const size_t ki = kept_at(a, n) + gi;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) st4(a.kd[k] + gi, kd[k], c.z, lo, hi);
+    for (int k = 0; k < 4; ++k) st4(a.kd[k] + ki, kd[k], c.z, lo, hi);
+  }
 }
 
 // the sums of N fields at a thread's rows
@@ -242,7 +251,7 @@ __device__ __forceinline__ void velocity_tile(const HalfArgs &a, const Cells &c,
   if (c.on) {
     F4 ds[3][2];
     read_sums(c, sums, ds);
-    velocity_rows<V, X, Q, K>(a, c, gi, ds, p, k.nz);
+    velocity_rows<V, X, Q, K>(a, c, gi, ds, p, k.nz, n);
   }
   int r0, r1;
   if (tile_work(a, c, r0, r1)) {  // this warp's column
@@ -281,7 +290,7 @@ __device__ __forceinline__ void load_scells(const HalfArgs &a, bool und, const C
 // keeps of them goes to kd and kt.
 template <int V, bool X, bool Q, bool K>
 __device__ __forceinline__ void stress_rows(const HalfArgs &a, const Cells &c, size_t gi, const F4 (&d)[2][2],
-                                            const SCells &s, walk::u64 nz)
+                                            const SCells &s, walk::u64 nz, int step)
 {
   typedef walk::Rows<X> A;
   typedef typename A::T T;
@@ -298,11 +307,12 @@ __device__ __forceinline__ void stress_rows(const HalfArgs &a, const Cells &c, s
       A::set(e[2 * f + 1], i, Q ? m : r.mul(r.mul(half, m), invdz));
     }
   if (K) {
+    const size_t ki = kept_at(a, step) + gi;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) st4(a.kd[k] + gi, e[k], c.z, lo, hi);
+    for (int k = 0; k < 4; ++k) st4(a.kd[k] + ki, e[k], c.z, lo, hi);
     if (V == TTI_TENSOR)
 #pragma unroll
-      for (int k = 0; k < 3; ++k) st4(a.kt[k] + gi, s.o[k], c.z, lo, hi);
+      for (int k = 0; k < 3; ++k) st4(a.kt[k] + ki, s.o[k], c.z, lo, hi);
   }
   F4 n[3], t[3];
 #pragma unroll
@@ -381,7 +391,7 @@ __device__ __forceinline__ void stress_tile(const HalfArgs &a, const Cells &c, b
     read_sums(c, sums, ds);
     SCells p;
     load_scells<V>(a, und, c, gi, sm, p);
-    stress_rows<V, X, Q, K>(a, c, gi, ds, p, k.nz);
+    stress_rows<V, X, Q, K>(a, c, gi, ds, p, k.nz, n);
   }
   int r0, r1;
   if (tile_work(a, c, r0, r1)) {  // this warp's column
@@ -403,9 +413,10 @@ __global__ void __launch_bounds__(walk::NT, 4) k_velocity_tiled(const __grid_con
   walk::issue_tile(m.box, 3, 4, nullptr, 0, 0, sm, 0, bar, z0, x0);
   const bool und = tile_undamped(a, z0, x0, WX);
   prefetch_velocity(a, und, z0, x0);
+  const int n = step_of(a);
   const walk::Coefs k = coefs<Q>(a, a.nzero);
   if (!walk::wait_boxes(a.err, bar, a.wait_limit, 0)) return;
-  velocity_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, a.n);
+  velocity_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, n);
 }
 
 // The stress update walks the tiles in the opposite order, so that it starts
@@ -425,9 +436,10 @@ __global__ void __launch_bounds__(walk::NT, K ? 3 : 4) k_stress_tiled(const __gr
   walk::issue_tile(m.box, 2, 5, m.in, s_inputs(V), a.tile_rows, sm, S_IN, bar, z0, x0);
   const bool und = tile_undamped(a, z0, x0, WX);
   prefetch_stress(a, und, z0, x0);
+  const int n = step_of(a);
   const walk::Coefs k = coefs<Q>(a, a.nzero);
   if (!walk::wait_boxes(a.err, bar, a.wait_limit, 0)) return;
-  stress_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, a.n);
+  stress_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, n);
 }
 
 // Batched launches copy the instance's arguments into shared memory: the fields

@@ -6,6 +6,7 @@
 #include <stdlib.h>
 
 #include <string>
+#include <vector>
 
 #include "../../include/ttifd.h"
 
@@ -146,6 +147,15 @@ struct Extent {
 
 struct Columns;
 
+// A captured graph of GRAPH_STEPS steps and the arguments it was captured
+// with (anything else captures it again): one for plain steps, one for steps
+// whose fields the gradient keeps.
+constexpr int GRAPH_STEPS = 10;
+struct StepGraph {
+  cudaGraphExec_t exec = nullptr;
+  std::vector<unsigned char> key;
+};
+
 }  // namespace ttifd
 
 // Host-side handle (C ABI object).
@@ -179,6 +189,9 @@ struct tti_handle {
   ttifd::Extent src_at, rec_at;      // cells of the source windows; of the receivers (handle_columns)
   ttifd::Extent rec_of[3];           // receivers by component
   bool fold_src = false, fold_post = false;  // the tiled kernels do the column work (else launches of its own)
+  int *d_clk = nullptr;              // step counters for the graphs (tiled::StepClock)
+  ttifd::StepGraph graph[2];
+  bool use_graphs = false;           // steps by graph replays (create_handle)
   double *d_energy = nullptr;  // [nt][2]
   int *d_flag = nullptr;       // nonfinite watchdog
   float *d_snap = nullptr;      // packed snapshot kinds of one step, snap_cap floats
