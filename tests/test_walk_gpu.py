@@ -79,3 +79,34 @@ def test_column_work(where, stype, monkeypatch, gpu_lib):
     for k, (a, b) in enumerate(zip(*out)):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (k, np.max(np.abs(a - b)))
     assert np.any(out[0][3] != 0)
+
+
+# Column work in the tile with more than one warp of receivers in a column and
+# more than one source over it, near the surface and away from it; the per-cell
+# kernels' launches of their own are the reference.
+@pytest.mark.parametrize("fs", [0, 1])
+@pytest.mark.parametrize("variant", ["coordinate_rotation", "tensor_rotation", "bond_transformation"])
+def test_crowded_columns(variant, fs, monkeypatch, gpu_lib):
+    import ttifd
+
+    nz, nx, nt, eal = 90, 30, 60, 4
+    m = synthetic.layered_model(nz, nx, seed=9)
+    w = synthetic.ricker(nt, 0.0008, 30.0, delay=0.01)
+    gx = np.concatenate([np.full(70, 9), np.arange(nx)])
+    gz = np.concatenate([np.arange(70), np.full(nx, 1)])
+    out = []
+    for kernel in ("naive", "tiled"):
+        monkeypatch.setenv("TTIFD_EXACT", "1")
+        monkeypatch.setenv("TTIFD_KERNEL", kernel)
+        with ttifd.Modeling(variant=variant, nz=nz, nx=nx, nt=nt, dx=10.0, dz=10.0, dt=0.0008, fpeak=30.0,
+                            ealThick=eal, freesurface=fs, stype=1, seistype=3, mt=3) as h:
+            h.upload_model(*synthetic.padded(m, eal))
+            h.set_source([9, 12, 8, 20], [1, 0, 6, 50], np.stack([w, 0.5 * w, -w, 2 * w]))
+            for k in (0, 1, 2):
+                h.set_receivers(k, gx, gz)
+            h.run()
+            out.append([h.fetch_traces(k) for k in (0, 1, 2)]
+                       + [h.fetch_field(f) for f in range(8 if variant == "tensor_rotation" else 5)])
+    for k, (a, b) in enumerate(zip(*out)):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (k, np.max(np.abs(a - b)))
+    assert all(np.any(b != 0) for b in out[0])

@@ -107,10 +107,10 @@ void source_tables(const tti_handle *h, SourceTables *t)
 // A single shot's steps go out as replays of a graph of GRAPH_STEPS steps where
 // the grid is one wave of tiles (4 a SM on 148 SMs) or less: there the kernels
 // are shorter than the host's launches or little longer, and the gaps between
-// them show. us a step by replays / by launches: 60 x 80 8.05 / 9.2, 200 x 400
-// 10.8 / 12.0, 300 x 600 12.3 / 13.3, 400 x 800 (440 tiles) 13.7 / 14.4. Above,
-// a replay is hardly faster (600 x 1200, 960 tiles, 18.9 / 19.1) and the first
-// run, which captures, slower (19.7 / 19.4). The capture costs what replays
+// them show. us a step by replays / by launches: 60 x 80 6.4 / 6.8, 200 x 400
+// 9.2 / 10.8, 300 x 600 10.6 / 12.1, 400 x 800 (440 tiles) 12.1 / 13.1. Above,
+// a replay is hardly faster (600 x 1200, 960 tiles, 18.65 / 18.9) and the first
+// run, which captures, slower (19.4 / 19.1). The capture costs what replays
 // save over 60 to 250 steps, so runs of fewer steps do without.
 constexpr int GRAPH_TILES = 4 * 148, GRAPH_NT = 200;
 
@@ -179,7 +179,13 @@ int sync_columns(tti_handle *h)
     return nt > 0 && e.x1 > 0 && e.x0 >= NH && e.x1 <= g.Nx - NH && tile(e.z1 - 1) - tile(e.z0) < 2;
   };
   h->fold_src = w.stype >= 2 && fold(h->src_at);
-  h->fold_post = fold(post);
+  // after the stress update only rows that are updated or images of such
+  // (column_work keeps them on chip)
+  const int top = w.freesurface ? g.izStart - NH : g.izStart;
+  int z_base, rows;
+  tiled::tiles(g, g.izStart, &z_base, &rows);
+  const bool images = !w.freesurface || g.izStart + NH < std::min(g.Nz - NH, z_base + rows);
+  h->fold_post = fold(post) && post.z0 >= top && post.z1 <= g.Nz - NH && images;
   CK(h, cudaMemcpyAsync(h->d_cols, &w, sizeof w, cudaMemcpyHostToDevice, h->stream));
   CK(h, cudaStreamSynchronize(h->stream));  // w goes out of scope
   h->cols_dirty = false;

@@ -4,8 +4,9 @@
 // (coord:847-863), the stress source (stype 1, coord:865-886, tensor:871-895)
 // and the receiver samples (isoelastic.c:103-144). Columns do not interact, so
 // one warp does a column, in the reference's order: the single-shot tiled
-// kernels in the tiles it falls in, k_post and k_sources as launches of their
-// own (batched shots, and columns outside the tiles).
+// kernels in the tiles it falls in (after the stress update arranged as in
+// tiled_step.cu), k_post and k_sources as launches of their own (batched shots,
+// and columns outside the tiles).
 #pragma once
 
 #include "launch.cuh"

@@ -220,10 +220,10 @@ __device__ __forceinline__ void read_sums(const Cells &c, const float *sums, F4 
 // 19.2 / 20.2, 1126 x 7872 147.1 / 150.6.
 // The rows whose column work a tile does: its own, the first and the last tile
 // also those above and below all tiles.
-__device__ __forceinline__ bool tile_work(const HalfArgs &a, const Cells &c, int &r0, int &r1)
+__device__ __forceinline__ bool tile_work(const HalfArgs &a, int z0, int &r0, int &r1)
 {
-  r0 = c.z0 == a.z_base ? 0 : c.z0;
-  r1 = c.z0 + a.tile_rows >= a.g.Nz - NH ? a.g.Nz : c.z0 + a.tile_rows;
+  r0 = z0 == a.z_base ? 0 : z0;
+  r1 = z0 + a.tile_rows >= a.g.Nz - NH ? a.g.Nz : z0 + a.tile_rows;
   return r0 < a.work_z1 && r1 > a.work_z0;
 }
 
@@ -254,7 +254,7 @@ __device__ __forceinline__ void velocity_tile(const HalfArgs &a, const Cells &c,
     velocity_rows<V, X, Q, K>(a, c, gi, ds, p, k.nz, n);
   }
   int r0, r1;
-  if (tile_work(a, c, r0, r1)) {  // this warp's column
+  if (tile_work(a, c.z0, r0, r1)) {  // this warp's column
     __syncwarp();
     if (c.x < a.g.Nx - NH) column_sources(a.g, a.f, *a.cols, c.x, n, r0, r1);
   }
@@ -286,11 +286,11 @@ __device__ __forceinline__ void load_scells(const HalfArgs &a, bool und, const C
 }
 
 // The stress update of a thread's rows from their stencil sums d[f] = (d1, d2)
-// of vx, vz (coord:804-845, tensor:799-851, bond:836-873); what the gradient
-// keeps of them goes to kd and kt.
+// of vx, vz (coord:804-845, tensor:799-851, bond:836-873): n the new sigma, t
+// the new tau (tensor). What the gradient keeps of them goes to kd and kt.
 template <int V, bool X, bool Q, bool K>
 __device__ __forceinline__ void stress_rows(const HalfArgs &a, const Cells &c, size_t gi, const F4 (&d)[2][2],
-                                            const SCells &s, walk::u64 nz, int step)
+                                            const SCells &s, walk::u64 nz, int step, F4 (&n)[3], F4 (&t)[3])
 {
   typedef walk::Rows<X> A;
   typedef typename A::T T;
@@ -314,7 +314,6 @@ __device__ __forceinline__ void stress_rows(const HalfArgs &a, const Cells &c, s
 #pragma unroll
       for (int k = 0; k < 3; ++k) st4(a.kt[k] + ki, s.o[k], c.z, lo, hi);
   }
-  F4 n[3], t[3];
 #pragma unroll
   for (int i = 0; i < A::N; ++i) {
     T vxx = A::get(e[0], i), vxz = A::get(e[1], i), vzx = A::get(e[2], i), vzz = A::get(e[3], i);
@@ -358,24 +357,223 @@ __device__ __forceinline__ void stress_rows(const HalfArgs &a, const Cells &c, s
              r.add(r.mul(c1, o2), r.mul(c2, r.add(r.add(r.mul(c15, vxx), r.mul(c35, vzz)), r.mul(c55, sh)))));
     }
   }
-  st4(a.f.sxx + gi, n[0], c.z, lo, hi);
-  st4(a.f.szz + gi, n[1], c.z, lo, hi);
-  st4(a.f.sxz + gi, n[2], c.z, lo, hi);
-  if (V == TTI_TENSOR) {
-    st4(a.f.txx + gi, t[0], c.z, lo, hi);
-    st4(a.f.tzz + gi, t[1], c.z, lo, hi);
-    st4(a.f.txz + gi, t[2], c.z, lo, hi);
+}
+
+__device__ __forceinline__ void st_shared4(float *p, const F4 &f)
+{
+  *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(f.p[0], f.p[1]);
+}
+
+// The column work after the stress update in the tile, one warp (all lanes) a
+// column: column_post's work on rows [r0, r1), arranged so that what it reads
+// is there when it is needed. With every load after the update, as k_post does
+// it, each dependent load cost an L2 latency at the end of the kernel: 5000
+// cycles a stress launch at 60 x 80, of which 1600 for the source and 2000 for
+// the receivers. us a step with the loads there / as below: coordinate 60 x 80
+// 8.0 / 6.4, 200 x 400 10.8 / 9.2, 600 x 1200 19.0 / 18.9, 1126 x 3000 62.0 /
+// 61.2; tensor 1126 x 3000 71.5 / 69.5.
+//   plan_column     before the wait for the previous kernel: the geometry
+//   sample_column   while the tile's copies are in flight: the velocity
+//                   receivers, the first stress source's amplitudes
+//   column_work     after the update: the rest, in shared memory
+// The host folds the work in only where every row of it is updated or an image
+// row (sync_columns).
+struct ColumnPlan {
+  int rz[3] = {-1, -1, -1}, rid[3];  // first 32 receivers of a component, one per lane
+  int src = -1, sz = -1;             // first source whose window has the column; this lane's row in it
+  bool more = false;                 // there may be further sources, receivers
+  float ws = 0.0f;                   // what that source adds to the lane's row
+};
+// What is left of it after the update (held through the stencil walks, so few
+// registers: whole plans spilled there). Rows are the tile's, + 8.
+struct ColumnRest {
+  static constexpr int NO_ROW = 255;
+  int pr = NO_ROW, sr = NO_ROW;  // of the lane's pressure sample and of the first source
+  bool more = false;
+  float ws = 0.0f;
+  float *rec = nullptr;  // where the pressure sample goes
+};
+
+__device__ __forceinline__ void plan_column(const HalfArgs &a, int ix, int r0, int r1, ColumnPlan &c)
+{
+  const Columns &p = *a.cols;
+  const int lane = threadIdx.x & 31;
+  if (p.rec_on) {
+    int rb[3], re[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      rb[k] = re[k] = 0;
+      if (p.colptr[k]) {
+        rb[k] = p.colptr[k][ix];
+        re[k] = p.colptr[k][ix + 1];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (rb[k] + lane < re[k]) {
+        c.rz[k] = p.rz[k][rb[k] + lane];
+        c.rid[k] = p.rid[k][rb[k] + lane];
+        if (c.rz[k] < r0 || c.rz[k] >= r1) c.rz[k] = -1;
+      }
+      c.more |= re[k] - rb[k] > 32;
+    }
+  }
+  if (p.stype == 1)
+    for (int q = 0; q < p.src.n; ++q) {
+      const int dx = ix - p.src.x[q];
+      if (dx < -NH || dx > NH) continue;
+      if (c.src >= 0) {
+        c.more = true;
+        break;
+      }
+      c.src = q;
+      c.sz = p.src.z[q] + lane - NH;
+      if (lane > 2 * NH || c.sz < r0 || c.sz >= r1) c.sz = -1;
+      else c.ws = p.t.k1[(dx + NH) * 11 + lane];
+    }
+}
+
+__device__ __forceinline__ void put_sample(const Columns &p, float *rec, float v)
+{
+  *rec = v;
+  if (!isfinite(v)) atomicOr(p.flag, 1);
+}
+
+template <int V>
+__device__ __forceinline__ ColumnRest sample_column(const HalfArgs &a, int ix, int z0, const ColumnPlan &c)
+{
+  const Columns &p = *a.cols;
+  const size_t col = (size_t)ix * a.g.ldz;
+  const float vx = c.rz[0] >= 0 ? a.f.vx[col + c.rz[0]] : 0.0f, vz = c.rz[1] >= 0 ? a.f.vz[col + c.rz[1]] : 0.0f;
+  const int it = time_index(p, step_of(a)), irec = record_index(p, it);
+  ColumnRest w;
+  w.more = c.more;
+  if (c.src >= 0) w.ws = __fmul_rn(c.ws, p.src.w[(size_t)c.src * p.src.nt + it]);
+  if (c.sz >= 0) {
+    w.sr = c.sz - z0 + 8;
+    if (V == TTI_TENSOR && c.sz < max(z0, a.g.izStart)) {  // tau of the image rows changes nowhere else
+      a.f.txx[col + c.sz] = __fadd_rn(a.f.txx[col + c.sz], w.ws);
+      a.f.tzz[col + c.sz] = __fadd_rn(a.f.tzz[col + c.sz], w.ws);
+    }
+  }
+  if (irec < 0) return w;
+  if (c.rz[2] >= 0) {
+    w.pr = c.rz[2] - z0 + 8;
+    w.rec = p.rec[2] + (size_t)irec * p.nrec[2] + c.rid[2];
+  }
+  if (c.rz[0] >= 0) put_sample(p, p.rec[0] + (size_t)irec * p.nrec[0] + c.rid[0], vx);
+  if (c.rz[1] >= 0) put_sample(p, p.rec[1] + (size_t)irec * p.nrec[1] + c.rid[1], vz);
+  return w;
+}
+
+// Sources after the first of a column and receivers after 32 of a component;
+// S: row 0 of the column's sigma.
+template <typename F>
+__device__ __forceinline__ void more_work(const HalfArgs &a, int ix, int r0, int r1, F source, const float *S)
+{
+  const Columns &p = *a.cols;
+  const int lane = threadIdx.x & 31, it = time_index(p, step_of(a)), irec = record_index(p, it);
+  bool first = true;
+  for (int q = 0; q < (p.stype == 1 ? p.src.n : 0); ++q) {
+    const int dx = ix - p.src.x[q], iz = p.src.z[q] + lane - NH;
+    if (dx < -NH || dx > NH) continue;
+    if (!first && lane <= 2 * NH && iz >= r0 && iz < r1)
+      source(iz, __fmul_rn(p.t.k1[(dx + NH) * 11 + lane], p.src.w[(size_t)q * p.src.nt + it]), false);
+    first = false;
+    __syncwarp();
+  }
+  if (irec < 0) return;
+  for (int k = 0; k < 3; ++k) {
+    if (!p.colptr[k]) continue;
+    const int re = p.colptr[k][ix + 1];
+    for (int j = p.colptr[k][ix] + lane + (k < 2 ? 32 : 0); j < re; j += 32) {
+      const int rz = p.rz[k][j];
+      if (rz < r0 || rz >= r1) continue;
+      const size_t i = (size_t)ix * a.g.ldz + rz;
+      const float v = k == TTI_REC_VX   ? a.f.vx[i]
+                      : k == TTI_REC_VZ ? a.f.vz[i]
+                                        : __fmul_rn(0.5f, __fadd_rn(S[rz], S[walk::SUM + rz]));
+      put_sample(p, p.rec[k] + (size_t)irec * p.nrec[k] + p.rid[k][j], v);
+    }
+  }
+}
+
+// S: the column's sigma, rows -8 .. 127 of the tile, in place of its sums; tau
+// (tensor) in place of its inputs.
+template <int V>
+__device__ __forceinline__ void column_work(const HalfArgs &a, const Cells &c, size_t gi, const F4 (&n)[3],
+                                            const F4 (&t)[3], float *sm, const ColumnRest &w, int r0, int r1)
+{
+  const Grid &g = a.g;
+  const int lane = threadIdx.x & 31;
+  const int cx = c.x - c.x0, s = g.izStart - c.z0;
+  float *S = sm + walk::LEAD + cx * walk::DP + 8, *U = sm + S_IN + cx * a.tile_rows;
+  constexpr int F = walk::SUM;  // from one field of S to the next
+  const int M = WX * a.tile_rows;
+  const bool fs = a.freesurface && g.izStart >= r0 && g.izStart < r1;
+  __syncwarp();  // every lane has read the column's sums and inputs
+  if (c.on) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) st_shared4(S + k * F + 4 * lane, n[k]);
+    if (V == TTI_TENSOR)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) st_shared4(U + k * M + 4 * lane, t[k]);
+  }
+  __syncwarp();
+  if (fs) {  // coord:847-863
+    if (lane >= 1 && lane <= NH) {
+      S[s - lane] = __fsub_rn(__fmul_rn(2.0f, S[s]), S[s + lane]);
+      S[F + s - lane] = -S[F + s + lane];
+      S[2 * F + s - lane] = -S[2 * F + s + lane];
+    }
+    __syncwarp();
+    if (lane == 0) S[F + s] = S[2 * F + s] = 0.0f;
+    __syncwarp();
+  }
+  auto source = [&](int iz, float ws, bool first) {
+    const int r = iz - c.z0;
+    S[r] = __fadd_rn(S[r], ws);
+    S[F + r] = __fadd_rn(S[F + r], ws);
+    if (V == TTI_TENSOR) {
+      if (r >= 0 && iz >= g.izStart) {
+        U[r] = __fadd_rn(U[r], ws);
+        U[M + r] = __fadd_rn(U[M + r], ws);
+      } else if (!first) {  // (the first source's: sample_column)
+        const size_t i = (size_t)c.x * g.ldz + iz;
+        a.f.txx[i] = __fadd_rn(a.f.txx[i], ws);
+        a.f.tzz[i] = __fadd_rn(a.f.tzz[i], ws);
+      }
+    }
+  };
+  const int pr = w.pr, sr = w.sr;
+  if (sr != ColumnRest::NO_ROW) source(c.z0 + sr - 8, w.ws, true);
+  __syncwarp();
+  if (w.more) more_work(a, c.x, r0, r1, source, S - c.z0);
+  else if (pr != ColumnRest::NO_ROW) put_sample(*a.cols, w.rec, __fmul_rn(0.5f, __fadd_rn(S[pr - 8], S[F + pr - 8])));
+  const int lo = fs ? g.izStart - NH : g.izStart, hi = min(g.Nz - NH, c.z0 + a.tile_rows);
+  float *const f[3] = {a.f.sxx, a.f.szz, a.f.sxz};
+  if (c.z + 3 >= lo && 4 * lane < a.tile_rows && c.z < hi)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) st4(f[k] + gi, ld4(S + k * F + 4 * lane), c.z, lo, hi);
+  const int above = c.z0 - 1 - lane;  // image rows above the tile
+  if (fs && lane < 8 && above >= lo)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) f[k][(size_t)c.x * g.ldz + above] = S[k * F - 1 - lane];
+  if (V == TTI_TENSOR && c.on) {
+    st4(a.f.txx + gi, ld4(U + 4 * lane), c.z, g.izStart, hi);
+    st4(a.f.tzz + gi, ld4(U + M + 4 * lane), c.z, g.izStart, hi);
+    st4(a.f.txz + gi, t[2], c.z, g.izStart, hi);
   }
 }
 
 // Stress update of a tile whose boxes (vx, vz) and inputs have arrived
 template <int V, bool X, bool Q, bool K>
 __device__ __forceinline__ void stress_tile(const HalfArgs &a, const Cells &c, bool und, const walk::Coefs &k,
-                                            float *sm, int n)
+                                            float *sm, int step, const ColumnRest *rest, bool work, int r0, int r1)
 {
-  const int gr = walk::groups(a.tile_rows), t = threadIdx.x >> 5, f = t >= gr;
-  const int d = (t - f * gr) * 32 + (threadIdx.x & 31);
-  const bool on = t < 2 * gr && d < a.tile_rows + WX - 1;  // one walk per warp: 2 gr <= 8
+  const int gr = walk::groups(a.tile_rows), w = threadIdx.x >> 5, f = w >= gr;
+  const int d = (w - f * gr) * 32 + (threadIdx.x & 31);
+  const bool on = w < 2 * gr && d < a.tile_rows + WX - 1;  // one walk per warp: 2 gr <= 8
   walk::u64 out[WX];
   if (on) {
     const float *box = sm + walk::LEAD + f * walk::BOX;
@@ -385,18 +583,27 @@ __device__ __forceinline__ void stress_tile(const HalfArgs &a, const Cells &c, b
   float *sums = sm + walk::LEAD;
   if (on) walk::put_sums(sums + 2 * f * walk::SUM, sums + (2 * f + 1) * walk::SUM, d, out);
   __syncthreads();  // the sums are complete
+  const size_t gi = (size_t)c.x * a.g.ldz + c.z;
+  F4 n[3], t[3];
   if (c.on) {
-    const size_t gi = (size_t)c.x * a.g.ldz + c.z;
     F4 ds[2][2];
     read_sums(c, sums, ds);
     SCells p;
     load_scells<V>(a, und, c, gi, sm, p);
-    stress_rows<V, X, Q, K>(a, c, gi, ds, p, k.nz, n);
+    stress_rows<V, X, Q, K>(a, c, gi, ds, p, k.nz, step, n, t);
   }
-  int r0, r1;
-  if (tile_work(a, c, r0, r1)) {  // this warp's column
-    __syncwarp();
-    if (c.x < a.g.Nx - NH) column_post(a.g, a.f, *a.cols, c.x, n, r0, r1);
+  if (work) {
+    if (c.x < a.g.Nx - NH) column_work<V>(a, c, gi, n, t, sm, *rest, r0, r1);  // this warp's column
+  } else if (c.on) {
+    const int lo = a.g.izStart, hi = min(a.g.Nz - NH, c.z0 + a.tile_rows);
+    st4(a.f.sxx + gi, n[0], c.z, lo, hi);
+    st4(a.f.szz + gi, n[1], c.z, lo, hi);
+    st4(a.f.sxz + gi, n[2], c.z, lo, hi);
+    if (V == TTI_TENSOR) {
+      st4(a.f.txx + gi, t[0], c.z, lo, hi);
+      st4(a.f.tzz + gi, t[1], c.z, lo, hi);
+      st4(a.f.txz + gi, t[2], c.z, lo, hi);
+    }
   }
 }
 
@@ -432,14 +639,21 @@ __global__ void __launch_bounds__(walk::NT, K ? 3 : 4) k_stress_tiled(const __gr
   const int z0 = a.z_base + (gridDim.x - 1 - blockIdx.x) * a.tile_rows;
   const int x0 = a.x_base + (gridDim.y - 1 - blockIdx.y) * WX;
   walk::init_bar(bar);
+  const int ix = x0 + (threadIdx.x >> 5);  // this warp's column
+  int r0, r1;
+  const bool work = tile_work(a, z0, r0, r1);
+  ColumnPlan plan;
+  if (work && ix < a.g.Nx - NH) plan_column(a, ix, r0, r1, plan);
   pdl_sync();
   walk::issue_tile(m.box, 2, 5, m.in, s_inputs(V), a.tile_rows, sm, S_IN, bar, z0, x0);
   const bool und = tile_undamped(a, z0, x0, WX);
   prefetch_stress(a, und, z0, x0);
   const int n = step_of(a);
+  ColumnRest rest;
+  if (work && ix < a.g.Nx - NH) rest = sample_column<V>(a, ix, z0, plan);
   const walk::Coefs k = coefs<Q>(a, a.nzero);
   if (!walk::wait_boxes(a.err, bar, a.wait_limit, 0)) return;
-  stress_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, n);
+  stress_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, n, &rest, work, r0, r1);
 }
 
 // Batched launches copy the instance's arguments into shared memory: the fields
@@ -528,7 +742,7 @@ __global__ void __launch_bounds__(walk::NT, 4) k_stress_batch(const __grid_const
         prefetch_stress(a, und, z0, x0);
       },
       [&](const HalfArgs &a, const Cells &c, bool und, int n) {
-        stress_tile<V, X, Q, false>(a, c, und, coefs<Q>(a, b.nzero), sm, n);
+        stress_tile<V, X, Q, false>(a, c, und, coefs<Q>(a, b.nzero), sm, n, nullptr, false, 0, 0);
       });
 }
 
