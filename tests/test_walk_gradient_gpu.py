@@ -53,3 +53,38 @@ def test_tile_edges(variant, nz, nx, eal, fs, edge, monkeypatch, gpu_lib):
         assert np.any(b != 0), k
         rel = np.linalg.norm(a.astype(np.float64) - b) / np.linalg.norm(b.astype(np.float64))
         assert rel <= 2e-5, (k, rel)
+
+
+# Column work in the tiles with more than one warp of receivers in a column and
+# more than one source over it; receivers of every component share cells.
+@pytest.mark.parametrize("fs", [0, 1])
+@pytest.mark.parametrize("variant", ["coordinate_rotation", "tensor_rotation", "bond_transformation"])
+def test_crowded_columns(variant, fs, monkeypatch, gpu_lib):
+    import ttifd
+
+    nz, nx, nt, eal = 90, 30, 50, 4
+    m = synthetic.layered_model(nz, nx, seed=9)
+    w = synthetic.ricker(nt, 0.0008, 30.0, delay=0.01)
+    gx = np.concatenate([np.full(70, 9), np.arange(nx), np.arange(nx)])
+    gz = np.concatenate([np.arange(70), np.full(nx, 1), np.full(nx, 1)])
+    out = []
+    for kernel in ("naive", "tiled"):
+        monkeypatch.setenv("TTIFD_KERNEL", kernel)
+        rng = np.random.default_rng(7)
+        with ttifd.Modeling(variant=variant, nz=nz, nx=nx, nt=nt, dx=10.0, dz=9.0, dt=0.0008, fpeak=30.0,
+                            ealThick=eal, freesurface=fs, stype=1, seistype=3) as h:
+            h.upload_model(*synthetic.padded(m, eal))
+            h.set_source([9, 12, 8, 20], [1, 0, 6, 50], np.stack([w, 0.5 * w, -w, 2 * w]))
+            for k, amp in ((0, 5e-12), (1, 5e-12), (2, 4e-5)):
+                h.set_receivers(k, gx, gz)
+                t = np.cumsum(rng.standard_normal((len(gx), h.nts)), axis=1)
+                h.grad_set_observed(k, (amp * t / 5).astype(np.float32))
+            h.grad_zero()
+            j = h.grad_run(2)
+            out.append((j, [h.grad_fetch(g) for g in ("vp", "eps", "delta", "theta")] + [h.grad_fetch_source(4)]))
+    (jr, ref), (jt, got) = out
+    assert abs(jt - jr) <= 1e-12 * jr
+    for k, (a, b) in enumerate(zip(got, ref)):
+        assert np.any(b != 0), k
+        rel = np.linalg.norm(a.astype(np.float64) - b) / np.linalg.norm(b.astype(np.float64))
+        assert rel <= 2e-5, (k, rel)

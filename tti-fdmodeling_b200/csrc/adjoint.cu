@@ -64,7 +64,7 @@ struct GradState {
   double *vrim_acc = nullptr;
   int vm = 0, vrim_n = 0;
   bool surf_merged = false;  // the column work runs inside the stress-half adjoint (else a separate launch)
-  int surf_zend = 0;         // rows at or below this hold no column work
+  int surf_z0 = 0, surf_z1 = 0;  // the rows with column work
 };
 
 namespace {
@@ -484,15 +484,19 @@ __global__ void __launch_bounds__(BZ *BX) k_adj_velocity_stencil(AdjArgs a)
 // and without a rotation at the velocity node (tensor, Bond) A = Fx, C = Fz,
 // B = D = 0: two boxes.
 //
-// Both are bound by memory latency and throughput: the first moves 128 bytes a
-// cell (coordinate), the second 92, 5 TB/s through L2 at 600 x 1200. What they
-// read per cell is requested before anything is waited for: halo boxes, kept
-// fields and moduli by TMA, lambda and the gradient sums into registers, which
-// sets the CTAs per SM (two of 128 registers; three of 80 spill and take 71
-// against 69 us a step at 600 x 1200, 352 against 272 in the tensor rotation at
-// 1126 x 3000). Loading them after the walks from lines prefetched into L2 took
-// 83 and 305. One reverse step: 600 x 1200 about 46 us (three kernels with a
-// cell per thread and the six terms: 63), 1126 x 3000 160 (237).
+// Both are bound by memory throughput: the first moves 128 bytes a cell
+// (coordinate), the second 92; at 1126 x 3000 they run at 85 percent of the
+// copy rate, at 600 x 1200 (in part out of L2) one wave and a half of tiles
+// leave a tail. What they read per cell is requested before anything is waited
+// for: halo boxes, kept fields and moduli by TMA, lambda and the gradient sums
+// into registers, which sets the CTAs per SM (two of 128 registers; three of 80
+// spill and take 71 against 69 us a step at 600 x 1200, 352 against 272 in the
+// tensor rotation at 1126 x 3000). Loads in flight need lines of L1, so these
+// kernels leave it what their shared memory does not use (launch_adj). Loading
+// after the walks from lines prefetched into L2 took 83 and 305; everything by
+// TMA is 1 to 2 us a step slower. One reverse step: 600 x 1200 42 us (three
+// kernels with a cell per thread and the six terms: 63), 1126 x 3000 140 (237),
+// tensor 37 and 123, Bond 32 and 115.
 using walk::F4;
 using walk::ld4;
 using walk::ldg4;
@@ -507,7 +511,7 @@ struct alignas(64) AdjTile {
   int kept0;           // this step's first field in `kept`
   int z_base, rows;    // first tile row (multiple of 8), rows of a tile
   int undamped_ok, und_z0;  // coef1 == 1, coef2 == dt on [E, Nx - E) x [und_z0, Nz - E) (checked at upload)
-  int surf_zend;       // rows at or below this hold no column work
+  int surf_z0, surf_z1;  // the rows with column work
   float nzero;         // -0.0f
   int *err;            // bit 4: a TMA wait timed out
 };
@@ -732,12 +736,151 @@ __device__ __forceinline__ void stress_local(const AdjTile &at, const TileCells 
     if (!(V == TTI_COORDINATE && k == 3)) st4(a.acc[k] + i, n.acc[k], c.z, lo, hi);
 }
 
+// The column work in the stress tiles: surface_warp's, arranged so that what it
+// reads is there when it is needed. With every access in global memory, each
+// load waiting for the one before, a tile with column work took 32000 cycles
+// against 10500 (600 x 1200, where one tile in six has some: 31 us a launch).
+//   plan_columns    before the wait for the previous kernel: the geometry
+//   inject_columns  while the tile's copies are in flight: residuals, lambda_v
+//   work_columns    after the stencils: the rest, in shared memory
+struct ColumnPlan {
+  int rz[3] = {-1, -1, -1}, rid[3];  // first 32 receivers of a component, one per lane: row of the tile, trace
+  int src = -1, sr = -1;             // first source whose window has the column; this lane's row in it
+  float w = 0.0f;                    // and its weight there
+  bool more = false;                 // there may be further sources, receivers
+};
+__device__ __forceinline__ void plan_columns(const SurfaceArgs &a, const TileCells &c, int r1, ColumnPlan &p)
+{
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (!a.res[k]) continue;
+    const int rb = a.colptr[k][c.x], re = a.colptr[k][c.x + 1];
+    if (rb + lane < re) {
+      const int rz = a.rzs[k][rb + lane];
+      p.rid[k] = a.rid[k][rb + lane];
+      if (rz >= c.z0 && rz < r1) p.rz[k] = rz - c.z0;
+    }
+    p.more |= re - rb > 32;
+  }
+  for (int n = 0; n < a.src.n; ++n) {
+    const int dx = c.x - a.src.x[n];
+    if (dx < -NH || dx > NH) continue;
+    if (p.src >= 0) {
+      p.more = true;
+      break;
+    }
+    p.src = n;
+    const int iz = a.src.z[n] + lane - NH;
+    if (lane <= 2 * NH && iz >= c.z0 && iz < r1) {
+      p.sr = iz - c.z0;
+      p.w = a.k1.k1[(dx + NH) * 11 + lane];
+    }
+  }
+}
+// lambda_v += residuals (atomically: receivers may share a cell); returns the
+// lane's pressure residual
+__device__ __forceinline__ float inject_columns(const AdjTile &at, const SurfaceArgs &a, const TileCells &c,
+                                                const ColumnPlan &p)
+{
+  const size_t i = (size_t)c.x * at.a.g.ldz + c.z0;
+  float res[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) res[k] = p.rz[k] >= 0 ? a.res[k][p.rid[k]] : 0.0f;
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    if (p.rz[k] >= 0) atomicAdd(a.lam[k] + i + p.rz[k], res[k]);
+  return 0.5f * res[2];
+}
+// Lambda_sigma of the warp's column in S (arrays of SUM floats, row 0 the
+// tile's), which takes the place of its sums.
+template <int V>
+__device__ __forceinline__ void work_columns(const AdjTile &at, const SurfaceArgs &a, const TileCells &c, int r1,
+                                             F4 (&l)[3], float *sm, int pr, float pv, int src, int sr,
+                                             float w, bool more)
+{
+  const Grid &g = at.a.g;
+  const int lane = threadIdx.x & 31;
+  constexpr int F = walk::SUM;
+  float *S = sm + walk::LEAD + (c.x - c.x0) * walk::DP;
+  __syncwarp();  // every lane has read the column's sums
+  if (c.on)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) *reinterpret_cast<ulonglong2 *>(S + q * F + 4 * lane) = make_ulonglong2(l[q].p[0], l[q].p[1]);
+  __syncwarp();
+  if (pr >= 0) {
+    atomicAdd(S + pr, pv);
+    atomicAdd(S + F + pr, pv);
+  }
+  if (more)
+    for (int k = 0; k < 3; ++k) {
+      if (!a.res[k]) continue;
+      for (int j = a.colptr[k][c.x] + 32 + lane; j < a.colptr[k][c.x + 1]; j += 32) {
+        const int rz = a.rzs[k][j];
+        if (rz < c.z0 || rz >= r1) continue;
+        const float r = a.res[k][a.rid[k][j]];
+        if (k < 2) atomicAdd(a.lam[k] + (size_t)c.x * g.ldz + rz, r);
+        else {
+          atomicAdd(S + rz - c.z0, 0.5f * r);
+          atomicAdd(S + F + rz - c.z0, 0.5f * r);
+        }
+      }
+    }
+  __syncwarp();
+  auto source = [&](int n, int row, float wt) {
+    float v = 0.0f;
+    if (row >= 0) {
+      float s = S[row] + S[F + row];
+      if (V == TTI_TENSOR)  // the source also adds to tau
+        s += a.lam[5][(size_t)c.x * g.ldz + c.z0 + row] + a.lam[6][(size_t)c.x * g.ldz + c.z0 + row];
+      v = wt * s;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0 && v != 0.0f) atomicAdd(a.gsrc + (size_t)n * a.src.nt + a.it, v);
+  };
+  if (src >= 0) source(src, sr, w);
+  if (more && src >= 0)
+    for (int n = src + 1; n < a.src.n; ++n) {
+      const int dx = c.x - a.src.x[n], iz = a.src.z[n] + lane - NH;
+      if (dx < -NH || dx > NH) continue;
+      const bool in = lane <= 2 * NH && iz >= c.z0 && iz < r1;
+      source(n, in ? iz - c.z0 : -1, in ? a.k1.k1[(dx + NH) * 11 + lane] : 0.0f);
+    }
+  __syncwarp();
+  const int s = g.izStart - c.z0;
+  if (a.fs && s - NH >= 0 && g.izStart + NH < r1) {  // (as in surface_warp)
+    float img = 0.0f;
+    if (lane >= 1 && lane <= NH) {
+      img = S[s - lane];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        S[q * F + s + lane] -= S[q * F + s - lane];
+        S[q * F + s - lane] = 0.0f;
+      }
+    }
+    float add[NH];
+#pragma unroll
+    for (int k = 1; k <= NH; ++k) add[k - 1] = __shfl_sync(0xffffffffu, img, k);
+    if (lane == 0) {
+      float t = S[s];
+#pragma unroll
+      for (int k = 0; k < NH; ++k) t += 2.0f * add[k];
+      S[s] = t;
+      S[F + s] = 0.0f;
+      S[2 * F + s] = 0.0f;
+    }
+  }
+  __syncwarp();
+  if (c.on)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) l[q] = ld4(S + q * F + 4 * lane);
+}
+
 // MODE 0: stencils, column work, local part. Where the column work reaches
 // cells outside the tiles, three launches instead: MODE 1 (stencils only),
-// k_adj_surface, MODE 2 (local part only).
-// One warp holds one column of the tile, so a tile with column work (rows
-// above surf_zend) stores lambda_sigma, does its columns' work warp by warp on
-// global memory, and reads it back.
+// k_adj_surface, MODE 2 (local part only). One warp holds one column of the
+// tile.
 template <int V, int MODE>
 __global__ void __launch_bounds__(walk::NT, 2) k_adj_stress(const __grid_constant__ AdjTile at,
                                                             const __grid_constant__ SurfaceArgs sa)
@@ -749,13 +892,15 @@ __global__ void __launch_bounds__(walk::NT, 2) k_adj_stress(const __grid_constan
   const AdjArgs &a = at.a;
   const Grid &g = a.g;
   const TileCells c = tile_cells(at, a.z_lo);
+  const int hi = min(g.Nz - NH, c.z0 + at.rows);
+  const bool surf = MODE == 0 && c.z0 < at.surf_z1 && c.z0 + at.rows > at.surf_z0, columns = surf && c.x < g.Nx - NH;
   walk::init_bar(bar);
+  ColumnPlan plan;
+  if (columns) plan_columns(sa, c, hi, plan);
   pdl_sync();
   issue_adj(at, sm, bar, NB, 5, 0, NK, NP, c);
   const walk::Coefs k = walk::coefs(rsg(0), rsg(1), rsg(2), rsg(3), rsg(4), at.nzero);
   const size_t i = (size_t)c.x * g.ldz + c.z;
-  const int hi = min(g.Nz - NH, c.z0 + at.rows);
-  const bool surf = MODE == 0 && c.z0 < at.surf_zend;
   const bool local = MODE != 1 && c.on && c.z + 3 >= g.izStart;
   // this thread's inputs, requested while the copies are in flight
   F4 l[3];
@@ -771,6 +916,7 @@ __global__ void __launch_bounds__(walk::NT, 2) k_adj_stress(const __grid_constan
       for (int q = 0; q < 3; ++q) l[q] = ld4(a.lam[2 + q] + i);
   }
   if (local) load_local<V>(at, adj_undamped(at, c), i, n);
+  const float pv = columns ? inject_columns(at, sa, c, plan) : 0.0f;
   if (!walk::wait_boxes(at.err, bar, tiled::tma::WAIT_LIMIT, 0)) return;
   if (MODE != 2) adj_walks<1, NB, false>(at, k, sm);
   if (c.on) {
@@ -798,22 +944,16 @@ __global__ void __launch_bounds__(walk::NT, 2) k_adj_stress(const __grid_constan
         R::set(l[2], q, at4(l[2], q) - dxz);
       }
     }
-    if (MODE == 1 || surf)
+    if (MODE == 1)
 #pragma unroll
       for (int q = 0; q < 3; ++q) st4(a.lam[2 + q] + i, l[q], c.z, a.z_lo, hi);
   }
   if (MODE == 1) return;
-  if (surf) {
-    __syncwarp();
-    if (c.x < g.Nx - NH) surface_warp(sa, c.x, c.z0, c.z0 + at.rows, threadIdx.x & 31);
-    __syncwarp();
-    if (c.on)
+  if (columns)
+    work_columns<V>(at, sa, c, hi, l, sm, plan.rz[2], pv, plan.src, plan.sr, plan.w, plan.more);
+  if (surf && c.on)  // image rows
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const float4 v = __ldcg(reinterpret_cast<const float4 *>(a.lam[2 + q] + i));
-        l[q] = F4{{walk::pack2(v.x, v.y), walk::pack2(v.z, v.w)}};
-      }
-  }
+    for (int q = 0; q < 3; ++q) st4(a.lam[2 + q] + i, l[q], c.z, a.z_lo, min(hi, g.izStart));
   if (local) stress_local<V>(at, c, i, l, n, sm + kept_off(NB), MODE == 2 || surf);
 }
 
@@ -909,7 +1049,10 @@ cudaError_t launch_adj(K kernel, AdjTile &at, int boxes, int kept, int z_first, 
     if (std::find(done.begin(), done.end(), key) == done.end()) {
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
       if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        // 164 of 228 KB: two stress or three velocity CTAs; the other 92 KB are
+        // L1. With L1 at its smallest a reverse step takes 44.6 against 41.7 us
+        // at 600 x 1200, 150 against 140 at 1126 x 3000.
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 72);
       if (e != cudaSuccess) return e;
       done.push_back(key);
     }
@@ -1222,9 +1365,9 @@ int vsource_tables(tti_handle *h, const SourceTables &tab)
 
 // Whether the column work can run inside the stress-half adjoint: every
 // receiver, stress-source window and image row must lie in the tiles (columns
-// [NH, Nx - NH), rows from the first tile's to Nz - NH), the image rows and
-// their mirrors in the first; *z_end: the first row below all of them.
-int surface_extent(tti_handle *h, bool *merged, int *z_end)
+// [NH, Nx - NH), rows from z_lo to Nz - NH), the image rows and their mirrors in
+// the first; [*z_begin, *z_end): the rows with such work.
+int surface_extent(tti_handle *h, bool *merged, int *z_begin, int *z_end)
 {
   const Grid &g = h->g;
   const tti_config &c = h->cfg;
@@ -1262,8 +1405,9 @@ int surface_extent(tti_handle *h, bool *merged, int *z_end)
       x1 = std::max(x1, std::min(g.Nx, v[h->nsrc + n] + NH + 1));
     }
   }
+  *z_begin = z;
   *z_end = e;
-  *merged = z >= z_base && e <= g.Nz - NH && (x1 == 0 || (x0 >= NH && x1 <= g.Nx - NH)) &&
+  *merged = z >= adj_z_lo(h) && e <= g.Nz - NH && (x1 == 0 || (x0 >= NH && x1 <= g.Nx - NH)) &&
             (!fs || g.izStart + NH + 1 <= z_base + tile_rows);
   return TTI_OK;
 }
@@ -1313,7 +1457,8 @@ int adjoint_tiles(tti_handle *h, const AdjArgs &a, const SurfaceArgs &sa, bool w
   constexpr int NB = stress_boxes(V), NK = stress_kept(V);
   const int z0 = a.z_lo;  // the first tile row, the same for every kernel (the kept fields' boxes have one height)
   if (!work || s->surf_merged) {
-    at.surf_zend = work ? s->surf_zend : 0;
+    at.surf_z0 = work ? s->surf_z0 : 0;
+    at.surf_z1 = work ? s->surf_z1 : 0;
     GCK(h, launch_adj(k_adj_stress<V, 0>, at, NB, NK + stress_par(V), z0, h->stream, sa));
   } else {
     GCK(h, launch_adj(k_adj_stress<V, 1>, at, NB, 0, z0, h->stream, sa));
@@ -1508,7 +1653,7 @@ int grad_prepare(tti_handle *h, int slots, int seg, SourceTables *tab)
   if ((rc = handle_columns(h))) return rc;
   handle_source_tables(h, tab);
   if ((rc = vsource_tables(h, *tab))) return rc;
-  return surface_extent(h, &s->surf_merged, &s->surf_zend);
+  return surface_extent(h, &s->surf_merged, &s->surf_z0, &s->surf_z1);
 }
 
 // Residuals d - dobs of every recorded component and J (read back into *J at
