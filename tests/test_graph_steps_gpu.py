@@ -72,3 +72,31 @@ def test_replays(variant, how, monkeypatch, gpu_lib):
     assert len(got) == len(ref) and any(np.any(b != 0) for b in ref)
     for k, (a, b) in enumerate(zip(got, ref)):
         assert np.array_equal(np.asarray(a).view(np.uint32), np.asarray(b).view(np.uint32)), k
+
+
+# Either side of the largest grid whose launches trigger the next one at their
+# start and go out as replays (296 tiles of 8 columns), against the per-cell
+# kernels.
+@pytest.mark.parametrize("tiles", [296, 297])
+@pytest.mark.parametrize("variant", ["coordinate_rotation", "tensor_rotation"])
+def test_two_launches_on_the_device(variant, tiles, monkeypatch, gpu_lib):
+    import ttifd
+
+    nz, eal, nt = 12, 2, 215
+    nx = 8 * tiles - 2 * eal
+    m = synthetic.layered_model(nz, nx, seed=4)
+    out = []
+    for kernel in ("tiled", "naive"):
+        monkeypatch.setenv("TTIFD_KERNEL", kernel)
+        with ttifd.Modeling(variant=variant, nz=nz, nx=nx, nt=nt, dx=10.0, dz=10.0, dt=0.0008, fpeak=30.0,
+                            ealThick=eal, freesurface=1, stype=1, seistype=3) as h:
+            h.upload_model(*synthetic.padded(m, eal))
+            w = synthetic.ricker(nt, 0.0008, 30.0, delay=0.01)
+            h.set_source([nx // 2, 7], [3, 5], np.stack([w, w]))
+            for k in (0, 1, 2):
+                h.set_receivers(k, np.arange(nx), 2)
+            h.run()
+            out.append([h.fetch_traces(k) for k in (0, 1, 2)] + [h.fetch_field(f) for f in range(5)])
+    for k, (a, b) in enumerate(zip(*out)):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (k, np.max(np.abs(a - b)))
+        assert np.any(b != 0), k

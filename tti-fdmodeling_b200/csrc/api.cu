@@ -105,14 +105,14 @@ void source_tables(const tti_handle *h, SourceTables *t)
 }
 
 // A single shot's steps go out as replays of a graph of GRAPH_STEPS steps where
-// the grid is one wave of tiles (4 a SM on 148 SMs) or less: there the kernels
-// are shorter than the host's launches or little longer, and the gaps between
-// them show. us a step by replays / by launches: 60 x 80 6.4 / 6.8, 200 x 400
-// 9.2 / 10.8, 300 x 600 10.6 / 12.1, 400 x 800 (440 tiles) 12.1 / 13.1. Above,
-// a replay is hardly faster (600 x 1200, 960 tiles, 18.65 / 18.9) and the first
-// run, which captures, slower (19.4 / 19.1). The capture costs what replays
-// save over 60 to 250 steps, so runs of fewer steps do without.
-constexpr int GRAPH_TILES = 4 * 148, GRAPH_NT = 200;
+// the CTAs of two launches fit the device together (early_trigger): there the
+// kernels are hardly longer than the host's launches, and the gaps between them
+// show. us a step by replays / by launches: 60 x 80 6.25 / 6.7, 200 x 400 7.6 /
+// 7.95, 300 x 600 (255 tiles) 8.2 / 8.3, the first run, which captures, 8.6 /
+// 10.5. Above, a replay is not faster (400 x 800, 440 tiles, 12.0 / 11.65; 600 x
+// 1200 18.5 / 18.5). The capture costs what replays save over 60 to 250 steps,
+// so runs of fewer steps do without.
+constexpr int GRAPH_TILES = 2 * 148, GRAPH_NT = 200;
 
 int check_cfg(const tti_config *c)
 {

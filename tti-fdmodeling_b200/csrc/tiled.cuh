@@ -38,6 +38,7 @@ struct alignas(16) HalfArgs {
   unsigned wait_limit;  // polls of the first TMA wait before it gives up (tma::WAIT_LIMIT)
   float hc[5]; // h * C_k
   float nzero; // -0.0f (see walk::coefs)
+  int early;   // trigger the next kernel at the start (early_trigger)
   // Gradient forward pass (null: nothing kept). Velocity update, coordinate
   // rotation: per cell the stress derivative combinations the adjoint's
   // theta_v terms need (sxz_x - sxx_z, szz_x - sxz_z, sxx_x + sxz_z,
@@ -79,6 +80,15 @@ inline void set_square(HalfArgs &a, bool exact)
 
 // Encodes a handle's MAPS tensor maps.
 bool encode_maps(CUtensorMap *map, const Grid &g, int variant, const Fields &f, const Params &p);
+// Whether a half-step launch of so many tiles triggers its dependent as soon as
+// it has waited for its own predecessor: only where the CTAs of two launches
+// fit the device together (4 a SM on 148 SMs). The next launch's CTAs then wait
+// in free slots. Where they do not fit, the part that finds a slot is spread
+// unevenly, so the trigger comes when a tile's sums are complete. us a step
+// early / late: 60 x 80 6.0 / 6.6, 300 x 600 (255 tiles) 7.95 / 9.1; 400 x 800
+// (440 tiles) 12.0 / 11.4, 500 x 1000 15.1 / 14.4, 600 x 1200 18.4 / 17.9,
+// 1126 x 3000 61.0 / 60.4.
+inline int early_trigger(long long tiles) { return 2 * tiles <= 4 * 148; }
 // The arguments of h's half-steps (a: handle_step_args), without column work.
 void fill_args(HalfArgs &ha, const tti_handle *h, const StepArgs &a);
 void velocity_maps(VelocityMaps &m, const void *maps);  // from a handle's maps

@@ -231,7 +231,7 @@ __device__ __forceinline__ bool tile_work(const HalfArgs &a, int z0, int &r0, in
 // per field and 32 diagonals, then one per column.
 template <int V, bool X, bool Q, bool K>
 __device__ __forceinline__ void velocity_tile(const HalfArgs &a, const Cells &c, bool und, const walk::Coefs &k,
-                                              float *sm, int n)
+                                              float *sm, int n, bool early)
 {
   const int gr = walk::groups(a.tile_rows);
   float *sums = sm + V_SUMS;
@@ -248,6 +248,7 @@ __device__ __forceinline__ void velocity_tile(const HalfArgs &a, const Cells &c,
   VCells p;
   if (c.on) load_vcells<V>(a, und, gi, p);
   __syncthreads();  // the sums are complete
+  if (!early) pdl_trigger();
   if (c.on) {
     F4 ds[3][2];
     read_sums(c, sums, ds);
@@ -569,7 +570,8 @@ __device__ __forceinline__ void column_work(const HalfArgs &a, const Cells &c, s
 // Stress update of a tile whose boxes (vx, vz) and inputs have arrived
 template <int V, bool X, bool Q, bool K>
 __device__ __forceinline__ void stress_tile(const HalfArgs &a, const Cells &c, bool und, const walk::Coefs &k,
-                                            float *sm, int step, const ColumnRest *rest, bool work, int r0, int r1)
+                                            float *sm, int step, bool early, const ColumnRest *rest, bool work, int r0,
+                                            int r1)
 {
   const int gr = walk::groups(a.tile_rows), w = threadIdx.x >> 5, f = w >= gr;
   const int d = (w - f * gr) * 32 + (threadIdx.x & 31);
@@ -583,6 +585,7 @@ __device__ __forceinline__ void stress_tile(const HalfArgs &a, const Cells &c, b
   float *sums = sm + walk::LEAD;
   if (on) walk::put_sums(sums + 2 * f * walk::SUM, sums + (2 * f + 1) * walk::SUM, d, out);
   __syncthreads();  // the sums are complete
+  if (!early) pdl_trigger();
   const size_t gi = (size_t)c.x * a.g.ldz + c.z;
   F4 n[3], t[3];
   if (c.on) {
@@ -616,14 +619,15 @@ __global__ void __launch_bounds__(walk::NT, 4) k_velocity_tiled(const __grid_con
   unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + V_BAR);
   const int z0 = a.z_base + blockIdx.x * a.tile_rows, x0 = a.x_base + blockIdx.y * WX;
   walk::init_bar(bar);
-  pdl_sync();
+  pdl_wait();
+  if (a.early) pdl_trigger();
   walk::issue_tile(m.box, 3, 4, nullptr, 0, 0, sm, 0, bar, z0, x0);
   const bool und = tile_undamped(a, z0, x0, WX);
   prefetch_velocity(a, und, z0, x0);
   const int n = step_of(a);
   const walk::Coefs k = coefs<Q>(a, a.nzero);
   if (!walk::wait_boxes(a.err, bar, a.wait_limit, 0)) return;
-  velocity_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, n);
+  velocity_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, n, a.early);
 }
 
 // The stress update walks the tiles in the opposite order, so that it starts
@@ -644,7 +648,8 @@ __global__ void __launch_bounds__(walk::NT, K ? 3 : 4) k_stress_tiled(const __gr
   const bool work = tile_work(a, z0, r0, r1);
   ColumnPlan plan;
   if (work && ix < a.g.Nx - NH) plan_column(a, ix, r0, r1, plan);
-  pdl_sync();
+  pdl_wait();
+  if (a.early) pdl_trigger();
   walk::issue_tile(m.box, 2, 5, m.in, s_inputs(V), a.tile_rows, sm, S_IN, bar, z0, x0);
   const bool und = tile_undamped(a, z0, x0, WX);
   prefetch_stress(a, und, z0, x0);
@@ -653,7 +658,7 @@ __global__ void __launch_bounds__(walk::NT, K ? 3 : 4) k_stress_tiled(const __gr
   if (work && ix < a.g.Nx - NH) rest = sample_column<V>(a, ix, z0, plan);
   const walk::Coefs k = coefs<Q>(a, a.nzero);
   if (!walk::wait_boxes(a.err, bar, a.wait_limit, 0)) return;
-  stress_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, n, &rest, work, r0, r1);
+  stress_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, n, a.early, &rest, work, r0, r1);
 }
 
 // Batched launches copy the instance's arguments into shared memory: the fields
@@ -725,7 +730,7 @@ __global__ void __launch_bounds__(walk::NT, 4) k_velocity_batch(const __grid_con
         prefetch_velocity(a, und, z0, x0);
       },
       [&](const HalfArgs &a, const Cells &c, bool und, int n) {
-        velocity_tile<V, X, Q, false>(a, c, und, coefs<Q>(a, b.nzero), sm, n);
+        velocity_tile<V, X, Q, false>(a, c, und, coefs<Q>(a, b.nzero), sm, n, true);
       });
 }
 
@@ -742,7 +747,7 @@ __global__ void __launch_bounds__(walk::NT, 4) k_stress_batch(const __grid_const
         prefetch_stress(a, und, z0, x0);
       },
       [&](const HalfArgs &a, const Cells &c, bool und, int n) {
-        stress_tile<V, X, Q, false>(a, c, und, coefs<Q>(a, b.nzero), sm, n, nullptr, false, 0, 0);
+        stress_tile<V, X, Q, false>(a, c, und, coefs<Q>(a, b.nzero), sm, n, true, nullptr, false, 0, 0);
       });
 }
 
@@ -869,7 +874,8 @@ void fill_args(HalfArgs &ha, const tti_handle *h, const StepArgs &a)
   ha.invdx = h->invdx;
   ha.invdz = h->invdz;
   ha.dt = c.dt;
-  tiles(h->g, h->g.izStart, &ha.z_base, &ha.tile_rows);
+  const dim3 nt = tiles(h->g, h->g.izStart, &ha.z_base, &ha.tile_rows);
+  ha.early = early_trigger((long long)nt.x * nt.y);
   ha.x_base = NH;
   ha.undamped_ok = h->undamped_ok;
   ha.freesurface = c.freesurface;
