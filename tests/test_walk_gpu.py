@@ -110,3 +110,30 @@ def test_crowded_columns(variant, fs, monkeypatch, gpu_lib):
     for k, (a, b) in enumerate(zip(*out)):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (k, np.max(np.abs(a - b)))
     assert all(np.any(b != 0) for b in out[0])
+
+
+# One velocity source per column: its window at the surface (rows that are not
+# updated), over two rows of tiles, and one row and column from the edge.
+@pytest.mark.parametrize("sx,sz", [(20, 1), (9, 108), (1, 60)])
+@pytest.mark.parametrize("stype", [2, 3, 4, 5, 6, 7, 8])
+def test_velocity_source(stype, sx, sz, monkeypatch, gpu_lib):
+    import ttifd
+
+    nz, nx, nt, eal = 150, 40, 50, 3
+    m = synthetic.layered_model(nz, nx, seed=8)
+    w = synthetic.ricker(nt, 0.0008, 30.0, delay=0.01)
+    out = []
+    for kernel in ("naive", "tiled"):
+        monkeypatch.setenv("TTIFD_EXACT", "1")
+        monkeypatch.setenv("TTIFD_KERNEL", kernel)
+        with ttifd.Modeling(variant=0, nz=nz, nx=nx, nt=nt, dx=10.0, dz=10.0, dt=0.0008, fpeak=30.0, ealThick=eal,
+                            freesurface=1, stype=stype, seistype=3) as h:
+            h.upload_model(*synthetic.padded(m, eal))
+            h.set_source([sx], [sz], w[None, :])
+            for k in (0, 1, 2):
+                h.set_receivers(k, np.arange(nx), sz)
+            h.run()
+            out.append([h.fetch_traces(k) for k in (0, 1, 2)] + [h.fetch_field(f) for f in range(5)])
+    for k, (a, b) in enumerate(zip(*out)):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (k, np.max(np.abs(a - b)))
+        assert np.any(b != 0), k

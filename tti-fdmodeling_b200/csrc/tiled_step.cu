@@ -115,6 +115,7 @@ __device__ __forceinline__ void load_coefs(const HalfArgs &a, bool und, size_t g
 // once the walks have read them, the tile's own inputs (HalfArgs::in),
 // tile_rows x WX each, the barrier.
 constexpr int V_SUMS = walk::LEAD + 3 * walk::BOX, V_BAR = V_SUMS + 6 * walk::SUM;
+constexpr int V_STASH = V_BAR + 16, V_END = V_STASH + walk::NT / 32 * 11 * 4;  // (single shots: source_terms)
 constexpr int S_IN = walk::LEAD + 2 * walk::BOX;
 static_assert(4 * walk::SUM <= 2 * walk::BOX, "the sums fit in place of the boxes");
 constexpr int s_inputs(int V) { return V == TTI_TENSOR ? 10 : 9; }
@@ -149,13 +150,13 @@ __device__ __forceinline__ void load_vcells(const HalfArgs &a, bool und, size_t 
 // d2) of sxx, szz, sxz (coord:614-672, tensor:617-666, bond:654-703).
 template <int V, bool X, bool Q, bool K>
 __device__ __forceinline__ void velocity_rows(const HalfArgs &a, const Cells &c, size_t gi, const F4 (&d)[3][2],
-                                              const VCells &p, walk::u64 nz, int n)
+                                              const VCells &p, walk::u64 nz, int n, F4 &vx, F4 &vz)
 {
   typedef walk::Rows<X> A;
   typedef typename A::T T;
   const A r{nz};
   const T invdx = r.c(a.invdx), invdz = r.c(a.invdz), half = r.c(0.5f);
-  F4 vx, vz, kd[4];
+  F4 kd[4];
 #pragma unroll
   for (int i = 0; i < A::N; ++i) {
     // x and z derivatives 0.5 (d1 +- d2) / dx, / dz (already scaled when Q)
@@ -193,10 +194,8 @@ __device__ __forceinline__ void velocity_rows(const HalfArgs &a, const Cells &c,
     A::set(vx, i, r.add(r.mul(c1, A::get(p.vx, i)), r.mul(br, fx)));
     A::set(vz, i, r.add(r.mul(c1, A::get(p.vz, i)), r.mul(br, fz)));
   }
-  const int lo = a.g.izStart, hi = min(a.g.Nz - NH, c.z0 + a.tile_rows);
-  st4(a.f.vx + gi, vx, c.z, lo, hi);
-  st4(a.f.vz + gi, vz, c.z, lo, hi);
   if (K && V == TTI_COORDINATE) {
+    const int lo = a.g.izStart, hi = min(a.g.Nz - NH, c.z0 + a.tile_rows);
     const size_t ki = kept_at(a, n) + gi;
 #pragma unroll
     for (int k = 0; k < 4; ++k) st4(a.kd[k] + ki, kd[k], c.z, lo, hi);
@@ -227,11 +226,89 @@ __device__ __forceinline__ bool tile_work(const HalfArgs &a, int z0, int &r0, in
   return r0 < a.work_z1 && r1 > a.work_z0;
 }
 
+__device__ __forceinline__ void st_shared4(float *p, const F4 &f)
+{
+  *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(f.p[0], f.p[1]);
+}
+
+// The velocity sources in the tile, one warp (all lanes) a column: as
+// column_sources, but what they add is ready when the update is done
+// (plan_sources before the wait for the previous kernel, source_terms while the
+// copies are in flight) and the column's new rows take it in shared memory.
+// Columns under several sources' windows go the general way. us a step, stype 4
+// at 60 x 80 8.0 / 7.6, 200 x 400 8.6 / 7.9, 600 x 1200 19.5 / 18.65; stype 6 in
+// the tensor rotation 401 x 857 13.3 / 12.8. A kernel of its own (W): where there
+// are no velocity sources the plain one takes 60.5 against 61.1 us a step at
+// 1126 x 3000.
+struct SourcePlan {
+  int src = -1, row = 0, mask = 0;  // the source; this lane's row; which of w there are
+  float w[4];                       // weights: to vx, to vz, then to vx, to vz again (stype 4: 2, then 3)
+  bool more = false;
+};
+__device__ __forceinline__ void plan_sources(const HalfArgs &a, int ix, int r0, int r1, SourcePlan &s)
+{
+  const Columns &p = *a.cols;
+  const int lane = threadIdx.x & 31;
+  for (int q = 0; q < p.src.n; ++q) {
+    const int dx = ix - p.src.x[q];
+    if (dx < -NH || dx > NH) continue;
+    if (s.src >= 0) {
+      s.more = true;
+      return;
+    }
+    s.src = q;
+  }
+  if (s.src < 0) return;
+  const int dx = ix - p.src.x[s.src], z = p.src.z[s.src], i = (dx + NH) * 11 + lane;
+  s.row = z + lane - NH;
+  if (p.stype == 8) {  // rows z and z - 1 of two columns
+    s.row = z - lane;
+    if (lane < 2 && (dx == 0 || dx == -1)) s.mask = 3;
+    s.w[0] = lane ? p.t.q8 : -p.t.q8;
+    s.w[1] = dx == 0 ? p.t.q8 : -p.t.q8;
+  } else if (lane <= 2 * NH) {
+    const int k = p.stype;
+    s.mask = k == 4 ? 15 : k == 5 ? 1 : k == 6 ? 2 : 3;
+    s.w[0] = k == 3 ? -p.t.kz[i] : k == 5 ? p.t.k5[i] : k == 7 ? p.t.k7[i] : p.t.kx[i];
+    s.w[1] = k == 3 ? p.t.kx[i] : k == 6 ? p.t.k5[i] : k == 7 ? p.t.k7[i] : p.t.kz[i];
+    s.w[2] = -p.t.kz[i];
+    s.w[3] = p.t.kx[i];
+  }
+  if (s.row < max(r0, 0) || s.row >= min(r1, a.g.Nz)) s.mask = 0;
+}
+
+// Rows of the tile: the terms go to `stash` (four floats a lane), returned are
+// the row and the mask. Rows that are not updated take them at once.
+constexpr int SRC_ON = 1 << 16, SRC_MORE = 1 << 17;
+__device__ __forceinline__ int source_terms(const HalfArgs &a, int ix, int z0, const SourcePlan &s, float *stash)
+{
+  if (s.more) return SRC_MORE;
+  if (s.src < 0) return 0;
+  const Columns &p = *a.cols;
+  const float t = p.src.w[(size_t)s.src * p.src.nt + time_index(p, step_of(a))];
+  if (!s.mask) return SRC_ON;
+  float u[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) u[k] = s.mask >> k & 1 ? __fmul_rn(s.w[k], t) : 0.0f;
+  if (s.row >= a.g.izStart && s.row < a.g.Nz - NH) {
+    *reinterpret_cast<float4 *>(stash) = make_float4(u[0], u[1], u[2], u[3]);
+    return SRC_ON | s.mask << 8 | (s.row - z0);
+  }
+  const size_t i = (size_t)ix * a.g.ldz + s.row;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (s.mask >> k & 1) {
+      float *v = (k & 1 ? a.f.vz : a.f.vx) + i;
+      *v = __fadd_rn(*v, u[k]);
+    }
+  return SRC_ON;
+}
+
 // Velocity update of a tile whose boxes (sxx, szz, sxz) have arrived: one warp
 // per field and 32 diagonals, then one per column.
-template <int V, bool X, bool Q, bool K>
+template <int V, bool X, bool Q, bool K, bool W>
 __device__ __forceinline__ void velocity_tile(const HalfArgs &a, const Cells &c, bool und, const walk::Coefs &k,
-                                              float *sm, int n, bool early)
+                                              float *sm, int n, bool early, int src)
 {
   const int gr = walk::groups(a.tile_rows);
   float *sums = sm + V_SUMS;
@@ -249,15 +326,45 @@ __device__ __forceinline__ void velocity_tile(const HalfArgs &a, const Cells &c,
   if (c.on) load_vcells<V>(a, und, gi, p);
   __syncthreads();  // the sums are complete
   if (!early) pdl_trigger();
+  const int lo = a.g.izStart, hi = min(a.g.Nz - NH, c.z0 + a.tile_rows);
+  F4 vx, vz;
   if (c.on) {
     F4 ds[3][2];
     read_sums(c, sums, ds);
-    velocity_rows<V, X, Q, K>(a, c, gi, ds, p, k.nz, n);
+    velocity_rows<V, X, Q, K>(a, c, gi, ds, p, k.nz, n, vx, vz);
+    if (!W || !(src & SRC_ON)) {
+      st4(a.f.vx + gi, vx, c.z, lo, hi);
+      st4(a.f.vz + gi, vz, c.z, lo, hi);
+    }
   }
-  int r0, r1;
-  if (tile_work(a, c.z0, r0, r1)) {  // this warp's column
+  if (!W) return;
+  const int lane = threadIdx.x & 31;
+  if (src & SRC_ON) {  // this warp's column
+    float *S = sums + (c.x - c.x0) * walk::DP;
+    const float *stash = sm + V_STASH + ((threadIdx.x >> 5) * 11 + lane) * 4;
+    __syncwarp();  // every lane has read the column's sums
+    if (c.on) {
+      st_shared4(S + 4 * lane, vx);
+      st_shared4(S + walk::SUM + 4 * lane, vz);
+    }
     __syncwarp();
-    if (c.x < a.g.Nx - NH) column_sources(a.g, a.f, *a.cols, c.x, n, r0, r1);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (src >> (8 + k) & 1) {
+        float *v = S + (k & 1) * walk::SUM + (src & 255);
+        *v = __fadd_rn(*v, stash[k]);
+      }
+    __syncwarp();
+    if (c.on) {
+      st4(a.f.vx + gi, ld4(S + 4 * lane), c.z, lo, hi);
+      st4(a.f.vz + gi, ld4(S + walk::SUM + 4 * lane), c.z, lo, hi);
+    }
+  }
+  if (src & SRC_MORE) {
+    int r0, r1;
+    tile_work(a, c.z0, r0, r1);
+    __syncwarp();
+    column_sources(a.g, a.f, *a.cols, c.x, n, r0, r1);
   }
 }
 
@@ -358,11 +465,6 @@ __device__ __forceinline__ void stress_rows(const HalfArgs &a, const Cells &c, s
              r.add(r.mul(c1, o2), r.mul(c2, r.add(r.add(r.mul(c15, vxx), r.mul(c35, vzz)), r.mul(c55, sh)))));
     }
   }
-}
-
-__device__ __forceinline__ void st_shared4(float *p, const F4 &f)
-{
-  *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(f.p[0], f.p[1]);
 }
 
 // The column work after the stress update in the tile, one warp (all lanes) a
@@ -611,7 +713,7 @@ __device__ __forceinline__ void stress_tile(const HalfArgs &a, const Cells &c, b
 }
 
 // Single-shot launches, one tile per CTA.
-template <int V, bool X, bool Q, bool K = false>
+template <int V, bool X, bool Q, bool K = false, bool W = false>
 __global__ void __launch_bounds__(walk::NT, 4) k_velocity_tiled(const __grid_constant__ HalfArgs a,
                                                                 const __grid_constant__ VelocityMaps m)
 {
@@ -619,15 +721,24 @@ __global__ void __launch_bounds__(walk::NT, 4) k_velocity_tiled(const __grid_con
   unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + V_BAR);
   const int z0 = a.z_base + blockIdx.x * a.tile_rows, x0 = a.x_base + blockIdx.y * WX;
   walk::init_bar(bar);
+  const int ix = x0 + (threadIdx.x >> 5);  // this warp's column
+  int r0, r1;
+  const bool work = W && tile_work(a, z0, r0, r1) && ix < a.g.Nx - NH;
+  SourcePlan plan;
+  if (work) plan_sources(a, ix, r0, r1, plan);
   pdl_wait();
   if (a.early) pdl_trigger();
   walk::issue_tile(m.box, 3, 4, nullptr, 0, 0, sm, 0, bar, z0, x0);
   const bool und = tile_undamped(a, z0, x0, WX);
   prefetch_velocity(a, und, z0, x0);
   const int n = step_of(a);
+  const int src = work ? source_terms(a, ix, z0, plan, sm + V_STASH + ((threadIdx.x >> 5) * 11 + (threadIdx.x & 31)) * 4) : 0;
   const walk::Coefs k = coefs<Q>(a, a.nzero);
   if (!walk::wait_boxes(a.err, bar, a.wait_limit, 0)) return;
-  velocity_tile<V, X, Q, K>(a, cells_of(a, z0, x0), und, k, sm, n, a.early);
+  // tiles without a source's window run the plain update: 61.4 against 62.5 us
+  // a step at 1126 x 3000, 18.65 against 19.1 at 600 x 1200
+  if (W && __syncthreads_or(src)) velocity_tile<V, X, Q, K, true>(a, cells_of(a, z0, x0), und, k, sm, n, a.early, src);
+  else velocity_tile<V, X, Q, K, false>(a, cells_of(a, z0, x0), und, k, sm, n, a.early, 0);
 }
 
 // The stress update walks the tiles in the opposite order, so that it starts
@@ -730,7 +841,7 @@ __global__ void __launch_bounds__(walk::NT, 4) k_velocity_batch(const __grid_con
         prefetch_velocity(a, und, z0, x0);
       },
       [&](const HalfArgs &a, const Cells &c, bool und, int n) {
-        velocity_tile<V, X, Q, false>(a, c, und, coefs<Q>(a, b.nzero), sm, n, true);
+        velocity_tile<V, X, Q, false, false>(a, c, und, coefs<Q>(a, b.nzero), sm, n, true, 0);
       });
 }
 
@@ -903,12 +1014,16 @@ void stress_maps(StressMaps &m, const void *maps)
 template <bool X, bool Q>
 cudaError_t velocity_xq(const HalfArgs &a, const VelocityMaps &m, int variant, cudaStream_t st)
 {
-  constexpr size_t smem = (size_t)(V_BAR + 16) * sizeof(float);
-  if (variant == TTI_COORDINATE)
-    return a.kd[0] ? launch_k(k_velocity_tiled<TTI_COORDINATE, X, Q, true>, a, m, smem, st)
-                   : launch_k(k_velocity_tiled<TTI_COORDINATE, X, Q>, a, m, smem, st);
-  if (variant == TTI_TENSOR) return launch_k(k_velocity_tiled<TTI_TENSOR, X, Q>, a, m, smem, st);
-  return launch_k(k_velocity_tiled<TTI_BOND, X, Q>, a, m, smem, st);
+  const bool kept = a.kd[0], work = a.work_z1 > a.work_z0;
+  const size_t smem = (size_t)(work ? V_END : V_BAR + 16) * sizeof(float);
+  auto go = [&](auto kernel, auto with_work) {
+    return work ? launch_k(with_work, a, m, smem, st) : launch_k(kernel, a, m, smem, st);
+  };
+  constexpr int C = TTI_COORDINATE, T = TTI_TENSOR, B = TTI_BOND;
+  if (variant == C && kept) return go(k_velocity_tiled<C, X, Q, true>, k_velocity_tiled<C, X, Q, true, true>);
+  if (variant == C) return go(k_velocity_tiled<C, X, Q>, k_velocity_tiled<C, X, Q, false, true>);
+  if (variant == T) return go(k_velocity_tiled<T, X, Q>, k_velocity_tiled<T, X, Q, false, true>);
+  return go(k_velocity_tiled<B, X, Q>, k_velocity_tiled<B, X, Q, false, true>);
 }
 
 template <int V, bool X, bool Q>
