@@ -188,7 +188,8 @@ int tti_elapsed_ms(const tti_handle *h, float *ms);
  * loop wall time, coord:927-930): advances `nsteps` steps like tti_step with
  * CUDA events on the handle's stream around each phase and returns the total
  * device ms per phase: ms[0] the velocity update, ms[1] the stress update,
- * ms[2] everything else (sources, free surface, receivers, energy). */
+ * ms[2] everything else (energy; sources, free surface and receivers where they
+ * run as launches of their own and not in the updates' tiles). */
 int tti_profile_steps(tti_handle *h, int nsteps, float ms[3]);
 /* Number of kernels this handle has launched since tti_create. */
 int tti_kernel_launches(const tti_handle *h, long long *n);

@@ -1,5 +1,5 @@
-// Device memory of the handles' bulk arrays (wavefields, parameters, packed
-// parameters, the raw model during the upload): a library-private
+// Device memory of the handles' bulk arrays (wavefields, parameters, geometry,
+// traces, the raw model during the upload): a library-private
 // stream-ordered pool per device that keeps up to POOL_KEEP bytes of freed
 // blocks. A process that creates handle after handle of the same grid (one
 // per shot) then maps device memory once: mapping 1.4 GB of fresh memory for a

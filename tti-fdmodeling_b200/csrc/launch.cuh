@@ -108,8 +108,7 @@ int handle_steps(tti_handle *h, int n1, float *const *keep, size_t stride);
 // brings the handle's Columns on the device up to date with its geometry
 int handle_columns(tti_handle *h);
 Extent handle_post_extent(const tti_handle *h);  // the cells of its work after the stress update
-// Fields of one kept step of the gradient (the arrays `keep` of handle_step
-// points at). Tiled kernels: the strain rates vxx vxz vzx vzz, then for the
+// Fields of one kept step of the gradient (the arrays `keep` of handle_steps). Tiled kernels: the strain rates vxx vxz vzx vzz, then for the
 // coordinate rotation the stress derivative combinations P Q R S (8 fields),
 // for the tensor rotation txx tzz txz before the stress half (7), for Bond
 // nothing more (4). Per-cell kernels: vx vz after the velocity half and the

@@ -18,11 +18,15 @@
 // with one cell per thread and ten shared reads per sum); its own inputs come
 // by TMA too, with which four CTAs fit an SM and no load waits behind a
 // barrier (91 us when loaded into registers after the walks). The velocity
-// update (70 us; 94 us before) is bound by the copies' latency at four CTAs per
-// SM (the registers' limit), 5.2 TB/s; TMA for its five inputs measured 71 us,
-// a persistent grid with the next tile's copies in flight 98 us.
+// update (66 us; 94 us before) is bound by the copies' latency at four CTAs per
+// SM (the registers' limit), 5.7 TB/s; TMA for its five inputs measured 71 us,
+// a persistent grid with the next tile's copies in flight 98 us, sums in the
+// boxes' place, which leaves more L1 but needs two barriers more, 74 us.
 // Tiles of at most 120 rows need four warps of diagonals per field (128 rows
-// need five): 200 x 400 takes 11.5 against 13.9 us a step with 128.
+// need five): 200 x 400 took 11.5 against 13.9 us a step with 128.
+//
+// A small grid is bound by the latency of its two launches, each about 2.5 us in
+// a graph of which 2 are copies' latency, walk, update and stores in series.
 #include <cudaTypedefs.h>
 
 #include <algorithm>
@@ -215,8 +219,9 @@ __device__ __forceinline__ void read_sums(const Cells &c, const float *sums, F4 
 }
 
 // Column work in the tiles instead of a launch between the half-steps: us a
-// step with and without, 60 x 80 9.1 / 9.8, 200 x 400 11.6 / 14.3, 600 x 1200
-// 19.2 / 20.2, 1126 x 7872 147.1 / 150.6.
+// step with and without, when it was moved (before it went off the critical
+// path, column_work), 60 x 80 9.1 / 9.8, 200 x 400 11.6 / 14.3, 600 x 1200 19.2 /
+// 20.2, 1126 x 7872 147.1 / 150.6.
 // The rows whose column work a tile does: its own, the first and the last tile
 // also those above and below all tiles.
 __device__ __forceinline__ bool tile_work(const HalfArgs &a, int z0, int &r0, int &r1)
