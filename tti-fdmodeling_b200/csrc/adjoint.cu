@@ -1601,21 +1601,11 @@ int tti_grad_zero(tti_handle *h)
 
 namespace {
 
-// Buffers and tables of a gradient run: `slots` full-state checkpoints and a
-// kept segment of `seg` steps (keep_fields each); the source tables in *tab.
-int grad_prepare(tti_handle *h, int slots, int seg, SourceTables *tab)
+// `slots` full-state checkpoints and a kept segment of `seg` steps (keep_fields
+// each).
+int reserve(tti_handle *h, int slots, int seg)
 {
-  int rc = grad_check(h);
-  if (rc) return rc;
-  GCK(h, cudaSetDevice(h->device));
-  if ((rc = grad_alloc(h))) return rc;
   GradState *s = h->grad;
-  const tti_config &c = h->cfg;
-  const bool want_v = c.seistype == 1 || c.seistype == 3, want_p = c.seistype == 2 || c.seistype == 3;
-  for (int k = 0; k < 3; ++k) {
-    const bool rec = (k < 2 ? want_v : want_p) && h->nrec[k] > 0;
-    if (rec && !s->have_obs[k]) return gerr(h, TTI_ERR_STATE, "observed traces missing for a recorded component");
-  }
   const int nf = h->cfg.variant == TTI_TENSOR ? 8 : 5;  // fields of a full state (checkpoints)
   const int nk = keep_fields(h);                       // fields of a kept step
   const size_t n = h->g.n;
@@ -1642,6 +1632,25 @@ int grad_prepare(tti_handle *h, int slots, int seg, SourceTables *tab)
         return gerr(h, TTI_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     }
   }
+  return TTI_OK;
+}
+
+// Buffers and tables of a gradient run: `slots` full-state checkpoints and a
+// kept segment of `seg` steps (keep_fields each); the source tables in *tab.
+int grad_prepare(tti_handle *h, int slots, int seg, SourceTables *tab)
+{
+  int rc = grad_check(h);
+  if (rc) return rc;
+  GCK(h, cudaSetDevice(h->device));
+  if ((rc = grad_alloc(h))) return rc;
+  GradState *s = h->grad;
+  const tti_config &c = h->cfg;
+  const bool want_v = c.seistype == 1 || c.seistype == 3, want_p = c.seistype == 2 || c.seistype == 3;
+  for (int k = 0; k < 3; ++k) {
+    const bool rec = (k < 2 ? want_v : want_p) && h->nrec[k] > 0;
+    if (rec && !s->have_obs[k]) return gerr(h, TTI_ERR_STATE, "observed traces missing for a recorded component");
+  }
+  if ((rc = reserve(h, slots, seg))) return rc;
   const int nt = c.nt;
   if (s->gsrc_n != h->nsrc * nt) {
     cudaFree(s->gsrc);
@@ -1739,6 +1748,24 @@ int grad_finish(tti_handle *h, const double &J, double *misfit)
 }  // namespace
 
 namespace ttifd {
+
+// The macro-steps of a binomial schedule, its numbers cut to what the run has.
+static int macro_steps(const tti_handle *h, int *snapshots, int *keep_steps)
+{
+  const int nt = h->cfg.nt;
+  *keep_steps = std::min(*keep_steps, nt);
+  const int M = (nt + *keep_steps - 1) / *keep_steps;
+  *snapshots = std::min(*snapshots, M - 1);
+  return M;
+}
+
+int grad_reserve(tti_handle *h, int snapshots, int keep_steps)
+{
+  macro_steps(h, &snapshots, &keep_steps);
+  int rc = grad_check(h);
+  if (!rc) rc = grad_alloc(h);
+  return rc ? rc : reserve(h, snapshots, keep_steps);
+}
 
 // One step of a gradient run's checkpoint schedule (macro-steps a .. b-1).
 struct Action {
@@ -1926,10 +1953,7 @@ int tti_grad_run(tti_handle *h, int ncheck, double *misfit)
 int tti_grad_run_binomial(tti_handle *h, int snapshots, int keep_steps, double *misfit)
 {
   if (!h || snapshots < 0 || keep_steps < 1) return TTI_ERR_ARG;
-  const int nt = h->cfg.nt;
-  keep_steps = std::min(keep_steps, nt);
-  const int M = (nt + keep_steps - 1) / keep_steps;
-  snapshots = std::min(snapshots, M - 1);
+  const int nt = h->cfg.nt, M = ttifd::macro_steps(h, &snapshots, &keep_steps);
   SourceTables tab;
   int rc = grad_prepare(h, snapshots, keep_steps, &tab);
   if (rc) return rc;

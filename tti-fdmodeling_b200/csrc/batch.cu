@@ -7,6 +7,7 @@
 // step counter, so the launches of G steps are captured once in a CUDA graph
 // and the graph is replayed for the whole loop.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <thread>
 #include <cstdarg>
@@ -511,14 +512,30 @@ int tti_batch_grad_run(tti_batch *b, int snapshots, int keep_steps, double *misf
   std::vector<double> J(n, 0.0);
   const auto t0 = std::chrono::steady_clock::now();
   {
-    // one host thread per instance: each drives its own stream, so the
-    // kernels of different shots overlap on the device
+    // host threads that take instances one after another, each instance on its
+    // own stream, so the kernels of different shots overlap on the device. Not
+    // all at once: up to 8, as more streams share the device's 8 queues, and no
+    // more than have their arrays (about 32 with the parameters) in L2, at least
+    // 4, which fill the device. ms with all / so many: 16 shots of 60 x 80 21.6 /
+    // 16.6 (8), 16 of 200 x 400 40.4 / 34.7 (8), 8 of 300 x 600 31.5 / 29.5 (4),
+    // 16 63.4 / 58.5 (4), 8 of 600 x 1200 53.3 / 51.5 (4), 6 of 1126 x 2000 34.6 /
+    // 34.9 (4).
+    size_t cells = 0;
+    for (const tti_handle *h : b->inst) cells = std::max(cells, h->g.n);
+    int l2 = 0;
+    BCK(b, cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, b->device));
+    const int workers = std::min<int>(n, std::clamp<size_t>(l2 / (32 * sizeof(float) * cells), 4, 8));
+    // device memory first: allocating between running shots stops them (a
+    // shortage is reported by the run that meets it)
+    for (tti_handle *h : b->inst)
+      if (grad_reserve(h, snapshots, keep_steps) != TTI_OK) break;
+    std::atomic<int> next{0};
     std::vector<std::thread> th;
-    th.reserve(n);
-    for (int i = 0; i < n; ++i)
-      th.emplace_back([&, i] {
+    th.reserve(workers);
+    for (int w = 0; w < workers; ++w)
+      th.emplace_back([&] {
         cudaSetDevice(b->device);
-        rc[i] = tti_grad_run_binomial(b->inst[i], snapshots, keep_steps, &J[i]);
+        for (int i; (i = next++) < n;) rc[i] = tti_grad_run_binomial(b->inst[i], snapshots, keep_steps, &J[i]);
       });
     for (auto &t : th) t.join();
   }

@@ -114,6 +114,8 @@ Extent handle_post_extent(const tti_handle *h);  // the cells of its work after 
 // nothing more (4). Per-cell kernels: vx vz after the velocity half and the
 // stresses (tensor: tau) before the stress half (5).
 int keep_fields(const tti_handle *h);
+// allocates what tti_grad_run_binomial of these numbers needs (adjoint.cu)
+int grad_reserve(tti_handle *h, int snapshots, int keep_steps);
 // frees the gradient's device memory of h (adjoint.cu)
 void grad_release(tti_handle *h);
 int create_handle(tti_handle **out, const tti_config *cfg, int device, const tti_handle *share, bool force_tiled);
