@@ -308,7 +308,6 @@ int tti_batch_create(tti_batch **out, int nmodels, const tti_config *cfg, int ni
     b->model_of[i] = m;
     if (!b->inst[i] && (rc = create_handle(&b->inst[i], &cfg[m], device, b->models[m], true)))
       return fail(rc, tti_last_error(nullptr));
-    b->inst[i]->alone = ninst == 1;
   }
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||

@@ -39,7 +39,6 @@ struct alignas(16) HalfArgs {
   float hc[5]; // h * C_k
   float nzero; // -0.0f (see walk::coefs)
   int early;   // trigger the next kernel at the start (early_trigger)
-  int three;   // three CTAs per SM (three_per_sm)
   // Gradient forward pass (null: nothing kept). Velocity update, coordinate
   // rotation: per cell the stress derivative combinations the adjoint's
   // theta_v terms need (sxz_x - sxx_z, szz_x - sxz_z, sxx_x + sxz_z,
@@ -90,16 +89,6 @@ bool encode_maps(CUtensorMap *map, const Grid &g, int variant, const Fields &f, 
 // (440 tiles) 12.0 / 11.4, 500 x 1000 15.1 / 14.4, 600 x 1200 18.4 / 17.9,
 // 1126 x 3000 61.0 / 60.4.
 inline int early_trigger(long long tiles) { return 2 * tiles <= 4 * 148; }
-// Grids that give the SMs between two and a half and three CTAs run with room
-// for three, and then trigger early: with a fourth slot the next launch's first
-// CTAs take it where they find it, and the others end up four on one SM and two
-// on the next. us a step, three / four: 300 x 850 (348 tiles) 10.46 / 10.40, 300
-// x 1000 (405) 10.45 / 10.9, 400 x 800 (440) 10.5 / 11.8, tensor 11.05 / 12.5; 400
-// x 850 (464) 12.7 / 12.1. Not for a batch's instances, which share the SMs.
-inline int three_per_sm(long long tiles) { return 2 * tiles > 5 * 148 && tiles <= 3 * 148; }
-// the least dynamic shared memory of which four do not fit (228 KB, 1 KB a CTA
-// the system's)
-constexpr size_t THREE_BYTES = 233472 / 4 - 1024 + 128;
 // The arguments of h's half-steps (a: handle_step_args), without column work.
 void fill_args(HalfArgs &ha, const tti_handle *h, const StepArgs &a);
 void velocity_maps(VelocityMaps &m, const void *maps);  // from a handle's maps

@@ -903,10 +903,8 @@ template <typename M>
 cudaError_t launch_k(void (*kernel)(HalfArgs, M), const HalfArgs &a, const M &m, size_t smem, cudaStream_t st)
 {
   int wave = 0;
-  const size_t three = std::max(smem, THREE_BYTES);
-  const cudaError_t e = prepare_kernel(kernel, three, &wave);
+  const cudaError_t e = prepare_kernel(kernel, smem, &wave);
   if (e != cudaSuccess) return e;
-  if (a.three) smem = three;
   int z_base, rows;
   const dim3 gr = tiles(a.g, a.g.izStart, &z_base, &rows);
   if (gr.x == 0 || gr.y == 0) return cudaSuccess;
@@ -993,9 +991,7 @@ void fill_args(HalfArgs &ha, const tti_handle *h, const StepArgs &a)
   ha.invdz = h->invdz;
   ha.dt = c.dt;
   const dim3 nt = tiles(h->g, h->g.izStart, &ha.z_base, &ha.tile_rows);
-  const long long tiles_ = (long long)nt.x * nt.y;
-  ha.three = h->alone && three_per_sm(tiles_);
-  ha.early = ha.three || early_trigger(tiles_);
+  ha.early = early_trigger((long long)nt.x * nt.y);
   ha.x_base = NH;
   ha.undamped_ok = h->undamped_ok;
   ha.freesurface = c.freesurface;

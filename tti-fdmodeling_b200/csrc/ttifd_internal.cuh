@@ -200,7 +200,6 @@ struct tti_handle {
   int *d_clk = nullptr;              // step counters for the graphs (tiled::StepClock)
   ttifd::StepGraph graph[2];
   bool use_graphs = false;           // steps by graph replays (create_handle)
-  bool alone = true;                 // not one of a batch's instances, which run side by side
   double *d_energy = nullptr;  // [nt][2]
   int *d_flag = nullptr;       // nonfinite watchdog
   float *d_snap = nullptr;      // packed snapshot kinds of one step, snap_cap floats
