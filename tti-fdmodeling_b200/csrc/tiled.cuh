@@ -182,6 +182,10 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned pari
   return false;
 }
 
+// Orders this thread's plain accesses to shared memory before copies (the async
+// proxy) that are issued behind the next block barrier.
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 __device__ __forceinline__ void tma_load_2d(float *dst, const CUtensorMap *map, int c_inner, int c_outer,
                                             unsigned long long *bar)
 {

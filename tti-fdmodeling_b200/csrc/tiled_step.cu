@@ -816,7 +816,9 @@ __device__ __forceinline__ bool work_item(const BatchArgs &b, int i, int n, unsi
 // for the stress update, as in the single-shot kernels): one item per CTA when
 // the grid covers the table, several (LOOP) when a persistent grid of one
 // resident wave walks it. The tile's shared memory is reused by the next item
-// only after every thread is done with it.
+// only after every thread is done with it: the stress sums take the boxes'
+// place with plain stores, which nothing but a proxy fence orders before the
+// next item's copies into it.
 template <bool LOOP, typename I, typename F>
 __device__ __forceinline__ void for_work(const BatchArgs &b, bool reverse, unsigned long long *bar, I issue, F f)
 {
@@ -830,6 +832,7 @@ __device__ __forceinline__ void for_work(const BatchArgs &b, bool reverse, unsig
   }
   for (int i = blockIdx.x; i < b.nwork; i += gridDim.x) {
     if (!work_item(b, reverse ? b.nwork - 1 - i : i, n, bar, ph, issue, f)) return;
+    tma::fence_async();  // the next copies land where this item's sums were stored
     __syncthreads();
   }
 }
