@@ -23,6 +23,21 @@ __device__ __forceinline__ int record_index(const Columns &p, int it)
   return p.rec_on && it % p.mt == 0 ? it / p.mt : -1;
 }
 
+// A column's sources at time index it. The pointers are read once: what they
+// lie in is in global memory too, and the sources' stores could change it.
+struct ColumnSources {
+  int first, last;
+  const int4 *sat;
+  const float *a;
+  int nt;
+  __device__ __forceinline__ ColumnSources(const Columns &p, int ix, int it)
+      : first(p.scol[ix]), last(p.scol[ix + 1]), sat(p.sat), a(p.amp + it), nt(p.nt)
+  {
+  }
+  __device__ __forceinline__ int4 at(int j) const { return __ldg(sat + j); }
+  __device__ __forceinline__ float amp(const int4 &s) const { return __ldg(a + (size_t)s.x * nt); }
+};
+
 // Rows [r0, r1) of column ix after the stress update, one warp (all lanes).
 // With `pdl` the column's receiver geometry (static since the receivers were
 // set) is read before waiting for the previous kernel, so those loads overlap
@@ -71,17 +86,17 @@ __device__ __forceinline__ void column_post(const Grid &g, const Fields &f, cons
     __syncwarp();
   }
   if (p.stype == 1) {
-    for (int q = 0; q < p.src.n; ++q) {
-      const int dx = ix - p.src.x[q];
-      if (dx < -NH || dx > NH) continue;
-      const int iz = p.src.z[q] + lane - NH;
+    const ColumnSources src(p, ix, it);
+    const bool tensor = p.tensor;
+    for (int j = src.first; j < src.last; ++j) {
+      const int4 s = src.at(j);
+      const int iz = s.y + lane - NH;
       if (lane <= 2 * NH && iz >= 0 && iz < g.Nz && iz >= r0 && iz < r1) {
-        const float a = p.src.w[(size_t)q * p.src.nt + it];
-        const float ws = __fmul_rn(p.t.k1[(dx + NH) * 11 + lane], a);
+        const float ws = __fmul_rn(__ldg(p.t.k1 + (s.z + NH) * 11 + lane), src.amp(s));
         const size_t c = col + iz;
         f.sxx[c] = __fadd_rn(f.sxx[c], ws);
         f.szz[c] = __fadd_rn(f.szz[c], ws);
-        if (p.tensor) {
+        if (tensor) {
           f.txx[c] = __fadd_rn(f.txx[c], ws);
           f.tzz[c] = __fadd_rn(f.tzz[c], ws);
         }
@@ -124,11 +139,14 @@ __device__ __forceinline__ void column_sources(const Grid &g, const Fields &f, c
 {
   const int lane = threadIdx.x & 31, it = time_index(p, n);
   const size_t col = (size_t)ix * g.ldz;
+  const ColumnSources src(p, ix, it);
   if (p.stype == 8) {  // coord:782-801: four cells, one lane
-    for (int q = 0; q < p.src.n && lane == 0; ++q) {
-      const int dx = ix - p.src.x[q], z = p.src.z[q];
+    const float k = p.t.q8;
+    for (int j = src.first; j < src.last && lane == 0; ++j) {
+      const int4 s = src.at(j);
+      const int dx = s.z, z = s.y;
       if (dx != 0 && dx != -1) continue;
-      const float a = p.src.w[(size_t)q * p.src.nt + it], k = p.t.q8;
+      const float a = src.amp(s);
       if (z >= r0 && z < r1) {
         dec(f.vx + col + z, k, a);
         if (dx == 0) acc(f.vz + col + z, k, a);
@@ -144,26 +162,25 @@ __device__ __forceinline__ void column_sources(const Grid &g, const Fields &f, c
   }
   const int first = p.stype == 4 ? 2 : p.stype, last = p.stype == 4 ? 3 : p.stype;  // stype 4: 2, then 3
   for (int kind = first; kind <= last; ++kind)
-    for (int q = 0; q < p.src.n; ++q) {
-      const int dx = ix - p.src.x[q];
-      if (dx < -NH || dx > NH) continue;
-      const int iz = p.src.z[q] + lane - NH, w = (dx + NH) * 11 + lane;
+    for (int j = src.first; j < src.last; ++j) {
+      const int4 s = src.at(j);
+      const int iz = s.y + lane - NH, w = (s.z + NH) * 11 + lane;
       if (lane <= 2 * NH && iz >= 0 && iz < g.Nz && iz >= r0 && iz < r1) {
-        const float a = p.src.w[(size_t)q * p.src.nt + it];
+        const float a = src.amp(s);
         float *vx = f.vx + col + iz, *vz = f.vz + col + iz;
         if (kind == 2) {
-          acc(vx, p.t.kx[w], a);
-          acc(vz, p.t.kz[w], a);
+          acc(vx, __ldg(p.t.kx + w), a);
+          acc(vz, __ldg(p.t.kz + w), a);
         } else if (kind == 3) {
-          dec(vx, p.t.kz[w], a);
-          acc(vz, p.t.kx[w], a);
+          dec(vx, __ldg(p.t.kz + w), a);
+          acc(vz, __ldg(p.t.kx + w), a);
         } else if (kind == 5) {
-          acc(vx, p.t.k5[w], a);
+          acc(vx, __ldg(p.t.k5 + w), a);
         } else if (kind == 6) {
-          acc(vz, p.t.k5[w], a);
+          acc(vz, __ldg(p.t.k5 + w), a);
         } else {
-          acc(vx, p.t.k7[w], a);
-          acc(vz, p.t.k7[w], a);
+          acc(vx, __ldg(p.t.k7 + w), a);
+          acc(vz, __ldg(p.t.k7 + w), a);
         }
       }
       __syncwarp();

@@ -67,7 +67,13 @@ void launch_energy(const StepArgs &a, int nz, int nx, double *out2, cudaStream_t
 struct Columns {
   int stype;  // 0: no sources
   int freesurface, tensor, nt, mode2, mt, rec_on;
-  SourceSet src;
+  // sources by the columns their windows cover: entries [scol[ix], scol[ix + 1])
+  // of sat, in the sources' order: source, row, column offset ix - x, and in a
+  // column's first one the number of its entries. shead[ix]: that first one (all
+  // 0: none), one load away.
+  const int *scol;
+  const int4 *sat, *shead;
+  const float *amp;  // [source][nt]
   SourceTables t;
   const int *colptr[3], *rz[3], *rid[3];  // receivers grouped by column (null: component off)
   float *rec[3];

@@ -254,17 +254,11 @@ __device__ __forceinline__ void plan_sources(const HalfArgs &a, int ix, int r0, 
 {
   const Columns &p = *a.cols;
   const int lane = threadIdx.x & 31;
-  for (int q = 0; q < p.src.n; ++q) {
-    const int dx = ix - p.src.x[q];
-    if (dx < -NH || dx > NH) continue;
-    if (s.src >= 0) {
-      s.more = true;
-      return;
-    }
-    s.src = q;
-  }
-  if (s.src < 0) return;
-  const int dx = ix - p.src.x[s.src], z = p.src.z[s.src], i = (dx + NH) * 11 + lane;
+  const int4 e = __ldg(p.shead + ix);
+  s.more = e.w > 1;
+  if (e.w != 1) return;
+  s.src = e.x;
+  const int dx = e.z, z = e.y, i = (dx + NH) * 11 + lane;
   s.row = z + lane - NH;
   if (p.stype == 8) {  // rows z and z - 1 of two columns
     s.row = z - lane;
@@ -290,7 +284,7 @@ __device__ __forceinline__ int source_terms(const HalfArgs &a, int ix, int z0, c
   if (s.more) return SRC_MORE;
   if (s.src < 0) return 0;
   const Columns &p = *a.cols;
-  const float t = p.src.w[(size_t)s.src * p.src.nt + time_index(p, step_of(a))];
+  const float t = p.amp[(size_t)s.src * p.nt + time_index(p, step_of(a))];
   if (!s.mask) return SRC_ON;
   float u[4];
 #pragma unroll
@@ -526,19 +520,15 @@ __device__ __forceinline__ void plan_column(const HalfArgs &a, int ix, int r0, i
       c.more |= re[k] - rb[k] > 32;
     }
   }
-  if (p.stype == 1)
-    for (int q = 0; q < p.src.n; ++q) {
-      const int dx = ix - p.src.x[q];
-      if (dx < -NH || dx > NH) continue;
-      if (c.src >= 0) {
-        c.more = true;
-        break;
-      }
-      c.src = q;
-      c.sz = p.src.z[q] + lane - NH;
-      if (lane > 2 * NH || c.sz < r0 || c.sz >= r1) c.sz = -1;
-      else c.ws = p.t.k1[(dx + NH) * 11 + lane];
-    }
+  if (p.stype == 1) {
+    const int4 e = __ldg(p.shead + ix);
+    if (e.w == 0) return;
+    c.more |= e.w > 1;
+    c.src = e.x;
+    c.sz = e.y + lane - NH;
+    if (lane > 2 * NH || c.sz < r0 || c.sz >= r1) c.sz = -1;
+    else c.ws = p.t.k1[(e.z + NH) * 11 + lane];
+  }
 }
 
 __device__ __forceinline__ void put_sample(const Columns &p, float *rec, float v)
@@ -556,7 +546,7 @@ __device__ __forceinline__ ColumnRest sample_column(const HalfArgs &a, int ix, i
   const int it = time_index(p, step_of(a)), irec = record_index(p, it);
   ColumnRest w;
   w.more = c.more;
-  if (c.src >= 0) w.ws = __fmul_rn(c.ws, p.src.w[(size_t)c.src * p.src.nt + it]);
+  if (c.src >= 0) w.ws = __fmul_rn(c.ws, p.amp[(size_t)c.src * p.nt + it]);
   if (c.sz >= 0) {
     w.sr = c.sz - z0 + 8;
     if (V == TTI_TENSOR && c.sz < max(z0, a.g.izStart)) {  // tau of the image rows changes nowhere else
@@ -581,14 +571,15 @@ __device__ __forceinline__ void more_work(const HalfArgs &a, int ix, int r0, int
 {
   const Columns &p = *a.cols;
   const int lane = threadIdx.x & 31, it = time_index(p, step_of(a)), irec = record_index(p, it);
-  bool first = true;
-  for (int q = 0; q < (p.stype == 1 ? p.src.n : 0); ++q) {
-    const int dx = ix - p.src.x[q], iz = p.src.z[q] + lane - NH;
-    if (dx < -NH || dx > NH) continue;
-    if (!first && lane <= 2 * NH && iz >= r0 && iz < r1)
-      source(iz, __fmul_rn(p.t.k1[(dx + NH) * 11 + lane], p.src.w[(size_t)q * p.src.nt + it]), false);
-    first = false;
-    __syncwarp();
+  if (p.stype == 1) {
+    const ColumnSources src(p, ix, it);
+    for (int j = src.first + 1; j < src.last; ++j) {
+      const int4 s = src.at(j);
+      const int iz = s.y + lane - NH;
+      if (lane <= 2 * NH && iz >= r0 && iz < r1)
+        source(iz, __fmul_rn(__ldg(p.t.k1 + (s.z + NH) * 11 + lane), src.amp(s)), false);
+      __syncwarp();
+    }
   }
   if (irec < 0) return;
   for (int k = 0; k < 3; ++k) {

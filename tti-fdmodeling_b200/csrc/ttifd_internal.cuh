@@ -186,7 +186,8 @@ struct tti_handle {
   float invdx = 0, invdz = 0, alpha_src = 0;
   // geometry
   int nsrc = 0;
-  int *d_sx = nullptr, *d_sz = nullptr;
+  int4 *d_sat = nullptr, *d_shead = nullptr;  // sources by column (Columns::sat); d_sat owns the block of these five
+  int *d_sx = nullptr, *d_sz = nullptr, *d_scol = nullptr;
   float *d_src = nullptr;
   int nrec[3] = {0, 0, 0};
   int *d_rz[3] = {};  // receiver rows in the caller's order; owns the block d_rzs, d_rid, d_rcol point into
