@@ -1216,11 +1216,8 @@ int adj_z_lo(const tti_handle *h)
   return h->cfg.freesurface ? std::max(NH, h->g.izStart - NH) : h->g.izStart;
 }
 
-int grad_alloc(tti_handle *h)
+int fill_grad(tti_handle *h, GradState *s)
 {
-  if (h->grad) return TTI_OK;
-  GradState *s = new GradState();
-  h->grad = s;
   const size_t n = h->g.n;
   auto al = [&](float **p) {
     if (cudaMalloc(p, n * sizeof(float)) != cudaSuccess) return false;
@@ -1260,6 +1257,20 @@ int grad_alloc(tti_handle *h)
   }
   GCK(h, cudaStreamSynchronize(h->stream));
   return TTI_OK;
+}
+
+// The gradient's arrays, allocated once: all of them, or after a failure none
+// (a later call tries again).
+int grad_alloc(tti_handle *h)
+{
+  if (h->grad) return TTI_OK;
+  h->grad = new GradState();
+  const int rc = fill_grad(h, h->grad);
+  if (rc == TTI_OK) return TTI_OK;
+  cudaStreamSynchronize(h->stream);  // zeroing under way
+  grad_release(h);
+  cudaGetLastError();
+  return rc;
 }
 
 AdjArgs adj_args(tti_handle *h, int slot)
@@ -1609,29 +1620,31 @@ int reserve(tti_handle *h, int slots, int seg)
   const int nf = h->cfg.variant == TTI_TENSOR ? 8 : 5;  // fields of a full state (checkpoints)
   const int nk = keep_fields(h);                       // fields of a kept step
   const size_t n = h->g.n;
-  if (s->ncheck != slots + 1 || s->seg != seg || s->nkeep != nk) {
+  if (s->ncheck == slots + 1 && s->seg == seg && s->nkeep == nk) return TTI_OK;
+  auto drop = [s] {  // nothing half-allocated stays behind; the handle stays usable
     cudaFree(s->ckpt);
     cudaFree(s->keep);
     s->ckpt = s->keep = nullptr;
-    if (cudaMalloc(&s->ckpt, sizeof(float) * nf * n * std::max(1, slots)) != cudaSuccess ||
-        cudaMalloc(&s->keep, sizeof(float) * nk * n * seg) != cudaSuccess) {
-      cudaGetLastError();
-      cudaFree(s->ckpt);  // nothing half-allocated stays behind; the handle stays usable
-      cudaFree(s->keep);
-      s->ckpt = s->keep = nullptr;
-      s->ncheck = s->seg = s->nkeep = 0;
-      return gerr(h, TTI_ERR_NOMEM, "device allocation of the checkpoints failed (use fewer steps per segment)");
-    }
-    s->ncheck = slots + 1;
-    s->seg = seg;
-    s->nkeep = nk;
-    if (h->use_tiled) {
-      int z_base, rows;
-      tiled::tiles(h->g, adj_z_lo(h), &z_base, &rows);
-      if (!tiled::encode_map3(s->maps + 8, h->g, s->keep, seg * nk, rows, WX))
-        return gerr(h, TTI_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    s->ncheck = s->seg = s->nkeep = 0;
+  };
+  drop();
+  if (cudaMalloc(&s->ckpt, sizeof(float) * nf * n * std::max(1, slots)) != cudaSuccess ||
+      cudaMalloc(&s->keep, sizeof(float) * nk * n * seg) != cudaSuccess) {
+    cudaGetLastError();
+    drop();
+    return gerr(h, TTI_ERR_NOMEM, "device allocation of the checkpoints failed (use fewer steps per segment)");
+  }
+  if (h->use_tiled) {
+    int z_base, rows;
+    tiled::tiles(h->g, adj_z_lo(h), &z_base, &rows);
+    if (!tiled::encode_map3(s->maps + 8, h->g, s->keep, seg * nk, rows, WX)) {
+      drop();
+      return gerr(h, TTI_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     }
   }
+  s->ncheck = slots + 1;
+  s->seg = seg;
+  s->nkeep = nk;
   return TTI_OK;
 }
 
