@@ -248,7 +248,10 @@ int tti_fetch_energy(tti_handle *h, float *ek, float *ep);
 #define TTI_G_EPS 1
 #define TTI_G_DELTA 2
 #define TTI_G_THETA 3
-/* Observed traces of one recorded component, [ntrace][(nt-1)/mt+1]. */
+/* Observed traces of one recorded component, [ntrace][(nt-1)/mt+1], ntrace its
+ * receivers at the time of the call. They stay until they are set again; a
+ * gradient run whose component has another number of receivers by then returns
+ * TTI_ERR_STATE. */
 int tti_grad_set_observed(tti_handle *h, int kind, const float *dobs);
 int tti_grad_zero(tti_handle *h);
 /* tti_elapsed_ms afterwards gives the device time of the whole run. */

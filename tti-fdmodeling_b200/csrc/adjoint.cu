@@ -52,7 +52,7 @@ struct GradState {
   float *gsrc = nullptr;    // [nsrc][nt]
   int gsrc_n = 0;
   double *d_J = nullptr;
-  bool have_obs[3] = {};
+  int obs_n[3] = {};        // traces in obs and res (0: none)
   CUtensorMap *maps = nullptr;  // host copies, 64-byte aligned: T0..T3, TV0..TV3, the kept steps, 7 parameters
   // velocity sources (stype 2-8): per source vm cells (ix, iz, index in the
   // rim list or -1; ix < 0: off the grid) with weights (wx, wz),
@@ -1586,13 +1586,14 @@ int tti_grad_set_observed(tti_handle *h, int kind, const float *dobs)
   cudaFree(s->obs[kind]);
   cudaFree(s->res[kind]);
   s->obs[kind] = s->res[kind] = nullptr;
+  s->obs_n[kind] = 0;
   GCK(h, cudaMalloc(&s->obs[kind], sizeof(float) * (size_t)n * nts));
   GCK(h, cudaMalloc(&s->res[kind], sizeof(float) * (size_t)n * nts));
   std::vector<float> tm((size_t)n * nts);  // [ntrace][nts] -> time-major
   for (int r = 0; r < n; ++r)
     for (int t = 0; t < nts; ++t) tm[(size_t)t * n + r] = dobs[(size_t)r * nts + t];
   GCK(h, cudaMemcpy(s->obs[kind], tm.data(), sizeof(float) * tm.size(), cudaMemcpyHostToDevice));
-  s->have_obs[kind] = true;
+  s->obs_n[kind] = n;
   return TTI_OK;
 }
 
@@ -1661,7 +1662,10 @@ int grad_prepare(tti_handle *h, int slots, int seg, SourceTables *tab)
   const bool want_v = c.seistype == 1 || c.seistype == 3, want_p = c.seistype == 2 || c.seistype == 3;
   for (int k = 0; k < 3; ++k) {
     const bool rec = (k < 2 ? want_v : want_p) && h->nrec[k] > 0;
-    if (rec && !s->have_obs[k]) return gerr(h, TTI_ERR_STATE, "observed traces missing for a recorded component");
+    if (rec && s->obs_n[k] == 0)
+      return gerr(h, TTI_ERR_STATE, "observed traces missing for a recorded component");
+    if (rec && s->obs_n[k] != h->nrec[k])  // the receivers were set again
+      return gerr(h, TTI_ERR_STATE, "as many observed traces as a recorded component has receivers are needed");
   }
   if ((rc = reserve(h, slots, seg))) return rc;
   const int nt = c.nt;
