@@ -46,3 +46,22 @@ def test_another_number_of_receivers(n, gpu_lib):
         _receivers(h, n, kinds=(1,))
         _observed(h, n, kinds=(1,))
         assert 0 < h.grad_run(2) < np.inf
+
+
+def test_component_that_is_not_recorded(gpu_lib):
+    """Observed traces of a component that seistype leaves out change nothing."""
+    out = []
+    for kinds in ((0, 1, 2), (0, 1)):
+        with _handle(seistype=1) as h:
+            _receivers(h, NX, (0, 1))
+            _observed(h, NX, (0, 1))
+            if 2 in kinds:  # the smaller arrays fall into the freed memory of the larger
+                h.set_receivers(2, np.arange(NX).repeat(8), 3)
+                h.grad_set_observed(2, np.full((8 * NX, NT), 1e3, np.float32))
+                _receivers(h, NX, (2,))
+                h.grad_set_observed(2, np.full((NX, NT), 1e3, np.float32))
+            h.grad_zero()
+            h.grad_run(2)
+            out.append([h.grad_fetch(n) for n in ("vp", "eps", "delta", "theta")])
+    for got, ref in zip(*out):
+        assert np.array_equal(got.view(np.uint32), ref.view(np.uint32)) and np.any(ref != 0)

@@ -1210,6 +1210,13 @@ int grad_check(tti_handle *h)
   return TTI_OK;
 }
 
+// Whether component k enters the misfit: seistype records it and it has receivers.
+bool recorded(const tti_handle *h, int k)
+{
+  const int s = h->cfg.seistype;
+  return (s == 3 || s == (k < 2 ? 1 : 2)) && h->nrec[k] > 0;
+}
+
 // first row of the transposed velocity stencils: with a free surface the image rows too
 int adj_z_lo(const tti_handle *h)
 {
@@ -1501,10 +1508,10 @@ int adjoint_step(tti_handle *h, int n, int slot, const SourceTables &tab)
   memset(&sa, 0, sizeof sa);
   sa.g = g;
   for (int k = 0; k < 8; ++k) sa.lam[k] = a.lam[k];
-  const bool inject = c.seistype > 0 && it % c.mt == 0;
+  const bool inject = it % c.mt == 0;
   bool any = false;
   for (int k = 0; k < 3; ++k) {
-    const bool on = inject && s->res[k] && h->nrec[k] > 0;
+    const bool on = inject && recorded(h, k);
     sa.colptr[k] = h->d_rcol[k];
     sa.rzs[k] = h->d_rzs[k];
     sa.rid[k] = h->d_rid[k];
@@ -1659,12 +1666,11 @@ int grad_prepare(tti_handle *h, int slots, int seg, SourceTables *tab)
   if ((rc = grad_alloc(h))) return rc;
   GradState *s = h->grad;
   const tti_config &c = h->cfg;
-  const bool want_v = c.seistype == 1 || c.seistype == 3, want_p = c.seistype == 2 || c.seistype == 3;
   for (int k = 0; k < 3; ++k) {
-    const bool rec = (k < 2 ? want_v : want_p) && h->nrec[k] > 0;
-    if (rec && s->obs_n[k] == 0)
+    if (!recorded(h, k)) continue;
+    if (s->obs_n[k] == 0)
       return gerr(h, TTI_ERR_STATE, "observed traces missing for a recorded component");
-    if (rec && s->obs_n[k] != h->nrec[k])  // the receivers were set again
+    if (s->obs_n[k] != h->nrec[k])  // the receivers were set again
       return gerr(h, TTI_ERR_STATE, "as many observed traces as a recorded component has receivers are needed");
   }
   if ((rc = reserve(h, slots, seg))) return rc;
@@ -1687,13 +1693,10 @@ int grad_prepare(tti_handle *h, int slots, int seg, SourceTables *tab)
 int grad_start_adjoint(tti_handle *h, double *J)
 {
   GradState *s = h->grad;
-  const tti_config &c = h->cfg;
-  const bool want_v = c.seistype == 1 || c.seistype == 3, want_p = c.seistype == 2 || c.seistype == 3;
   const size_t n = h->g.n;
   GCK(h, cudaMemsetAsync(s->d_J, 0, sizeof(double), h->stream));
   for (int k = 0; k < 3; ++k) {
-    const bool rec = (k < 2 ? want_v : want_p) && h->nrec[k] > 0;
-    if (!rec) continue;
+    if (!recorded(h, k)) continue;
     const size_t m = (size_t)h->nrec[k] * h->nts;
     k_residual<<<std::min<size_t>(1024, (m + 255) / 256), 256, 0, h->stream>>>(h->d_rec[k], s->obs[k], s->res[k], m,
                                                                                s->d_J);
