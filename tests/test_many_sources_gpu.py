@@ -19,8 +19,10 @@ def _shot(h, n, where):
     sx[n // 2:] = sx[0]  # half of them in one column
     w = synthetic.ricker(NT, 0.0008, 30.0, delay=0.01)
     h.set_source(sx, sz, np.stack([w * np.float32(a) for a in rng.uniform(-2, 2, n)]))
+    # and more than a warp of receivers in a column, which with two sources none reaches
+    gx, gz = np.append(np.arange(NX), np.full(40, NX - 1)), np.append(np.full(NX, 3), np.arange(40))
     for k in (0, 1, 2):
-        h.set_receivers(k, np.arange(NX), 3)
+        h.set_receivers(k, gx, gz)
 
 
 def _result(h):

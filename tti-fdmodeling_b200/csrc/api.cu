@@ -152,6 +152,8 @@ int sync_columns(tti_handle *h)
   w.nt = c.nt;
   w.mode2 = c.mode == 2;
   w.mt = c.mt;
+  w.sx0 = h->src_at.x0;
+  w.sx1 = h->src_at.x1;
   w.scol = h->d_scol;
   w.sat = h->d_sat;
   w.shead = h->d_shead;
@@ -998,30 +1000,33 @@ int tti_set_source(tti_handle *h, int ntrace, const int *posx, const int *posz, 
   // their positions, the column offsets. A warp of the column work reads what
   // its column has. Going through all sources instead, a load each, 300 along the
   // surface of 600 x 1200 cells took 82 us a step, where one takes 18 (now 21);
-  // 750 at 1126 x 3000 228 (now 64).
-  const int Nx = h->g.Nx;
-  std::vector<int> col(Nx + 1, 0);
+  // 750 at 1126 x 3000 228 (now 65).
+  auto first_x = [&](int i) { return std::max(0, posx[i] + h->g.E - NH); };
+  auto last_x = [&](int i) { return std::min(h->g.Nx, posx[i] + h->g.E + NH + 1); };
   for (int i = 0; i < ntrace; ++i) {
-    const int x = posx[i] + h->g.E, z = posz[i] + h->g.E, x0 = std::max(0, x - NH), x1 = std::min(Nx, x + NH + 1);
-    h->src_at.add(x0, x1, std::max(0, z - NH), std::min(h->g.Nz, z + NH + 1));
-    for (int k = x0; k < x1; ++k) ++col[k + 1];
+    const int z = posz[i] + h->g.E;
+    h->src_at.add(first_x(i), last_x(i), std::max(0, z - NH), std::min(h->g.Nz, z + NH + 1));
   }
-  for (int k = 0; k < Nx; ++k) col[k + 1] += col[k];
-  const size_t m = (size_t)col[Nx];
-  std::vector<int> blk(4 * (m + Nx) + 2 * (size_t)ntrace + Nx + 1, 0), next(col.begin(), col.end());
-  int *head = blk.data() + 4 * m, *sx = head + 4 * (size_t)Nx, *sz = sx + ntrace;
+  const int x0 = h->src_at.x0, ncol = h->src_at.x1 - x0;
+  std::vector<int> col(ncol + 1, 0);
+  for (int i = 0; i < ntrace; ++i)
+    for (int k = first_x(i); k < last_x(i); ++k) ++col[k - x0 + 1];
+  for (int k = 0; k < ncol; ++k) col[k + 1] += col[k];
+  const size_t m = (size_t)col[ncol];
+  std::vector<int> blk(4 * (m + ncol) + 2 * (size_t)ntrace + ncol + 1, 0), next(col.begin(), col.end());
+  int *head = blk.data() + 4 * m, *sx = head + 4 * (size_t)ncol, *sz = sx + ntrace;
   std::copy(col.begin(), col.end(), sz + ntrace);
   for (int i = 0; i < ntrace; ++i) {
     sx[i] = posx[i] + h->g.E;
     sz[i] = posz[i] + h->g.E;
-    for (int k = std::max(0, sx[i] - NH); k < std::min(Nx, sx[i] + NH + 1); ++k) {
-      int *e = blk.data() + 4 * (size_t)next[k]++;
+    for (int k = first_x(i); k < last_x(i); ++k) {
+      int *e = blk.data() + 4 * (size_t)next[k - x0]++;
       e[0] = i;
       e[1] = sz[i];
       e[2] = k - sx[i];
     }
   }
-  for (int k = 0; k < Nx; ++k)
+  for (int k = 0; k < ncol; ++k)
     if (col[k + 1] > col[k]) {
       int *e = blk.data() + 4 * (size_t)col[k];
       e[3] = col[k + 1] - col[k];
@@ -1029,7 +1034,7 @@ int tti_set_source(tti_handle *h, int ntrace, const int *posx, const int *posz, 
     }
   CK(h, pool_alloc(reinterpret_cast<void **>(&h->d_sat), sizeof(int) * blk.size(), h->stream));
   h->d_shead = h->d_sat + m;
-  h->d_sx = reinterpret_cast<int *>(h->d_shead + Nx);
+  h->d_sx = reinterpret_cast<int *>(h->d_shead + ncol);
   h->d_sz = h->d_sx + ntrace;
   h->d_scol = h->d_sz + ntrace;
   CK(h, pool_alloc(reinterpret_cast<void **>(&h->d_src), sizeof(float) * (size_t)ntrace * c.nt, h->stream));

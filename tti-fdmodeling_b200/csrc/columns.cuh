@@ -23,19 +23,19 @@ __device__ __forceinline__ int record_index(const Columns &p, int it)
   return p.rec_on && it % p.mt == 0 ? it / p.mt : -1;
 }
 
-// A column's sources at time index it. The pointers are read once: what they
-// lie in is in global memory too, and the sources' stores could change it.
+// whether column ix may have sources
+__device__ __forceinline__ bool source_column(const Columns &p, int ix) { return ix >= p.sx0 && ix < p.sx1; }
+
+// Such a column's sources at time index it.
 struct ColumnSources {
-  int first, last;
-  const int4 *sat;
-  const float *a;
-  int nt;
-  __device__ __forceinline__ ColumnSources(const Columns &p, int ix, int it)
-      : first(p.scol[ix]), last(p.scol[ix + 1]), sat(p.sat), a(p.amp + it), nt(p.nt)
+  const Columns &p;
+  int it, first, last;
+  __device__ __forceinline__ ColumnSources(const Columns &q, int ix, int t)
+      : p(q), it(t), first(q.scol[ix - q.sx0]), last(q.scol[ix - q.sx0 + 1])
   {
   }
-  __device__ __forceinline__ int4 at(int j) const { return __ldg(sat + j); }
-  __device__ __forceinline__ float amp(const int4 &s) const { return __ldg(a + (size_t)s.x * nt); }
+  __device__ __forceinline__ int4 at(int j) const { return __ldg(p.sat + j); }
+  __device__ __forceinline__ float amp(const int4 &s) const { return __ldg(p.amp + (size_t)s.x * p.nt + it); }
 };
 
 // Rows [r0, r1) of column ix after the stress update, one warp (all lanes).
@@ -85,9 +85,10 @@ __device__ __forceinline__ void column_post(const Grid &g, const Fields &f, cons
     }
     __syncwarp();
   }
-  if (p.stype == 1) {
+  if (p.stype == 1 && source_column(p, ix)) {
     const ColumnSources src(p, ix, it);
-    const bool tensor = p.tensor;
+
+#pragma unroll 1
     for (int j = src.first; j < src.last; ++j) {
       const int4 s = src.at(j);
       const int iz = s.y + lane - NH;
@@ -96,7 +97,7 @@ __device__ __forceinline__ void column_post(const Grid &g, const Fields &f, cons
         const size_t c = col + iz;
         f.sxx[c] = __fadd_rn(f.sxx[c], ws);
         f.szz[c] = __fadd_rn(f.szz[c], ws);
-        if (tensor) {
+        if (p.tensor) {
           f.txx[c] = __fadd_rn(f.txx[c], ws);
           f.tzz[c] = __fadd_rn(f.tzz[c], ws);
         }
@@ -139,6 +140,7 @@ __device__ __forceinline__ void column_sources(const Grid &g, const Fields &f, c
 {
   const int lane = threadIdx.x & 31, it = time_index(p, n);
   const size_t col = (size_t)ix * g.ldz;
+  if (!source_column(p, ix)) return;
   const ColumnSources src(p, ix, it);
   if (p.stype == 8) {  // coord:782-801: four cells, one lane
     const float k = p.t.q8;
@@ -162,6 +164,7 @@ __device__ __forceinline__ void column_sources(const Grid &g, const Fields &f, c
   }
   const int first = p.stype == 4 ? 2 : p.stype, last = p.stype == 4 ? 3 : p.stype;  // stype 4: 2, then 3
   for (int kind = first; kind <= last; ++kind)
+#pragma unroll 1
     for (int j = src.first; j < src.last; ++j) {
       const int4 s = src.at(j);
       const int iz = s.y + lane - NH, w = (s.z + NH) * 11 + lane;

@@ -67,10 +67,11 @@ void launch_energy(const StepArgs &a, int nz, int nx, double *out2, cudaStream_t
 struct Columns {
   int stype;  // 0: no sources
   int freesurface, tensor, nt, mode2, mt, rec_on;
-  // sources by the columns their windows cover: entries [scol[ix], scol[ix + 1])
-  // of sat, in the sources' order: source, row, column offset ix - x, and in a
-  // column's first one the number of its entries. shead[ix]: that first one (all
-  // 0: none), one load away.
+  // sources by the columns [sx0, sx1) that their windows cover: column ix = sx0 + k
+  // has the entries [scol[k], scol[k + 1]) of sat, in the sources' order: source,
+  // row, column offset ix - x, and in a column's first one the number of its
+  // entries. shead[k]: that first one (all 0: none), one load away.
+  int sx0, sx1;
   const int *scol;
   const int4 *sat, *shead;
   const float *amp;  // [source][nt]
