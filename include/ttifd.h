@@ -314,18 +314,18 @@ int tti_batch_upload_model(tti_batch *b, int m, const float *vp, const float *vs
  * 1: shot after shot), and the loop replays a CUDA graph of `graph_steps`
  * steps (0: no graph). */
 int tti_batch_set_order(tti_batch *b, int group, int graph_steps);
-/* Grid of the batched half-step launches: 0 = one CTA per (instance, tile)
- * work item, 1 = persistent (one resident wave of CTAs walks the work table).
- * Both give the same bits. */
+/* Grid of the batched half-step launches: 0 or 1, kept for callers that set
+ * it. Either way they run one CTA per (instance, tile) work item: a resident
+ * wave of CTAs that walked the work table, which 1 stood for, gave the same bits
+ * and was slower at every size. */
 int tti_batch_set_schedule(tti_batch *b, int persistent);
 /* The schedule in use (any output may be NULL). */
 int tti_batch_get_schedule(const tti_batch *b, int *group, int *graph_steps, int *persistent);
 /* Times every group size in {all, 1, 4, 16} (those below the shot count)
- * with and without a graph of 20 steps, with one CTA per work item and with a
- * persistent grid, each over nsteps steps (at least one graph replay, at most
- * the longest instance's nt) in two rounds, keeps the fastest and resets the
- * batch. Outputs (may be NULL): the choice and its ms per step; the grid
- * chosen is read with tti_batch_get_schedule. */
+ * with and without a graph of 20 steps, each over nsteps steps (at least one
+ * graph replay, at most the longest instance's nt) in two rounds, keeps the
+ * fastest and resets the batch. Outputs (may be NULL): the choice and its ms per
+ * step. */
 int tti_batch_autotune(tti_batch *b, int nsteps, int *group, int *graph_steps, float *ms_per_step);
 /* Zeroes every instance and rebuilds the launch tables from the current
  * sources and receivers. */

@@ -1,7 +1,5 @@
-"""The persistent grid over several waves of work items: every CTA runs four or
-five tiles one after another in the same shared memory, at alternating phases of
-its barrier, with items of finished instances in between. The per-tile grid runs
-one item per CTA; fields and traces agree bit for bit."""
+"""Either grid setting over several waves of work items, with items of finished
+instances in between: fields and traces agree bit for bit."""
 import numpy as np
 import pytest
 
@@ -20,7 +18,7 @@ def _tiles(nx):
 
 
 @pytest.mark.parametrize("variant", ["coordinate_rotation", "tensor_rotation", "bond_transformation"])
-def test_several_items_a_cta(variant, monkeypatch, gpu_lib):
+def test_several_waves(variant, monkeypatch, gpu_lib):
     import ttifd
 
     monkeypatch.delenv("TTIFD_EXACT", raising=False)

@@ -42,7 +42,7 @@ struct tti_batch {
   int npost = 0, nsrc = 0, post_cols = 0, src_cols = 0;  // their number, their widest
   int *d_step = nullptr;
   int group = 0;  // work-table order: shots of a model interleaved tile by tile in groups of `group` (0: all)
-  bool persistent = false;  // one resident wave of CTAs walks the work table (else one CTA per item)
+  bool persistent = false;  // as set (tti_batch_set_schedule)
   int graph_steps = 20;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -186,7 +186,7 @@ int build_tables(tti_batch *b)
 tiled::BatchLaunch batch_launch(const tti_batch *b, bool vel, int offset)
 {
   return tiled::BatchLaunch{vel ? b->d_vel : b->d_str, vel ? (const void *)b->d_vmaps : b->d_smaps, b->d_work, b->nwork, b->d_step, offset, b->variant, b->exact,
-                            b->square, b->inst[0]->wait_limit, b->persistent};
+                            b->square, b->inst[0]->wait_limit};
 }
 
 // The launches of `n` time steps of all instances: each launch adds its own
@@ -370,13 +370,11 @@ int tti_batch_set_order(tti_batch *b, int group, int graph_steps)
 int tti_batch_set_schedule(tti_batch *b, int persistent)
 {
   if (!b || persistent < 0 || persistent > 1) return berr(b, TTI_ERR_ARG, "grid schedule must be 0 or 1");
-  if ((persistent == 1) != b->persistent) {  // the captured launches set the grid sizes
-    if (b->exec) cudaGraphExecDestroy(b->exec);
-    if (b->graph) cudaGraphDestroy(b->graph);
-    b->exec = nullptr;
-    b->graph = nullptr;
-    b->persistent = persistent == 1;
-  }
+  // No launch depends on it. A resident wave of CTAs that walked the work table
+  // was slower everywhere: us a step per item / walked, 16 shots of 1126 x 3000
+  // 911 / 1130, 12 models of mixed sizes 266 / 318, 6 x 600 x 1200 98 / 128, 24 x
+  // 200 x 400 69 / 95, 24 x 60 x 80 17.9 / 20.1 (tensor and Bond alike).
+  b->persistent = persistent == 1;
   return TTI_OK;
 }
 
@@ -452,46 +450,41 @@ int tti_batch_autotune(tti_batch *b, int nsteps, int *group, int *graph_steps, f
   for (int g : {1, 4, 16})
     if (g < ninst_max) groups.push_back(g);
   const int graphs[] = {0, 20};
-  const int NS = 2;  // grids: one CTA per tile, or a persistent wave
   // Each candidate is timed twice, in two rounds over all of them, and keeps
   // its faster time; a graph candidate is timed over at least one replay of
   // its graph (the step loop only replays it when that many steps remain).
   const int warm = std::min(2, nsteps);
-  std::vector<float> t_best(groups.size() * 2 * NS, -1.0f);
+  std::vector<float> t_best(groups.size() * 2, -1.0f);
   for (int round = 0; round < 2; ++round)
-    for (int ts = 0; ts < NS; ++ts)
-      for (size_t gi = 0; gi < groups.size(); ++gi)
-        for (int q = 0; q < 2; ++q) {
-          const int g = groups[gi], gs = graphs[q];
-          int timed = nsteps - warm;
-          if (gs > 0) timed = std::max(timed, gs);
-          timed = std::min(timed, b->max_nt - warm);
-          if (timed <= 0) continue;
-          int rc = tti_batch_set_order(b, g, gs);
-          if (!rc) rc = tti_batch_set_schedule(b, ts);
-          if (!rc) rc = tti_batch_reset(b);
-          if (!rc) rc = tti_batch_step(b, warm);  // warm-up (and graph instantiation)
-          if (!rc) rc = tti_batch_step(b, timed);
-          if (rc) return rc;
-          const float t = b->last_ms / timed;
-          float &tb = t_best[(ts * groups.size() + gi) * 2 + q];
-          if (tb < 0 || t < tb) tb = t;
-        }
-  float best = -1.0f;
-  int bg = 0, bs = 20, bt = 0;
-  for (int ts = 0; ts < NS; ++ts)
     for (size_t gi = 0; gi < groups.size(); ++gi)
       for (int q = 0; q < 2; ++q) {
-        const float t = t_best[(ts * groups.size() + gi) * 2 + q];
-        if (t >= 0 && (best < 0 || t < best)) {
-          best = t;
-          bg = groups[gi];
-          bs = graphs[q];
-          bt = ts;
-        }
+        const int g = groups[gi], gs = graphs[q];
+        int timed = nsteps - warm;
+        if (gs > 0) timed = std::max(timed, gs);
+        timed = std::min(timed, b->max_nt - warm);
+        if (timed <= 0) continue;
+        int rc = tti_batch_set_order(b, g, gs);
+        if (!rc) rc = tti_batch_reset(b);
+        if (!rc) rc = tti_batch_step(b, warm);  // warm-up (and graph instantiation)
+        if (!rc) rc = tti_batch_step(b, timed);
+        if (rc) return rc;
+        const float t = b->last_ms / timed;
+        float &tb = t_best[gi * 2 + q];
+        if (tb < 0 || t < tb) tb = t;
       }
+  float best = -1.0f;
+  int bg = 0, bs = 20;
+  for (size_t gi = 0; gi < groups.size(); ++gi)
+    for (int q = 0; q < 2; ++q) {
+      const float t = t_best[gi * 2 + q];
+      if (t >= 0 && (best < 0 || t < best)) {
+        best = t;
+        bg = groups[gi];
+        bs = graphs[q];
+      }
+    }
   int rc = tti_batch_set_order(b, bg, bs);
-  if (!rc) rc = tti_batch_set_schedule(b, bt);
+  if (!rc) rc = tti_batch_set_schedule(b, 0);
   if (!rc) rc = tti_batch_reset(b);
   if (rc) return rc;
   if (group) *group = bg;

@@ -136,7 +136,6 @@ struct BatchLaunch {
   int variant;
   bool exact, square;    // square: every instance has folded coefficients (set_square)
   unsigned wait_limit;   // polls of a box wait before it gives up
-  bool persistent;       // one resident wave of CTAs walks the table (else one CTA per item)
 };
 cudaError_t launch_velocity_batch(const BatchLaunch &l, cudaStream_t st);
 cudaError_t launch_stress_batch(const BatchLaunch &l, cudaStream_t st);
@@ -181,10 +180,6 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned pari
   }
   return false;
 }
-
-// Orders this thread's plain accesses to shared memory before copies (the async
-// proxy) that are issued behind the next block barrier.
-__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void tma_load_2d(float *dst, const CUtensorMap *map, int c_inner, int c_outer,
                                             unsigned long long *bar)

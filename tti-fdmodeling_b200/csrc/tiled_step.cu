@@ -785,58 +785,34 @@ __device__ __forceinline__ const HalfArgs &stage_args(const HalfArgs *src, void 
   return *static_cast<const HalfArgs *>(dst);
 }
 
-// One work item: the copies need only the item (its tile origin) and the
-// instance's maps, so they are in flight before the arguments are staged.
-// Returns false when the wait timed out. `bar` is followed by the staged
-// arguments, 16-byte aligned.
+// A CTA's work item: item blockIdx.x of the table (from its end for the stress
+// update, as in the single-shot kernels). The copies need only the item (its
+// tile origin) and the instance's maps, so they are in flight before the
+// arguments are staged. `bar` is followed by the staged arguments, 16-byte
+// aligned.
 template <typename I, typename F>
-__device__ __forceinline__ bool work_item(const BatchArgs &b, int i, int n, unsigned long long *bar, unsigned &ph,
-                                          I issue, F f)
+__device__ __forceinline__ void work_item(const BatchArgs &b, bool reverse, unsigned long long *bar, I issue, F f)
 {
+  walk::init_bar(bar);
+  pdl_sync();
+  const int n = *b.step + b.offset, i = reverse ? b.nwork - 1 - blockIdx.x : blockIdx.x;
   const int4 w = __ldg(reinterpret_cast<const int4 *>(b.work + i));  // inst, z0, x0 and the undamped bit, nt
-  if (n >= w.w) return true;  // uniform over the CTA
+  if (n >= w.w) return;  // uniform over the CTA
   const HalfArgs *src = b.inst + w.x;
   const int x0 = w.z & ~Work::UNDAMPED;
   const bool und = w.z & Work::UNDAMPED;
   issue(*src, w.x, und, w.y, x0);
   const HalfArgs &a = stage_args(src, bar + 2);
-  if (!walk::wait_boxes(src->err, bar, b.wait_limit, ph)) return false;
+  if (!walk::wait_boxes(src->err, bar, b.wait_limit, 0)) return;
   f(a, cells_of(a, w.y, x0), und, n);
-  ph ^= 1;
-  return true;
 }
 
-// Work items blockIdx.x, blockIdx.x + gridDim.x, ... of the table (reversed
-// for the stress update, as in the single-shot kernels): one item per CTA when
-// the grid covers the table, several (LOOP) when a persistent grid of one
-// resident wave walks it. The tile's shared memory is reused by the next item
-// only after every thread is done with it: the stress sums take the boxes'
-// place with plain stores, which nothing but a proxy fence orders before the
-// next item's copies into it.
-template <bool LOOP, typename I, typename F>
-__device__ __forceinline__ void for_work(const BatchArgs &b, bool reverse, unsigned long long *bar, I issue, F f)
-{
-  walk::init_bar(bar);
-  pdl_sync();
-  const int n = *b.step + b.offset;
-  unsigned ph = 0;
-  if (!LOOP) {
-    work_item(b, reverse ? b.nwork - 1 - blockIdx.x : blockIdx.x, n, bar, ph, issue, f);
-    return;
-  }
-  for (int i = blockIdx.x; i < b.nwork; i += gridDim.x) {
-    if (!work_item(b, reverse ? b.nwork - 1 - i : i, n, bar, ph, issue, f)) return;
-    tma::fence_async();  // the next copies land where this item's sums were stored
-    __syncthreads();
-  }
-}
-
-template <int V, bool X, bool Q, bool LOOP>
+template <int V, bool X, bool Q>
 __global__ void __launch_bounds__(walk::NT, 4) k_velocity_batch(const __grid_constant__ BatchArgs b)
 {
   extern __shared__ __align__(128) float sm[];
   unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + V_BAR);
-  for_work<LOOP>(
+  work_item(
       b, false, bar,
       [&](const HalfArgs &a, int inst, bool und, int z0, int x0) {
         walk::issue_tile(static_cast<const VelocityMaps *>(b.maps)[inst].box, 3, 4, nullptr, 0, 0, sm, 0, bar, z0, x0);
@@ -847,12 +823,12 @@ __global__ void __launch_bounds__(walk::NT, 4) k_velocity_batch(const __grid_con
       });
 }
 
-template <int V, bool X, bool Q, bool LOOP>
+template <int V, bool X, bool Q>
 __global__ void __launch_bounds__(walk::NT, 4) k_stress_batch(const __grid_constant__ BatchArgs b)
 {
   extern __shared__ __align__(128) float sm[];
   unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + s_bar(V));
-  for_work<LOOP>(
+  work_item(
       b, true, bar,
       [&](const HalfArgs &a, int inst, bool und, int z0, int x0) {
         const StressMaps &m = static_cast<const StressMaps *>(b.maps)[inst];
@@ -864,43 +840,29 @@ __global__ void __launch_bounds__(walk::NT, 4) k_stress_batch(const __grid_const
       });
 }
 
-// Sets a kernel's shared-memory attributes once and returns its CTAs per SM
-// times the SM count of the current device (one resident wave).
+// Sets a kernel's shared-memory attributes, once per device.
 template <typename K>
-cudaError_t prepare_kernel(K kernel, size_t bytes, int *wave)
+cudaError_t prepare_kernel(K kernel, size_t bytes)
 {
-  struct Seen {
-    const void *k;
-    int dev, wave;
-  };
   static std::mutex mu;
-  static std::vector<Seen> seen;
+  static std::vector<std::pair<const void *, int>> seen;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
+  const std::pair<const void *, int> key{(const void *)kernel, dev};
   std::lock_guard<std::mutex> lock(mu);
-  for (const Seen &q : seen)
-    if (q.k == (const void *)kernel && q.dev == dev) {
-      *wave = q.wave;
-      return cudaSuccess;
-    }
-  int sms = 0, per_sm = 0;
+  if (std::find(seen.begin(), seen.end(), key) != seen.end()) return cudaSuccess;
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, walk::NT, bytes);
-  if (e != cudaSuccess) return e;
-  *wave = std::max(1, per_sm) * sms;
-  seen.push_back(Seen{(const void *)kernel, dev, *wave});
-  return cudaSuccess;
+  if (e == cudaSuccess) seen.push_back(key);
+  return e;
 }
 
 template <typename M>
 cudaError_t launch_k(void (*kernel)(HalfArgs, M), const HalfArgs &a, const M &m, size_t smem, cudaStream_t st)
 {
-  int wave = 0;
-  const cudaError_t e = prepare_kernel(kernel, smem, &wave);
+  const cudaError_t e = prepare_kernel(kernel, smem);
   if (e != cudaSuccess) return e;
   int z_base, rows;
   const dim3 gr = tiles(a.g, a.g.izStart, &z_base, &rows);
@@ -1061,43 +1023,32 @@ cudaError_t launch_stress(const HalfArgs &a, const void *maps, int variant, bool
 // shared memory of a batched kernel whose barrier is at float `bar`
 constexpr size_t batch_smem(int bar) { return (size_t)(bar + 4) * sizeof(float) + sizeof(HalfArgs); }
 
-// One CTA per work item, or (persistent) one resident wave of CTAs that walks
-// the table: the SM count times the kernel's CTAs per SM at its shared memory.
+// One CTA per work item.
 template <typename K>
-cudaError_t launch_batch_k(K one, K loop, size_t smem, const BatchLaunch &l, cudaStream_t st)
+cudaError_t launch_batch_k(K kernel, size_t smem, const BatchLaunch &l, cudaStream_t st)
 {
-  const K kernel = l.persistent ? loop : one;
-  int wave = 0;
-  cudaError_t e = prepare_kernel(kernel, smem, &wave);
+  const cudaError_t e = prepare_kernel(kernel, smem);
   if (e != cudaSuccess || l.nwork == 0) return e;
   const BatchArgs b{l.inst, l.maps, l.work, l.step, l.nwork, l.offset, -0.0f, l.wait_limit};
-  return launch_pdl(kernel, dim3(l.persistent ? std::min(l.nwork, wave) : l.nwork), dim3(walk::NT), smem, st, b);
+  return launch_pdl(kernel, dim3(l.nwork), dim3(walk::NT), smem, st, b);
 }
 
 template <bool X, bool Q>
 cudaError_t velocity_batch_x(const BatchLaunch &l, cudaStream_t st)
 {
-  if (l.variant == TTI_COORDINATE)
-    return launch_batch_k(k_velocity_batch<TTI_COORDINATE, X, Q, false>, k_velocity_batch<TTI_COORDINATE, X, Q, true>,
-                          batch_smem(V_BAR), l, st);
-  if (l.variant == TTI_TENSOR)
-    return launch_batch_k(k_velocity_batch<TTI_TENSOR, X, Q, false>, k_velocity_batch<TTI_TENSOR, X, Q, true>,
-                          batch_smem(V_BAR), l, st);
-  return launch_batch_k(k_velocity_batch<TTI_BOND, X, Q, false>, k_velocity_batch<TTI_BOND, X, Q, true>,
-                          batch_smem(V_BAR), l, st);
+  constexpr size_t smem = batch_smem(V_BAR);
+  if (l.variant == TTI_COORDINATE) return launch_batch_k(k_velocity_batch<TTI_COORDINATE, X, Q>, smem, l, st);
+  if (l.variant == TTI_TENSOR) return launch_batch_k(k_velocity_batch<TTI_TENSOR, X, Q>, smem, l, st);
+  return launch_batch_k(k_velocity_batch<TTI_BOND, X, Q>, smem, l, st);
 }
 
 template <bool X, bool Q>
 cudaError_t stress_batch_x(const BatchLaunch &l, cudaStream_t st)
 {
-  if (l.variant == TTI_COORDINATE)
-    return launch_batch_k(k_stress_batch<TTI_COORDINATE, X, Q, false>, k_stress_batch<TTI_COORDINATE, X, Q, true>,
-                          batch_smem(s_bar(TTI_COORDINATE)), l, st);
-  if (l.variant == TTI_TENSOR)
-    return launch_batch_k(k_stress_batch<TTI_TENSOR, X, Q, false>, k_stress_batch<TTI_TENSOR, X, Q, true>,
-                          batch_smem(s_bar(TTI_TENSOR)), l, st);
-  return launch_batch_k(k_stress_batch<TTI_BOND, X, Q, false>, k_stress_batch<TTI_BOND, X, Q, true>,
-                          batch_smem(s_bar(TTI_BOND)), l, st);
+  constexpr int C = TTI_COORDINATE, T = TTI_TENSOR, B = TTI_BOND;
+  if (l.variant == C) return launch_batch_k(k_stress_batch<C, X, Q>, batch_smem(s_bar(C)), l, st);
+  if (l.variant == T) return launch_batch_k(k_stress_batch<T, X, Q>, batch_smem(s_bar(T)), l, st);
+  return launch_batch_k(k_stress_batch<B, X, Q>, batch_smem(s_bar(B)), l, st);
 }
 
 cudaError_t launch_velocity_batch(const BatchLaunch &l, cudaStream_t st)

@@ -491,7 +491,7 @@ class Batch:
     GRIDS = ["per-tile", "persistent"]
 
     def set_schedule(self, grid):
-        """Grid of the half-step launches: "per-tile" (0) or "persistent" (1)."""
+        """Grid of the half-step launches: "per-tile" (0) or "persistent" (1); both run one CTA per tile."""
         self._call("batch_set_schedule", self._b, self.GRIDS.index(grid) if isinstance(grid, str) else grid)
 
     def schedule(self) -> dict:
