@@ -335,11 +335,12 @@ int tti_batch_step(tti_batch *b, int nsteps);
 /* reset + step(max nt): every instance from it = 0 to its own nt. */
 int tti_batch_run(tti_batch *b);
 int tti_batch_elapsed_ms(const tti_batch *b, float *ms);
-/* Gradients of all instances at once: each instance (with its source,
- * receivers and tti_grad_set_observed traces) runs tti_grad_run_binomial
- * with the given schedule from its own host thread on its own stream, so the
- * shots' kernels overlap on the device, and the instances of a model share
- * its parameter arrays. Afterwards the sums of a model's instances are added
+/* Gradients of all instances: each instance (with its source, receivers and
+ * tti_grad_set_observed traces) runs tti_grad_run_binomial with the given
+ * schedule on its own stream. 4 to 8 host threads (as many as have their arrays
+ * in L2) take the instances one after another, so that many shots' kernels
+ * overlap on the device. The device memory of all of them is reserved first. The
+ * instances of a model share its parameter arrays. Afterwards the sums of a model's instances are added
  * into its first instance (tti_grad_fetch there gives the model's gradient
  * over those shots) and the other instances' sums are cleared.
  * tti_batch_elapsed_ms gives the wall time of the whole call. misfits

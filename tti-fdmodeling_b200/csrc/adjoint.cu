@@ -1299,7 +1299,7 @@ AdjArgs adj_args(tti_handle *h, int slot)
 }
 
 // Cells and weights of the velocity sources from the forward step's own
-// tables (the same float weights sources_block adds with), and the cells of
+// tables (the same float weights column_sources adds with), and the cells of
 // all windows outside the velocity update.
 int vsource_tables(tti_handle *h, const SourceTables &tab)
 {

@@ -80,14 +80,19 @@ inline void set_square(HalfArgs &a, bool exact)
 
 // Encodes a handle's MAPS tensor maps.
 bool encode_maps(CUtensorMap *map, const Grid &g, int variant, const Fields &f, const Params &p);
-// Whether a half-step launch of so many tiles triggers its dependent as soon as
-// it has waited for its own predecessor: only where the CTAs of two launches
-// fit the device together (4 a SM on 148 SMs). The next launch's CTAs then wait
-// in free slots. Where they do not fit, the part that finds a slot is spread
-// unevenly, so the trigger comes when a tile's sums are complete. us a step
-// early / late: 60 x 80 6.0 / 6.6, 300 x 600 (255 tiles) 7.95 / 9.1; 400 x 800
-// (440 tiles) 12.0 / 11.4, 500 x 1000 15.1 / 14.4, 600 x 1200 18.4 / 17.9,
+// Whether a single shot's half-step launch of so many tiles triggers its
+// dependent as soon as it has waited for its own predecessor: only where the
+// CTAs of two launches fit the device together (4 a SM on 148 SMs, as the plain
+// half-steps run; the stress kernel that keeps fields for the gradient runs 3, so
+// of 223 to 296 tiles two of its launches do not quite fit). The next launch's
+// CTAs then wait in free slots. Where they do not fit, the part that finds a slot
+// is spread unevenly, so the trigger comes when a tile's sums are complete. us a
+// step early / late: 60 x 80 6.0 / 6.6, 300 x 600 (255 tiles) 7.95 / 9.1; 400 x
+// 800 (440 tiles) 12.0 / 11.4, 500 x 1000 15.1 / 14.4, 600 x 1200 18.4 / 17.9,
 // 1126 x 3000 61.0 / 60.4.
+// The batched half-steps always trigger early; there it is close either way: 16
+// shots of 1126 x 3000 911.5 / 907, 12 models of mixed sizes 265.8 / 264.8, 6 x 600
+// x 1200 98.1 / 99.0, 24 x 200 x 400 69.4 / 70.1, 24 x 60 x 80 17.9 / 16.9.
 inline int early_trigger(long long tiles) { return 2 * tiles <= 4 * 148; }
 // The arguments of h's half-steps (a: handle_step_args), without column work.
 void fill_args(HalfArgs &ha, const tti_handle *h, const StepArgs &a);

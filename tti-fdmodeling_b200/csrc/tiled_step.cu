@@ -7,9 +7,10 @@
 // (cp.async.bulk.tensor, completion on an mbarrier, bounded wait); the box
 // starts at row z0 - 8, so its innermost coordinate stays 16-byte aligned, and
 // coordinates outside the array read zeros. The stencil sums come from the
-// diagonal walks of walk.cuh (52 shared accesses per four cells of the velocity
-// update instead of 240), then each lane updates four rows of one column with
-// 128-bit accesses and packed arithmetic. The velocity kernel reads only stress
+// diagonal walks of walk.cuh (per four cells of the velocity update 51 shared
+// loads, 24 stores of the sums and 6 16-byte reads of them, instead of 240 loads),
+// then each lane updates four rows of one column with 128-bit accesses and packed
+// arithmetic. The velocity kernel reads only stress
 // and the stress kernel only velocity from the boxes, so in-place updates are
 // race-free.
 //
@@ -116,7 +117,7 @@ __device__ __forceinline__ void load_coefs(const HalfArgs &a, bool und, size_t g
 
 // Shared memory of a velocity tile: the three boxes, the six sum arrays, the
 // barrier. Stress tile: the two boxes, whose place the four sum arrays take
-// once the walks have read them, the tile's own inputs (HalfArgs::in),
+// once the walks have read them, the tile's own inputs (StressMaps::in),
 // tile_rows x WX each, the barrier.
 constexpr int V_SUMS = walk::LEAD + 3 * walk::BOX, V_BAR = V_SUMS + 6 * walk::SUM;
 constexpr int V_STASH = V_BAR + 16, V_END = V_STASH + walk::NT / 32 * 11 * 4;  // (single shots: source_terms)
@@ -600,7 +601,7 @@ __device__ __forceinline__ void more_work(const HalfArgs &a, int ix, int r0, int
   }
 }
 
-// S: the column's sigma, rows -8 .. 127 of the tile, in place of its sums; tau
+// S: the column's sigma, rows -8 .. 119 of the tile, in place of its sums; tau
 // (tensor) in place of its inputs.
 template <int V>
 __device__ __forceinline__ void column_work(const HalfArgs &a, const Cells &c, size_t gi, const F4 (&n)[3],

@@ -167,8 +167,9 @@ __device__ __forceinline__ bool wait_boxes(int *err, unsigned long long *bar, un
   return true;
 }
 
-// One warp's L2 prefetch of a tile's rows of an array: lanes take the four
-// 128-byte lines of each of the WX columns.
+// One warp's L2 prefetch of a tile's rows of an array: lanes take four 128-byte
+// lines of each of the WX columns. (A tile of 120 rows that begins 16 or 24 rows
+// into a line reaches into a fifth, which is left to the loads.)
 __device__ __forceinline__ void prefetch_lines(const float *base, const Grid &g, int x0, int z0, int rows)
 {
   static_assert(WX == 8 && WZ <= 128, "four lines of eight columns");
